@@ -937,10 +937,8 @@ def run_prefill(args):
         "config": {"workload": "varlen causal prefill attention, one layer, 32 q / 8 kv heads of 128, 1 x 16384 tokens "
                                "(headline) and 4 x 4096 tokens", "l2": "q, k, v and out of a call: 168 MB > 126 MB L2"},
         "cases": res, "gpu_launches": launches, "clocks": clocks.summary(),
-        "roofline": {"bound": "tensor", "kernel": "prefill_tc_kernel", "achieved": head["tflops"], "peak": peak,
+        "roofline": {"bound": "tensor", "kernel": "attn_tc_kernel", "achieved": head["tflops"], "peak": peak,
                      "unit": "TFLOP/s", "frac": head["tflops"] / peak,
-                     "executed": head["tflops"] * 1.5,
-                     "executed_note": "the kernel recomputes Q.K^T in its second pass: 3 tile products per 2 counted",
                      "peak_source": "measured burst cuBLAS bf16 (MEASURED_PEAKS.json)" if peaks else "fallback",
                      "traffic": None},
     }))
