@@ -154,13 +154,21 @@ silu_and_mul_kernel(const T* __restrict__ x, T* __restrict__ out, int I, int64_t
 }
 
 // ---------------------------------------------------------------------------------------------
-// Fused q/k RMSNorm + rotary embedding + cache writes.  One warp per token walks the token's heads
-// four at a time (eight lanes per head; a lane owns D/16 consecutive dims of each half of the
-// head — the rotation pairs dim d with d + D/2 — and moves them as one vector), with the next
-// four heads' loads in flight: q heads -> q_out; k heads -> k_out and the K cache; v heads -> the
-// V cache.  Warps past the tokens redo the q heads of a window token and write them into the
-// observation-window buffer.
+// Fused q/k RMSNorm + rotary embedding + cache writes.  A warp walks some heads of one kind (q, k or v) of one token, four at a
+// time (eight lanes per head; a lane owns D/16 consecutive dims of each half of the head — the rotation pairs dim d with d + D/2
+// — and moves them as one vector), with the next four heads' loads in flight: q heads -> q_out; k heads -> k_out and the K
+// cache; v heads -> the V cache, a plain copy.  Rows past the tokens redo the q heads of a window token and write them into
+// the observation-window buffer.
+//
+// What bounds it is the loads in flight: with one kind of head a warp keeps one weight and the token's cosines and sines in
+// registers (twice the warps per SM that a walk over all heads of a token left room for), and v heads do no arithmetic.  Many
+// tokens: 32 heads a warp, so that cosines, sines and weights are fetched once for eight turns.  Few tokens (below QK_SPREAD,
+// where a warp per token does not fill the SMs): four heads a warp, one turn of latency.
+// 32 / 8 heads of 128, bf16: 16384 tokens 89 us = 4.9 TB/s (16 heads a warp 96, 8 105, 4 130; one warp for all kinds 114), 4 tokens
+// 2.6 us (7.6).
 // ---------------------------------------------------------------------------------------------
+constexpr int QK_SPREAD = 1024;
+
 struct QkArgs {
   const void* qkv; const int64_t* positions; const float* cos_sin;
   const void* q_weight; const void* k_weight;
@@ -170,6 +178,7 @@ struct QkArgs {
   int n_tokens, n_triples, Hq, Hkv;
   int64_t qkv_stride, cache_stride_seq, cache_stride_slot;
   float eps;
+  int per, nq, nk;                // heads a warp walks; warps of a token's q heads, and of its k (and of its v) heads
 };
 
 // N consecutive elements of T moved as one (or two) vector accesses
@@ -225,23 +234,21 @@ template <typename T, int D>
 __global__ void __launch_bounds__(256) qk_norm_rope_store_kernel(const QkArgs a) {
   constexpr int P = D / 16;
   const int lane = threadIdx.x & 31, l8 = lane & 7, hg = lane >> 3;   // 4 heads per warp at a time
-  // one warp per work item: a token, or (items >= n_tokens) a window triple
-  const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (item >= a.n_tokens + a.n_triples) return;
-  const T* qkv = reinterpret_cast<const T*>(a.qkv);
-  const bool window = item >= a.n_tokens;
-  int n, qid = 0, idx = 0;
-  if (!window) n = item;
-  else {
+  const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), part = blockIdx.y;
+  const bool is_q = part < a.nq, is_v = part >= a.nq + a.nk, window = item >= a.n_tokens;
+  if (item >= a.n_tokens + a.n_triples || (window && !is_q)) return;
+  int n = item, qid = 0, idx = 0;
+  if (window) {
     const int t = item - a.n_tokens;
     if (a.n_triples_dev && t >= *a.n_triples_dev) return;   // n_triples was only the upper bound
     n = a.triples[3 * t]; qid = a.triples[3 * t + 1]; idx = a.triples[3 * t + 2];
   }
-  const T* row = qkv + (int64_t)n * a.qkv_stride;
-  const int H = window ? a.Hq : a.Hq + 2 * a.Hkv;
+  const int heads = is_q ? a.Hq : a.Hkv, base = is_q ? 0 : is_v ? a.Hq + a.Hkv : a.Hq;   // of this kind, and where they start in a row
+  const int h_begin = (part - (is_q ? 0 : is_v ? a.nq + a.nk : a.nq)) * a.per, h_end = min(h_begin + a.per, heads);
+  const T* row = reinterpret_cast<const T*>(a.qkv) + (int64_t)n * a.qkv_stride + (int64_t)base * D;
   // the first heads' elements are requested before the (dependent) cos/sin loads
   auto load_head = [&](int h, Chunk<T, P>& ca, Chunk<T, P>& cb) {
-    if (h < H) {
+    if (h < h_end) {
       ca = ld_chunk<T, P>(row + (int64_t)h * D + l8 * P);
       cb = ld_chunk<T, P>(row + (int64_t)h * D + D / 2 + l8 * P);
     } else {
@@ -250,45 +257,47 @@ __global__ void __launch_bounds__(256) qk_norm_rope_store_kernel(const QkArgs a)
     }
   };
   Chunk<T, P> ca, cb, na, nb;
-  load_head(hg, ca, cb);
-  // this lane's slices of the token's cos/sin row and of the two weights
+  load_head(h_begin + hg, ca, cb);
+  const int slot = !is_q && a.slot_mapping ? a.slot_mapping[n] : -1;
+  if (is_v) {
+    if (slot == -1) return;
+    T* dst = reinterpret_cast<T*>(a.v_cache) + (int64_t)slot * a.Hkv * D;
+    for (int h = h_begin + hg; h < h_end; h += 4) {
+      load_head(h + 4, na, nb);
+      st_chunk<T, P>(dst + (int64_t)h * D + l8 * P, ca);
+      st_chunk<T, P>(dst + (int64_t)h * D + D / 2 + l8 * P, cb);
+      ca = na; cb = nb;
+    }
+    return;
+  }
+  // this lane's slices of the token's cos/sin row and of the weight
   const float* cs = a.cos_sin + a.positions[n] * D;
+  const T* wp = reinterpret_cast<const T*>(is_q ? a.q_weight : a.k_weight);
   float c[P], sn[P];
   {
     const Chunk<float, P> cc = ld_chunk<float, P>(cs + l8 * P), sc = ld_chunk<float, P>(cs + D / 2 + l8 * P);
 #pragma unroll
     for (int j = 0; j < P; ++j) { c[j] = cc.v[j]; sn[j] = sc.v[j]; }
   }
-  const Chunk<T, P> qw1 = ld_chunk<T, P>(reinterpret_cast<const T*>(a.q_weight) + l8 * P);
-  const Chunk<T, P> qw2 = ld_chunk<T, P>(reinterpret_cast<const T*>(a.q_weight) + D / 2 + l8 * P);
-  const Chunk<T, P> kw1 = ld_chunk<T, P>(reinterpret_cast<const T*>(a.k_weight) + l8 * P);
-  const Chunk<T, P> kw2 = ld_chunk<T, P>(reinterpret_cast<const T*>(a.k_weight) + D / 2 + l8 * P);
-  const int slot = (!window && a.slot_mapping) ? a.slot_mapping[n] : -1;
-  T* wbase = window ? reinterpret_cast<T*>(a.query_cache) + (int64_t)qid * a.cache_stride_seq +
-                          (int64_t)idx * a.cache_stride_slot : nullptr;
-  // every lane runs the same number of iterations (the shuffles need the whole warp)
-  for (int h0 = 0; h0 < H; h0 += 4) {
+  const Chunk<T, P> w1 = ld_chunk<T, P>(wp + l8 * P), w2 = ld_chunk<T, P>(wp + D / 2 + l8 * P);
+  T* d0 = nullptr;                // where the heads go: output (or window buffer), ...
+  T* d1 = nullptr;                // ... and cache
+  if (window) d0 = reinterpret_cast<T*>(a.query_cache) + (int64_t)qid * a.cache_stride_seq + (int64_t)idx * a.cache_stride_slot;
+  else if (is_q) d0 = reinterpret_cast<T*>(a.q_out) + (int64_t)n * a.Hq * D;
+  else {
+    if (a.k_out) d0 = reinterpret_cast<T*>(a.k_out) + (int64_t)n * a.Hkv * D;
+    if (slot != -1) d1 = reinterpret_cast<T*>(a.k_cache) + (int64_t)slot * a.Hkv * D;
+  }
+  // every lane runs the same number of turns (the shuffles need the whole warp)
+  for (int h0 = h_begin; h0 < h_end; h0 += 4) {
     const int h = h0 + hg;
     load_head(h + 4, na, nb);   // the next four heads, in flight while these are computed
-    const bool live = h < H;
-    const bool is_q = h < a.Hq, is_k = !is_q && h < a.Hq + a.Hkv;
     Chunk<T, P> o1, o2;
-    if (is_q) norm_rope_head<T, D>(ca, cb, qw1, qw2, c, sn, a.eps, o1, o2);
-    else norm_rope_head<T, D>(ca, cb, kw1, kw2, c, sn, a.eps, o1, o2);   // (v heads: result unused)
-    if (live) {
-      T* d0 = nullptr; T* d1 = nullptr;
-      if (window) d0 = wbase + (int64_t)h * D;
-      else if (is_q) d0 = reinterpret_cast<T*>(a.q_out) + ((int64_t)n * a.Hq + h) * D;
-      else if (is_k) {
-        if (a.k_out) d0 = reinterpret_cast<T*>(a.k_out) + ((int64_t)n * a.Hkv + (h - a.Hq)) * D;
-        if (slot != -1) d1 = reinterpret_cast<T*>(a.k_cache) + ((int64_t)slot * a.Hkv + (h - a.Hq)) * D;
-      } else if (slot != -1) {   // v head: plain copy into the cache
-        T* vd = reinterpret_cast<T*>(a.v_cache) + ((int64_t)slot * a.Hkv + (h - a.Hq - a.Hkv)) * D;
-        st_chunk<T, P>(vd + l8 * P, ca);
-        st_chunk<T, P>(vd + D / 2 + l8 * P, cb);
-      }
-      if (d0) { st_chunk<T, P>(d0 + l8 * P, o1); st_chunk<T, P>(d0 + D / 2 + l8 * P, o2); }
-      if (d1) { st_chunk<T, P>(d1 + l8 * P, o1); st_chunk<T, P>(d1 + D / 2 + l8 * P, o2); }
+    norm_rope_head<T, D>(ca, cb, w1, w2, c, sn, a.eps, o1, o2);
+    if (h < h_end) {
+      const int64_t at = (int64_t)h * D + l8 * P;
+      if (d0) { st_chunk<T, P>(d0 + at, o1); st_chunk<T, P>(d0 + at + D / 2, o2); }
+      if (d1) { st_chunk<T, P>(d1 + at, o1); st_chunk<T, P>(d1 + at + D / 2, o2); }
     }
     ca = na; cb = nb;
   }
@@ -547,7 +556,10 @@ extern "C" int zp_qk_norm_rope_store(const void* qkv, const int64_t* positions, 
   a.qkv_stride = qkv_stride; a.cache_stride_seq = cache_stride_seq; a.cache_stride_slot = cache_stride_slot;
   a.eps = eps;
   cudaStream_t st = (cudaStream_t)stream;
-  const int grid = (n_tokens + n_triples + 7) / 8;   // eight warps per block, one work item each
+  a.per = n_tokens < zp::QK_SPREAD ? 4 : 32;
+  a.nq = (Hq + a.per - 1) / a.per;
+  a.nk = (Hkv + a.per - 1) / a.per;
+  const dim3 grid((n_tokens + n_triples + 7) / 8, a.nq + 2 * a.nk);   // eight warps per block, one token each
   ZP_DISPATCH_DTYPE(dtype, T, {
     if (D == 128) zp::qk_norm_rope_store_kernel<T, 128><<<grid, 256, 0, st>>>(a);
     else zp::qk_norm_rope_store_kernel<T, 64><<<grid, 256, 0, st>>>(a);
