@@ -33,3 +33,38 @@ def test_qk_norm_rope_is_the_same_for_few_and_many_tokens(dtype, heads, kv_heads
         return torch.cat([q for q, _ in out]), torch.cat([k for _, k in out]), kc, vc, qc
     for x, y in zip(run([(0, N)]), run([(0, 550), (550, N)])):
         assert torch.equal(x, y)
+
+
+def _draws(seed, rows, V):
+    """The Exp(1) draws of the built-in generator (fp64 logarithm of the same uniform numbers)."""
+    m = 0xFFFFFFFF
+
+    def mix(x):
+        x = x ^ (x >> 16)
+        x = (x * 0x7feb352d) & m
+        x = x ^ (x >> 15)
+        x = (x * 0x846ca68b) & m
+        return x ^ (x >> 16)
+    r, i = torch.arange(rows, device="cuda")[:, None], torch.arange(V, device="cuda")[None]
+    h = mix(((seed & m) ^ ((r * 0x9e3779b9) & m)) + ((i * 0x85ebca6b) & m) & m)
+    h = mix(h ^ (seed >> 32) ^ r)
+    u = ((h >> 8).float() + 0.5) * (1.0 / 16777216.0)
+    return (-torch.log(u.double())).clamp_min(1e-10)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,V", [(1, 1), (3, 7), (5, 8191), (4, 8192), (2, 16385), (3, 50257), (9, 151936)])
+@pytest.mark.parametrize("spread", [0.01, 3.0])
+def test_sampler_takes_the_best_of_all_draws(dtype, rows, V, spread):
+    """Against the race over every draw in fp64: the sampled token's ratio is the largest up to the draws' fp32 rounding (a fast
+    logarithm, 2^-21 of its argument's distance from 1, and a few roundings)."""
+    from zipage_b200.layers import step_ops as P
+    z = (torch.randn(rows, V, device="cuda", generator=_gen(V)) * spread).to(dtype)
+    t = 0.5 + torch.rand(rows, device="cuda", generator=_gen(rows))
+    seed = (5 << 32) + 12345 + V
+    tok = P.sample(z, t, seed=seed)
+    q = _draws(seed, rows, V)
+    x = z.double() / t.double()[:, None]
+    e = torch.exp(x - x.max(-1, keepdim=True).values)
+    lower, upper = (e / (q + 1e-6)).max(-1).values, (e / (q - 1e-6).clamp_min(1e-10)).gather(1, tok[:, None])[:, 0]
+    assert (upper >= lower * (1 - 1e-5)).all()

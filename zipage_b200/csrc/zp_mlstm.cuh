@@ -49,19 +49,4 @@ __device__ __forceinline__ MlstmSeq mlstm_seq(const MlstmArgs& a, int b) {
   return s;
 }
 
-// ---- thread-block clusters along the value dims: per-row sums over the whole head ---------------
-__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ uint32_t cluster_size() { uint32_t r; asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// a float of the same shared-memory variable in another block of the cluster
-__device__ __forceinline__ float ld_cluster(const float* p, uint32_t rank) {
-  uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p)), ra;
-  float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
-  return v;
-}
-
 }  // namespace zp
