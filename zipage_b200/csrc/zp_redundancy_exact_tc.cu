@@ -188,7 +188,7 @@ redundancy_exact_tc_kernel(const __grid_constant__ CUtensorMap tmK, const XtPara
   extern __shared__ unsigned char smem_raw[];
   unsigned char* bufs = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   XtShared& sh = *reinterpret_cast<XtShared*>(bufs + XT_NSLOT * XT_PAGE_BYTES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < XT_NSLOT; ++i) { mbar_init(&sh.full[i], 1); mbar_init(&sh.empty[i], 1); }
@@ -232,7 +232,7 @@ redundancy_exact_tc_kernel(const __grid_constant__ CUtensorMap tmK, const XtPara
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       prefetch_tensormap(&tmK);
       SlotFifo fifo;
       bool ok = true;
@@ -275,7 +275,7 @@ redundancy_exact_tc_kernel(const __grid_constant__ CUtensorMap tmK, const XtPara
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       SlotFifo fifo;
       int nj = 0;
       uint32_t use = 0;   // items issued per row group so far (both groups take part in every page)
@@ -284,18 +284,18 @@ redundancy_exact_tc_kernel(const __grid_constant__ CUtensorMap tmK, const XtPara
         const Job jb(p, job);
         if (!jb.valid) continue;
         const int sa = fifo.pop();
-        if (!mbar_wait<true>(&sh.full[sa], fifo.use(sa) & 1, abortp, p.error_word, 201)) break;
+        if (!mbar_wait(&sh.full[sa], fifo.use(sa) & 1, abortp, p.error_word, 201)) break;
         mbar_arrive(&sh.aready[nj & 1]);
         const uint32_t a_addr = smem_u32(bufs + sa * XT_PAGE_BYTES);
         for (int pg = jb.mp; ok && pg < p.NB; ++pg) {
           if (jb.table[pg] == -1) continue;
           const int sb = fifo.pop();
           fifo.push(sb);
-          if (!mbar_wait<true>(&sh.full[sb], fifo.use(sb) & 1, abortp, p.error_word, 202)) { ok = false; break; }
+          if (!mbar_wait(&sh.full[sb], fifo.use(sb) & 1, abortp, p.error_word, 202)) { ok = false; break; }
           const uint32_t b_addr = smem_u32(bufs + sb * XT_PAGE_BYTES);
 #pragma unroll
           for (int g = 0; g < 2; ++g) {
-            if (!mbar_wait<true>(&sh.tempty[g], (use & 1) ^ 1, abortp, p.error_word, 203)) { ok = false; break; }
+            if (!mbar_wait(&sh.tempty[g], (use & 1) ^ 1, abortp, p.error_word, 203)) { ok = false; break; }
             fence_after_sync();
             umma_k128(tmem_base + g * 256, a_addr + g * 16384, XT_BLOCK_BYTES, b_addr, XT_BLOCK_BYTES, IDESC);
             umma_commit(&sh.tfull[g]);

@@ -84,7 +84,7 @@ redundancy_tc_kernel(const __grid_constant__ CUtensorMap tmK, const RtParams p) 
   RtShared& sh = *reinterpret_cast<RtShared*>(bufs + RT_NS * RT_PAGE_BYTES);
   constexpr int NS = RT_NS;
   auto stage_ptr = [&](int s) { return bufs + s * RT_PAGE_BYTES; };
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     // a stage is released by the MMA commit and by the team that read it for the norms
@@ -122,7 +122,7 @@ redundancy_tc_kernel(const __grid_constant__ CUtensorMap tmK, const RtParams p) 
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       prefetch_tensormap(&tmK);
       int t = 0;
       bool ok = true;
@@ -144,7 +144,7 @@ redundancy_tc_kernel(const __grid_constant__ CUtensorMap tmK, const RtParams p) 
     // ---------------- MMA issuer ----------------
     // Pages of a job are issued in pairs (one per team): both first halves, then both second
     // halves, so that each team's accumulator is refilled while the other team's is being read.
-    if (lane == 0) {
+    if (elect_one()) {
       int t = 0;
       bool ok = true;
       auto issue = [&](int tt, int hh) -> bool {   // item (page tt, row half hh) into team tt & 1

@@ -207,7 +207,7 @@ window_score_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     return;
   }
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int R = G * p.qcl_pass;
 
   if (threadIdx.x == 0) {
@@ -243,7 +243,7 @@ window_score_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
   };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       prefetch_tensormap(&tmK);
       prefetch_tensormap(&tmQ);
       int s = 0, sph = 0, n = 0;  // ring stage and its phase; n counts the units that have tiles
@@ -279,7 +279,7 @@ window_score_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC_QK = idesc_f16(UmmaFmt<T>::fmt, 128, 256);
       constexpr uint32_t IDESC_KQ = idesc_f16(UmmaFmt<T>::fmt, 128, 128);
       int gt = 0, n = 0, s = 0, sph = 0;
