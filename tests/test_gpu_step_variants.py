@@ -68,3 +68,27 @@ def test_sampler_takes_the_best_of_all_draws(dtype, rows, V, spread):
     e = torch.exp(x - x.max(-1, keepdim=True).values)
     lower, upper = (e / (q + 1e-6)).max(-1).values, (e / (q - 1e-6).clamp_min(1e-10)).gather(1, tok[:, None])[:, 0]
     assert (upper >= lower * (1 - 1e-5)).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,heads,kv_heads,width", [(1, 8, 8, 16), (2, 16, 1, 9), (5, 32, 8, 16), (3, 4, 2, 17), (70, 8, 1, 4)])
+def test_paged_decode_splits(dtype, B, heads, kv_heads, width):
+    """Short tables split within a cluster, longer ones (17 pages) through scratch."""
+    from zipage_b200.layers.attention import paged_decode_attention
+    g, D = _gen(B), 128
+    lens = torch.tensor([1, 63, 64, 65, width * 256][:B] + [128 + 13 * i for i in range(max(0, B - 5))], dtype=torch.int32, device="cuda")
+    table = torch.full((B, width), -1, dtype=torch.int32, device="cuda")
+    need = ((lens + 255) // 256).tolist()
+    ids = torch.randperm(sum(need), device="cuda", generator=g).to(torch.int32)
+    for b, part in enumerate(ids.split(need)):
+        table[b, :need[b]] = part
+    kc, vc = (torch.randn(sum(need), 256, kv_heads, D, device="cuda", generator=g).to(dtype) for _ in range(2))
+    q = torch.randn(B, 1, heads, D, device="cuda", generator=g).to(dtype)
+    out = paged_decode_attention(q, kc, vc, lens, table)
+    unit = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * 1.1      # weights and result are rounded once each
+    for b in range(B):
+        n = int(lens[b])
+        k, v = (c[table[b, :need[b]].long()].flatten(0, 1)[:n].double().repeat_interleave(heads // kv_heads, 1) for c in (kc, vc))
+        w = torch.softmax(torch.einsum("hd,shd->hs", q[b, 0].double(), k) * D ** -0.5, -1)
+        ref, mag = torch.einsum("hs,shd->hd", w, v), torch.einsum("hs,shd->hd", w, v.abs())
+        assert ((out[b, 0].double() - ref).abs() <= 2 * unit * mag + 1e-6).all()

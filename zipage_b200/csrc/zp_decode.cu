@@ -184,6 +184,18 @@ static int pick_splits(int B, int Hkv, int NBmax) {
   return s < 1 ? 1 : s;
 }
 
+// The mma.sync kernel splits between any two 64-key tiles, and up to 8 splits of a sequence are a cluster that needs no scratch and no
+// second launch.  A cluster takes contexts of up to DEC_CLUSTER_KEYS, where its splits have at most as many keys as two pages;
+// beyond, a small batch needs more than 8 splits to fill the SMs.
+// 4 sequences of 700 to 2304 keys, 16 heads on 8, a layer: 11.7 us (whole pages a split, scratch and a merge kernel: 15.7).
+constexpr int64_t DEC_CLUSTER_KEYS = 4096;
+static int pick_cluster(int B, int Hkv, int NBmax, int BS) {
+  const int64_t keys = (int64_t)NBmax * BS, want = (148 * 6 + B * Hkv - 1) / (B * Hkv);      // two rounds of three blocks an SM
+  int s = 1;
+  while (s < 8 && s < want && keys / (2 * s) >= 128) s *= 2;
+  return s;
+}
+
 template <typename T, int D, int GP>
 static int launch_decode(DecArgs a, cudaStream_t st) {
   constexpr int LPK = D / (16 / sizeof(T));
@@ -241,9 +253,15 @@ extern "C" int zp_paged_decode(const void* q, const void* k_cache, const void* v
   a.B = B; a.NBmax = NBmax; a.Hq = Hq; a.Hkv = Hkv; a.BS = BS;
   a.kv_stride_page = kv_stride_page;
   a.scale_log2e = softmax_scale * 1.4426950408889634f;
+  const bool mma = (dtype == ZP_DTYPE_BF16 || dtype == ZP_DTYPE_F16) && D == 128 && BS % 64 == 0 && G <= 16;
   a.nsplit = zp::pick_splits(B, Hkv, NBmax);
   a.part = nullptr;
-  if (a.nsplit > 1) {
+  if (const size_t off = (uintptr_t)workspace % 8; workspace && off) {      // (partial results are read in pairs)
+    workspace = (char*)workspace + (8 - off);
+    workspace_bytes = workspace_bytes > 8 - off ? workspace_bytes - (8 - off) : 0;
+  }
+  if (mma && (int64_t)NBmax * BS <= zp::DEC_CLUSTER_KEYS) a.nsplit = zp::pick_cluster(B, Hkv, NBmax, BS);
+  else if (a.nsplit > 1) {
     const size_t need = (size_t)B * Hkv * a.nsplit * zp::gp_of(G) * (D + 2) * sizeof(float);
     if (!workspace || workspace_bytes < need) {
       // no scratch: run unsplit (correct, but one block per (sequence, kv head) leaves a small
@@ -255,7 +273,6 @@ extern "C" int zp_paged_decode(const void* q, const void* k_cache, const void* v
     else a.part = reinterpret_cast<float*>(workspace);
   }
   cudaStream_t st = (cudaStream_t)stream;
-  const bool mma = (dtype == ZP_DTYPE_BF16 || dtype == ZP_DTYPE_F16) && D == 128 && BS % 64 == 0 && G <= 16;
   if (mma)
     return zp::paged_decode_mma(q, k_cache, v_cache, cache_seqlens, block_table, out, a.part, B, NBmax,
                                 Hq, Hkv, BS, a.nsplit, zp::gp_of(G), kv_stride_page, a.scale_log2e, dtype,

@@ -7,19 +7,22 @@
 // with 16-byte cp.async copies (two stages, XOR-swizzled 16-byte chunks so that ldmatrix is
 // conflict-free), each of the four warps takes 16 keys of a tile: S = Q K^T (16 MMAs), online
 // softmax in registers, O += P V (16 MMAs, V through ldmatrix.trans).  Warps, then key splits, are
-// merged with the (max, sum, weighted output) rule.  One block per (sequence, kv head, split).
+// merged with the (max, sum, weighted output) rule.  One block per (sequence, kv head, split).  The splits of short contexts (a
+// cache kept within its budget) are a cluster and merge through distributed shared memory; with long contexts, more than
+// DM_CLUSTER splits leave partial results that a second kernel merges.
 #include "zp_mma.cuh"
 
 namespace zp {
 
 constexpr int DM_THREADS = 128;
 constexpr int DM_TILE = 64;                // keys per tile
+constexpr int DM_CLUSTER = 8;              // splits of a cluster (portable size)
 constexpr int DM_TILE_BYTES = DM_TILE * MMA_ROW_BYTES;  // 16 KB per K or V tile
 
 struct DmArgs {
   const void* q; const void* k; const void* v;
   const int32_t* seqlens; const int32_t* table;
-  void* out; float* part;  // part: [B][Hkv][nsplit][gp][130] when nsplit > 1 (gp = padded group size)
+  void* out; float* part;  // part: [B][Hkv][nsplit][gp][130], gp = padded group size; NULL with nsplit > 1: the splits are a cluster
   int B, NBmax, Hq, Hkv, BS, nsplit, gp;
   int64_t kv_stride_page;
   float scale_log2e;
@@ -33,10 +36,9 @@ __global__ void __launch_bounds__(DM_THREADS) paged_decode_mma_kernel(const DmAr
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, tq = lane & 3;  // fragment row / column-pair index
   const int n = a.seqlens[b];
-  const int npages = (n + a.BS - 1) / a.BS;
-  const int pages_per_split = (npages + a.nsplit - 1) / a.nsplit;
-  const int k_begin = min(split * pages_per_split * a.BS, n);
-  const int k_end = min((split + 1) * pages_per_split * a.BS, n);
+  const int per = ((n + a.nsplit - 1) / a.nsplit + DM_TILE - 1) / DM_TILE * DM_TILE;   // whole tiles: page sizes are multiples of one
+  const int k_begin = min(split * per, n);
+  const int k_end = min(k_begin + per, n);
   const int32_t* table = a.table + (int64_t)b * a.NBmax;
   const char* kc = reinterpret_cast<const char*>(a.k);
   const char* vc = reinterpret_cast<const char*>(a.v);
@@ -163,6 +165,7 @@ __global__ void __launch_bounds__(DM_THREADS) paged_decode_mma_kernel(const DmAr
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
   __syncthreads();
   float* mbuf = reinterpret_cast<float*>(smem);  // [4 warps][16 rows][130]: O(128), m, l
+  float (*both)[130] = reinterpret_cast<float (*)[130]>(mbuf + 4 * 16 * 130);      // the block's [16 rows][130], for the other splits
   {
     float* w0 = mbuf + ((size_t)warp * 16 + g) * 130;
     float* w1 = w0 + 8 * 130;
@@ -187,7 +190,10 @@ __global__ void __launch_bounds__(DM_THREADS) paged_decode_mma_kernel(const DmAr
       num = fmaf(wgt, rr[d], num);
       den = fmaf(wgt, rr[129], den);
     }
-    if (a.nsplit == 1) {
+    if (a.nsplit > 1 && !a.part) {
+      both[row][d] = num;
+      if (d == 0) { both[row][128] = M; both[row][129] = den; }
+    } else if (a.nsplit == 1) {
       reinterpret_cast<T*>(a.out)[((int64_t)b * a.Hq + h * G + row) * 128 + d] =
           Elem<T>::from_f32(den > 0.f ? num / den : 0.f);
     } else {
@@ -196,40 +202,89 @@ __global__ void __launch_bounds__(DM_THREADS) paged_decode_mma_kernel(const DmAr
       if (d == 0) { pp[128] = M; pp[129] = den; }
     }
   }
+  if (a.nsplit == 1 || a.part) return;
+  // ---- merge the splits through distributed shared memory: each block finishes its part of the group's entries ----
+  cluster_sync();
+  for (int idx = split * DM_THREADS + tid; idx < G * 128; idx += a.nsplit * DM_THREADS) {
+    const int row = idx >> 7, d = idx & 127;
+    float m[DM_CLUSTER], M = -INFINITY, num = 0.f, den = 0.f;
+#pragma unroll
+    for (int s = 0; s < DM_CLUSTER; ++s)
+      if (s < a.nsplit) M = fmaxf(M, m[s] = ld_cluster(&both[row][128], s));
+#pragma unroll
+    for (int s = 0; s < DM_CLUSTER; ++s) {
+      if (s >= a.nsplit) break;
+      const float wgt = m[s] == -INFINITY ? 0.f : exp2f(m[s] - M);
+      num = fmaf(wgt, ld_cluster(&both[row][d], s), num);
+      den = fmaf(wgt, ld_cluster(&both[row][129], s), den);
+    }
+    reinterpret_cast<T*>(a.out)[((int64_t)b * a.Hq + h * G + row) * 128 + d] = Elem<T>::from_f32(den > 0.f ? num / den : 0.f);
+  }
+  cluster_sync();      // (a block's shared memory stays until the others have read it)
 }
 
+// A warp per query head.  The splits' maxima and sums are read by one lane each (at most 32 splits), so that their latency is
+// paid once; then every lane adds up four entries with the splits' loads in flight together.  (A block per key/value head that
+// walked its splits one after the other took 7.5 us for 4 sequences x 16 heads x 9 splits.)
 template <typename T>
-__global__ void decode_mma_merge_kernel(const DmArgs a) {
-  const int b = blockIdx.x, h = blockIdx.y;
-  const int G = a.Hq / a.Hkv;
-  for (int idx = threadIdx.x; idx < G * 128; idx += blockDim.x) {
-    const int row = idx >> 7, d = idx & 127;
-    const float* base = a.part + ((((int64_t)b * a.Hkv + h) * a.nsplit) * a.gp + row) * 130;
-    const int64_t sstride = (int64_t)a.gp * 130;
-    float M = -INFINITY;
-    for (int s = 0; s < a.nsplit; ++s) M = fmaxf(M, base[s * sstride + 128]);
-    float num = 0.f, den = 0.f;
-    for (int s = 0; s < a.nsplit; ++s) {
-      const float* rr = base + s * sstride;
-      const float w = rr[128] == -INFINITY ? 0.f : exp2f(rr[128] - M);
-      num = fmaf(w, rr[d], num);
-      den = fmaf(w, rr[129], den);
-    }
-    reinterpret_cast<T*>(a.out)[((int64_t)b * a.Hq + h * G + row) * 128 + d] =
-        Elem<T>::from_f32(den > 0.f ? num / den : 0.f);
+__global__ void __launch_bounds__(128) decode_mma_merge_kernel(const DmArgs a) {
+  const int b = blockIdx.x, hq = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (hq >= a.Hq) return;
+  const int G = a.Hq / a.Hkv, h = hq / G, row = hq % G;
+  const float* base = a.part + (((int64_t)b * a.Hkv + h) * a.nsplit * a.gp + row) * 130;
+  const int64_t pitch = (int64_t)a.gp * 130;
+  float m = -INFINITY, l = 0.f;
+  if (lane < a.nsplit) {
+    const float2 ml = *reinterpret_cast<const float2*>(base + lane * pitch + 128);
+    m = ml.x; l = ml.y;
+  }
+  const float M = warp_max(m);
+  const float w = m == -INFINITY ? 0.f : exp2f(m - M);
+  const float den = warp_sum(w * l);
+  float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int s = 0; s < a.nsplit; ++s) {
+    const float ws = __shfl_sync(0xffffffffu, w, s);
+    const float2* rr = reinterpret_cast<const float2*>(base + s * pitch + lane * 4);   // (rows of 130 floats: 8-byte aligned)
+    const float2 x = rr[0], y = rr[1];
+    num.x = fmaf(ws, x.x, num.x); num.y = fmaf(ws, x.y, num.y);
+    num.z = fmaf(ws, y.x, num.z); num.w = fmaf(ws, y.y, num.w);
+  }
+  const float inv = den > 0.f ? 1.f / den : 0.f;
+  T* out = reinterpret_cast<T*>(a.out) + ((int64_t)b * a.Hq + hq) * 128 + lane * 4;
+  const uint2 o = make_uint2(pack2<T>(num.x * inv, num.y * inv), pack2<T>(num.z * inv, num.w * inv));
+  if ((uintptr_t)a.out % 8 == 0) *reinterpret_cast<uint2*>(out) = o;
+  else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[i] = reinterpret_cast<const T*>(&o)[i];
   }
 }
 
 template <typename T>
 static int launch_decode_mma(const DmArgs& a, cudaStream_t st) {
-  const size_t smem = 2 * 2 * DM_TILE_BYTES;  // 64 KB (also holds the 4 x 16 x 130 float merge buffer)
+  const size_t smem = 2 * 2 * DM_TILE_BYTES;  // 64 KB (also holds the merge buffers, 5 x 16 x 130 floats)
   auto kern = paged_decode_mma_kernel<T>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) { set_error("zp_paged_decode: %s", cudaGetErrorString(e)); return ZP_ERR_CUDA; }
+  if (a.nsplit > 1 && !a.part) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.B, a.Hkv, a.nsplit);
+    cfg.blockDim = dim3(DM_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = attr.val.clusterDim.y = 1; attr.val.clusterDim.z = a.nsplit;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kern, a);
+    if (e != cudaSuccess) { set_error("zp_paged_decode: %s", cudaGetErrorString(e)); return ZP_ERR_CUDA; }
+    return check_launch("zp_paged_decode(mma, clusters)");
+  }
   kern<<<dim3(a.B, a.Hkv, a.nsplit), DM_THREADS, smem, st>>>(a);
   int rc = check_launch("zp_paged_decode(mma)");
   if (rc || a.nsplit == 1) return rc;
-  decode_mma_merge_kernel<T><<<dim3(a.B, a.Hkv), 128, 0, st>>>(a);
+  decode_mma_merge_kernel<T><<<dim3(a.B, (a.Hq + 3) / 4), 128, 0, st>>>(a);
   return check_launch("zp_paged_decode(mma) merge");
 }
 
