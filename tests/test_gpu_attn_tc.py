@@ -44,11 +44,89 @@ def test_prefill_edges(dtype, heads, kv_heads, lens_q, lens_k):
     q[:, 0] *= 6                                          # peaked rows, whose reference moves from tile to tile
     out = varlen_prefill_attention(q, k, v, max(lens_q), _cu(lens_q), max(lens_k), _cu(lens_k), impl="tcgen05")
     _no_device_error()
-    # the weight and the result are rounded to T once each (half a unit in the last place); the rest is fp32
-    unit = (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12) * 2 * 1.1
+    # weights and result are rounded to T once each, to 8 or 11 significant bits; the rest is fp32
+    unit = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * 1.1
     a = b = 0
     for x, y in zip(lens_q, lens_k):
         seen = torch.arange(y, device="cuda")[None] <= torch.arange(x, device="cuda")[:, None] + y - x
         ref, mag = _softmax(q[a:a + x], k[b:b + y], v[b:b + y], D ** -0.5, seen)
         assert ((out[a:a + x].double() - ref).abs() <= unit * 2 * mag + 1e-6).all()
+        a, b = a + x, b + y
+
+
+def _paged(rows, lens, page, table):
+    """rows [sum(lens), ...] on the pages of `table`; everything else holds NaN."""
+    cache = torch.full((int(table.max()) + 1, page, *rows.shape[1:]), float("nan"), dtype=rows.dtype, device="cuda")
+    at = 0
+    for b, n in enumerate(lens):
+        for i in range(0, n, page):
+            part = rows[at + i:at + min(n, i + page)]
+            cache[table[b, i // page], :len(part)] = part
+        at += n
+    return cache
+
+
+@pytest.mark.parametrize("many", [False, True])          # launches of few and of many query tiles take different kernels
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 2, 128, 128), (6, 2, 128, 128), (3, 3, 96, 40), (8, 2, 64, 64)])
+@pytest.mark.parametrize("window,softcap,keep,biased,chunk", [(0, 0.0, 0, False, 0), (130, 30.0, 0, False, 0), (200, 0.0, 70, True, 0), (0, 50.0, 0, False, 256)])
+def test_window_edges(many, heads, kv_heads, dim, vdim, window, softcap, keep, biased, chunk):
+    from zipage_b200.layers.attention import window_attention
+    copies = 1 + 710 // (10 * heads) if many else 1
+    lens_q, lens_k = [1, 129, 400, 250] * copies, [513, 129, 700, 251] * copies
+    g = torch.Generator(device="cuda").manual_seed(heads + dim)
+    n = lambda rows, h, d: torch.randn(rows, h, d, device="cuda", generator=g).to(torch.bfloat16)
+    q, k, v = n(sum(lens_q), heads, dim), n(sum(lens_k), kv_heads, dim), n(sum(lens_k), kv_heads, vdim)
+    pad = lambda t: torch.nn.functional.pad(t, (0, -t.shape[2] % 16))
+    need = [(m + 63) // 64 for m in lens_k]
+    ids, table = torch.randperm(sum(need), device="cuda", generator=g).to(torch.int32), torch.full((len(need), max(need)), -1, dtype=torch.int32, device="cuda")
+    for b, part in enumerate(ids.split(need)):
+        table[b, :need[b]] = part
+    kc, vc = _paged(pad(k), lens_k, 64, table), _paged(pad(v), lens_k, 64, table)
+    slopes = torch.rand(heads, device="cuda", generator=g) * 0.05 if biased else None
+    gate, sink = n(sum(lens_q), heads, 1)[..., 0].contiguous(), torch.randn(heads, device="cuda", generator=g)
+    out = window_attention(q.flatten(1), kc, vc, torch.tensor(lens_k, dtype=torch.int32, device="cuda"), table, heads, dim, vdim, dim ** -0.5, window,
+                           softcap, cu_seqlens_q=_cu(lens_q), max_seqlen_q=max(lens_q), impl="auto" if many else "tcgen05", chunk=chunk, keep=keep, slopes=slopes, sink=sink,
+                           gate=gate, gate_mode="head")
+    _no_device_error()
+    for i, (x, y) in enumerate(zip(lens_q, lens_k)):
+        a, b = sum(lens_q[:i]), sum(lens_k[:i])
+        if 4 <= i < len(lens_q) - 4:
+            continue
+        p, j = torch.arange(y - x, y, device="cuda")[:, None], torch.arange(y, device="cuda")[None]
+        seen = j <= p
+        if window:
+            seen &= (p - j < window) | (j < keep)
+        if chunk:
+            seen &= p // chunk == j // chunk
+        G = heads // kv_heads
+        kk, vv = k[b:b + y].double().repeat_interleave(G, 1), v[b:b + y].double().repeat_interleave(G, 1)
+        s = torch.einsum("thd,shd->hts", q[a:a + x].double(), kk) * dim ** -0.5
+        s = softcap * torch.tanh(s / softcap) if softcap else s
+        s = s - slopes.double()[:, None, None] * (p - j) if biased else s
+        s = torch.cat([s.masked_fill(~seen[None], float("-inf")), sink.double()[:, None, None].expand(-1, x, 1)], -1)
+        w = torch.softmax(s, -1)[..., :-1] * torch.sigmoid(gate[a:a + x].double()).T[..., None]
+        ref, mag = torch.einsum("hts,shd->thd", w, vv), torch.einsum("hts,shd->thd", w, vv.abs())
+        # one rounding of the result to 8 significant bits (at most 2^-8 of it); weights carry 16 bits, their exponents an fp32 rounding
+        assert ((out[a:a + x].view(x, heads, vdim).double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * mag + 1e-6).all()
+
+
+@pytest.mark.parametrize("many", [False, True])
+@pytest.mark.parametrize("dim,rot,vdim,rank", [(128, 64, 128, 512), (64, 0, 64, 64), (96, 32, 40, 64), (128, 128, 128, 128)])
+def test_latent_prefill_edges(many, dim, rot, vdim, rank):
+    from zipage_b200.layers.latent_attention import latent_prefill
+    copies = 16 if many else 1
+    heads, lens_q, lens_k = 3, [1, 127, 300, 513] * copies, [130, 127, 301, 900] * copies
+    g = torch.Generator(device="cuda").manual_seed(dim + rot)
+    n = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    rows, keys = sum(lens_q), sum(lens_k)
+    q, kv, lat = n(rows, heads * (dim + rot)), n(keys, heads * (dim + vdim)), n(keys, rank + rot)
+    out = torch.empty(rows, heads * vdim, dtype=torch.bfloat16, device="cuda")
+    latent_prefill(q, kv, lat, _cu(lens_q), _cu(lens_k), max(lens_q), out, heads, dim, rot, vdim, rank, (dim + rot) ** -0.5)
+    _no_device_error()
+    a = b = 0
+    for x, y in zip(lens_q, lens_k):
+        k = torch.cat([kv[b:b + y, :heads * dim].view(y, heads, dim), lat[b:b + y, None, rank:].expand(-1, heads, -1)], -1)
+        seen = torch.arange(y, device="cuda")[None] <= torch.arange(x, device="cuda")[:, None] + y - x
+        ref, mag = _softmax(q[a:a + x].view(x, heads, dim + rot), k, kv[b:b + y, heads * dim:].view(y, heads, vdim), (dim + rot) ** -0.5, seen)
+        assert ((out[a:a + x].view(x, heads, vdim).double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * mag + 1e-6).all()
         a, b = a + x, b + y

@@ -16,14 +16,21 @@
 // exponentials 1024 of the special-function unit, so neither may wait for the other; two tiles in flight hide the
 // softmax's latency, and as a thread owns a whole row no maximum or sum ever crosses threads.
 //
-// Roles (three warpgroups, one block per SM): warp 0 = TMA producer and TMEM owner, warp 1 = MMA issuer, warps 4-7 and 8-11 =
-// softmax of tile 0 and 1, which take over registers of the first group (a row's 128 scores stay in them).  The MMAs of one issuing thread run in order, so S_t of the next key tile may be issued
-// right behind the product that reads p from the same columns.  Shared memory: both query tiles, a ring of 16 KB key
-// blocks (128 keys x 64 entries), a ring of value tiles.
+// Roles (one block per SM): warp 0 = work, TMA loads and TMEM, warp 1 = products, from warp 4 on softmax, P::GROUPS groups of
+// four warps a tile (two split its columns), which take over registers of the first group.  One thread issues the
+// products of both tiles in turn, which keeps them half a step apart (with an issuer per tile they fell into step and
+// overlapped less: 2.43 ms at 1 x 16384).  Its MMAs run in order, so S_t of the next key tile is issued right behind the product that
+// reads p from the same columns.  A wait costs it some 200 clocks even where it is over, more than the MMAs behind it take
+// to issue: a key tile has one barrier, and the second tile does not wait for keys again.  Shared memory: both query
+// tiles, a ring of 16 KB key blocks (128 keys x 64 entries), a ring of value tiles.
+//
+// A block's instructions have to be fetched, some 16 clocks each the first time, so code is short where that costs
+// little: masks are bit tests in a loop of their own, the capped softmax is a loop over 32 columns.  (Uncapped scores stay in
+// registers: reloading them from TMEM 32 columns at a time took 2.59 ms at 1 x 16384.)
 //
 // Blocks stay: each takes over the grid's tiles that have not started yet (cluster launch control), so that the next
 // item's queries and keys arrive during the last softmax and the output of the item before.  The grid's order is
-// the order of the work: levels of equal length, the longest first.
+// the order of the work: levels of query tiles, the longest first.  (A launch of a few tiles has no pairs: see pick_mode.)
 // Every wait is bounded; after one that runs out the block raises the device error word and leaves.
 #pragma once
 #include "zp_tc.cuh"
@@ -33,20 +40,15 @@ namespace attn {
 
 using namespace tc;
 
-constexpr int THREADS = 384;
-constexpr int REGS_FEED = 72, REGS_SOFTMAX = 216;      // of 168 a thread at launch: 72 + 2 x 216 = 3 x 168
+// registers of the feeding group's threads and of the others': 72 + 2 x 216 = 3 x 168 at launch, 56 + 4 x 104 <= 5 x 96
+constexpr int threads_of(int groups) { return 128 + 256 * groups; }
+constexpr int feed_regs(int groups) { return groups == 1 ? 72 : 56; }
+constexpr int softmax_regs(int groups) { return groups == 1 ? 216 : 104; }
 constexpr int BLK = 16384;               // 128 rows x 64 elements x 2 bytes
-constexpr int MAXRING = 12;
+constexpr int NBAR = 8;                  // barriers of a ring, more than tiles in flight
 constexpr uint32_t O_COL = 256;          // TMEM columns: S_0 | S_1 | O_0 | O_1, 128 each
 constexpr int SLACK = 128;               // alignment padding that the launch provides for
 constexpr float LOG2E = 1.4426950408889634f;
-
-struct __align__(16) Shared {
-  uint4 work[2];                         // answers of cluster launch control
-  uint64_t wfull[2], wempty[2], qfull, qempty, kfull[MAXRING], kempty[MAXRING], vfull[MAXRING], vempty[MAXRING], sfull[2], pfull[2], pvdone[2];
-  uint32_t tmem_base;
-  int abort_flag;
-};
 
 // Two tiles of one sequence.
 struct Item {
@@ -55,11 +57,25 @@ struct Item {
   int keys;                              // keys of the sequence: rows past them are not read
   int n[2];                              // key tiles 0 .. n - 1 of each
   int kept, t0;                          // key tile j is number j < kept ? j : t0 + j - kept
+  bool real;                             // false: no more work
   __device__ __forceinline__ int most() const { return max(n[0], n[1]); }
-  __device__ __forceinline__ int last(int j) const { return j < n[1] ? 1 : 0; }      // the tiles that take part in step j: the later one, ...
-  __device__ __forceinline__ int first(int j) const { return j < n[0] ? 0 : 1; }     // ... and the earlier one
   __device__ __forceinline__ int key0(int j) const { return (j < kept ? j : t0 + j - kept) * 128; }
 };
+struct __align__(16) Shared {
+  uint4 work;                            // answer of cluster launch control
+  Item item[2];                          // what the producer found, for the other roles
+  uint64_t wfull, ifull[2], iempty[2], qfull, qempty, kfull[NBAR], kempty[NBAR], vfull[NBAR], vempty[NBAR], sfull[2], pfull[2][2], pvdone[2], lfull[2];
+  float sum[2][2][128];                  // row sums of the column halves of each tile
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+// How a kernel's tiles share items.
+enum { PAIR_HEADS = 0, PAIR_ROWS = 1, SINGLE = 2 };      // two heads of a key/value head, two row blocks of a head, no second tile
+__device__ __forceinline__ int level_rows(int mode) { return mode == PAIR_ROWS ? 256 : 128; }
+__device__ __forceinline__ int item_head(int mode, int x, int t) { return mode == PAIR_HEADS ? 2 * x + t : x; }
+__device__ __forceinline__ int item_row(int mode, int first, int t) { return mode == PAIR_ROWS ? first + t * 128 : first; }
+__device__ __forceinline__ int item_rows(int mode, int rows, int t) { return mode == SINGLE && t ? 0 : min(128, rows); }
 template <typename V> __device__ __forceinline__ V of_tile(const V (&a)[2], int t) { return t ? a[1] : a[0]; }      // (an index would put a in memory)
 struct Rings { int nbq, nbv, nk, nv; };  // 64-entry blocks of a query (key) row and of a value row; key blocks and value tiles in the rings
 
@@ -111,6 +127,15 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+  uint32_t x[16], y[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) { x[i] = r[i]; y[i] = r[16 + i]; }
+  tmem_st16(taddr, x);
+  tmem_st16(taddr + 16, y);
+}
+// the lowest n bits, n from below 0 to above 32
+__device__ __forceinline__ uint32_t low_bits(int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u; }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 // the same answer in all lanes of the warp
@@ -120,10 +145,13 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
 
 // What P has to bring:
 //   T                            element type;  SPLIT: weights as hi + lo (T = bf16);  MASKED: rows have a first visible key too
+//   GROUPS                       1, or 2 where the reference is fixed (halves of a row need no common maximum then)
 //   LAZY                         powers of two by which a score may exceed its row's reference;  CAPPED: the reference is fixed
 //   rings, error_word            members
 //   item(id, it)                 the work of block `id`; false: none
-//   load_q(dst, bar, it, t), load_k(dst, bar, it, key0, i), load_v(dst, bar, it, key0, i): TMA loads of one block each
+//   prefetch()                   of its tensor maps
+//   load_q(dst, bar, it, t)      TMA loads of a query tile;  Step(p, it, key0): where a key tile lies, and with it
+//   load_k(dst, bar, it, step, i), load_v(dst, bar, it, step, i): TMA loads of one block each
 //   Row(p, it, t, r)             one query row, with lim (last visible key) and, where MASKED, lo and keep (keys j < lo are not seen
 //                                unless j < keep), ref0 (first reference; -inf unless CAPPED), and
 //     scale()                    what a raw product is multiplied by to become the exponent of 2, or
@@ -133,8 +161,10 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
 //     entries(p, c, v)           (P::GATED) factors of 32 entries
 //   out(row, head, c), dv        address of entry c of a row, entries of a head
 template <class P>
-__global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_constant__ P p) {
+__global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const __grid_constant__ P p) {
   using T = typename P::T;
+  constexpr int GROUPS = P::GROUPS, COLS = 128 / GROUPS;      // columns of a group
+  static_assert(GROUPS == 1 || P::CAPPED, "one maximum per row");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* qbuf = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   if (qbuf - smem_raw > SLACK) {         // (no room for more padding)
@@ -148,16 +178,21 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
   const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&sh.wfull[i], 1); mbar_init(&sh.wempty[i], 10);
-      mbar_init(&sh.sfull[i], 1); mbar_init(&sh.pfull[i], 4); mbar_init(&sh.pvdone[i], 1);
+      mbar_init(&sh.ifull[i], 1); mbar_init(&sh.iempty[i], 1 + 8 * GROUPS);
+      mbar_init(&sh.sfull[i], 1); mbar_init(&sh.pvdone[i], 1); mbar_init(&sh.lfull[i], 8);
+      for (int u = 0; u < 2; ++u) mbar_init(&sh.pfull[i][u], 4);
     }
-    mbar_init(&sh.qfull, 1); mbar_init(&sh.qempty, 1);
-    for (int i = 0; i < g.nk; ++i) { mbar_init(&sh.kfull[i], 1); mbar_init(&sh.kempty[i], 1); }
-    for (int i = 0; i < g.nv; ++i) { mbar_init(&sh.vfull[i], 1); mbar_init(&sh.vempty[i], 1); }
+    mbar_init(&sh.wfull, 1); mbar_init(&sh.qfull, 1);
+    mbar_init(&sh.qempty, 1);
+    for (int i = 0; i < NBAR; ++i) {
+      mbar_init(&sh.kfull[i], 1); mbar_init(&sh.kempty[i], 1);
+      mbar_init(&sh.vfull[i], 1); mbar_init(&sh.vempty[i], 1);
+    }
     sh.abort_flag = 0;
     fence_mbar_init();
   }
   if (warp == 0) {
+    if (lane == 0) p.prefetch();
     tmem_alloc(&sh.tmem_base, 512);
     tmem_relinquish();
   }
@@ -166,228 +201,240 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
   fence_after_sync();
   const uint32_t tmem = sh.tmem_base;
   volatile int* abortp = &sh.abort_flag;
-  dim3 id(blockIdx.x, blockIdx.y, blockIdx.z);
-  Item it;
-
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_FEED));
-    if (warp == 0 && elect_one()) {
-      uint32_t kslot = 0, kround = 0, vslot = 0, vround = 0, nq = 0;
-      bool ok = true;
-      for (uint32_t w = 0; ok; ++w) {
-        ok = mbar_wait(&sh.wempty[w & 1], ((w >> 1) & 1) ^ 1, abortp, p.error_word, 821);
-        if (!ok) break;
-        ask_work(&sh.work[w & 1], &sh.wfull[w & 1]);
-        if (p.item(id, it) && it.most() > 0) {
-          ok = mbar_wait<true>(&sh.qempty, (nq & 1) ^ 1, abortp, p.error_word, 822);
-          if (!ok) break;
-          mbar_arrive_expect_tx(&sh.qfull, (uint32_t)(((it.n[0] > 0) + (it.n[1] > 0)) * g.nbq * BLK));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(feed_regs(GROUPS)));
+    if (warp == 0) {
+      if (elect_one()) {
+        // ---------------- work and loads ----------------
+        Item it;
+        dim3 id(blockIdx.x, blockIdx.y, blockIdx.z);
+        uint32_t tiles = 0, kslot = 0, vslot = 0, nq = 0, asked = 0;      // key (value) tiles so far, next block (tile) of the rings
+        uint32_t kfree = g.nk, kfreed = 0, vfreed = 0;                    // free key blocks, key and value tiles given back
+        bool ok = true;
+        ask_work(&sh.work, &sh.wfull);
+        // the next block of the grid; every answer that was asked for is waited for, and a refusal is the last one
+        auto next = [&]() -> bool {
+          ok = mbar_wait(&sh.wfull, asked & 1, abortp, p.error_word, 821);
+          ++asked;
+          if (!ok || !read_work(&sh.work, id)) return false;
+          ask_work(&sh.work, &sh.wfull);
+          return true;
+        };
+        it.real = true;
+        for (uint32_t w = 0; ok && it.real; ++w) {
+          it.real = p.item(id, it);
+          while (!it.real && next()) it.real = p.item(id, it);
+          if (!ok || !mbar_wait<true>(&sh.iempty[w & 1], ((w >> 1) & 1) ^ 1, abortp, p.error_word, 822)) break;
+          sh.item[w & 1] = it;
+          mbar_arrive(&sh.ifull[w & 1]);
+          if (!it.real) break;
+          if (it.most() > 0) {
+            ok = mbar_wait<true>(&sh.qempty, (nq & 1) ^ 1, abortp, p.error_word, 823);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&sh.qfull, (uint32_t)(((it.n[0] > 0) + (it.n[1] > 0)) * g.nbq * BLK));
 #pragma unroll
-          for (int t = 0; t < 2; ++t)
-            if (it.n[t] > 0) p.load_q(qbuf + t * g.nbq * BLK, &sh.qfull, it, t);
-          ++nq;
-          for (int j = 0; ok && j < it.most(); ++j) {
-            const int key0 = it.key0(j);
-            for (int i = 0; i < g.nbq; ++i) {
-              if (!mbar_wait<true>(&sh.kempty[kslot], (kround & 1) ^ 1, abortp, p.error_word, 823)) { ok = false; break; }
-              mbar_arrive_expect_tx(&sh.kfull[kslot], BLK);
-              p.load_k(kring + kslot * BLK, &sh.kfull[kslot], it, key0, i);
-              if (++kslot == (uint32_t)g.nk) { kslot = 0; ++kround; }
-            }
-            if (!ok || !mbar_wait<true>(&sh.vempty[vslot], (vround & 1) ^ 1, abortp, p.error_word, 824)) { ok = false; break; }
-            mbar_arrive_expect_tx(&sh.vfull[vslot], (uint32_t)(g.nbv * BLK));
-            for (int i = 0; i < g.nbv; ++i) p.load_v(vring + (vslot * g.nbv + i) * BLK, &sh.vfull[vslot], it, key0, i);
-            if (++vslot == (uint32_t)g.nv) { vslot = 0; ++vround; }
+            for (int t = 0; t < 2; ++t)
+              if (it.n[t] > 0) p.load_q(qbuf + t * g.nbq * BLK, &sh.qfull, it, t);
+            ++nq;
           }
-          if (!ok) break;
-        }
-        // (also after a refusal: the answer has to arrive before the block may end)
-        ok = mbar_wait(&sh.wfull[w & 1], (w >> 1) & 1, abortp, p.error_word, 825) && read_work(&sh.work[w & 1], id);
-        mbar_arrive(&sh.wempty[w & 1]);
-      }
-    }
-    if (warp == 1 && elect_one()) {
-      constexpr uint32_t ID_S = idesc_f16(UmmaFmt<T>::fmt, 128, 128);
-      const uint32_t id_o = idesc_f16(UmmaFmt<T>::fmt, 128, 64 * g.nbv) | (1u << 16);      // V is MN-major
-      const uint32_t q_addr = smem_u32(qbuf), k_addr = smem_u32(kring), v_addr = smem_u32(vring);
-      uint32_t cnt[2] = {0, 0}, kslot0 = 0, kround0 = 0, vslot = 0, vround = 0, nq = 0;      // (key blocks of step 0 of an item, value tile)
-      bool ok = true;
-      for (uint32_t w = 0; ok; ++w) {
-        if (p.item(id, it) && it.most() > 0) {
-          const int most = it.most();
-          ok = mbar_wait(&sh.qfull, nq & 1, abortp, p.error_word, 826);
-          ++nq;
-          uint32_t ks_[2] = {kslot0, kslot0}, kr_[2] = {kround0, kround0};      // where each tile is in the key ring
-          auto issue_s = [&](int t, int j) -> bool {
-            const bool release = t == it.last(j);
-            uint32_t s = ks_[t], r = kr_[t];
-            for (int i = 0; i < g.nbq; ++i) {
-              if (!mbar_wait(&sh.kfull[s], r & 1, abortp, p.error_word, 827)) return false;
-              fence_after_sync();
-              const uint64_t ad = smem_desc_sw128(q_addr + (t * g.nbq + i) * BLK), bd = smem_desc_sw128(k_addr + s * BLK);
-#pragma unroll
-              for (int k = 0; k < 4; ++k) umma_f16(tmem + t * 128, ad + 2u * k, bd + 2u * k, ID_S, (i | k) ? 1u : 0u);
-              if (release) umma_commit(&sh.kempty[s]);
-              if (++s == (uint32_t)g.nk) { s = 0; ++r; }
+          for (int j = 0; ok && j < it.most(); ++j, ++tiles) {
+            const typename P::Step step(p, it, it.key0(j));
+            uint64_t* bar = &sh.kfull[tiles % NBAR];
+            mbar_arrive_expect_tx(bar, (uint32_t)(g.nbq * BLK));
+            for (int i = 0; ok && i < g.nbq; ++i) {
+              if (kfree == 0) {                            // the oldest key tile's blocks
+                ok = mbar_wait<true>(&sh.kempty[kfreed % NBAR], (kfreed / NBAR) & 1, abortp, p.error_word, 824);
+                ++kfreed;
+                kfree += g.nbq;
+                if (!ok) break;
+              }
+              --kfree;
+              p.load_k(kring + kslot * BLK, bar, it, step, i);
+              if (++kslot == (uint32_t)g.nk) kslot = 0;
             }
-            ks_[t] = s; kr_[t] = r;
-            if (release) { kslot0 = s; kround0 = r; }
+            if (ok && tiles - vfreed == (uint32_t)g.nv) {
+              ok = mbar_wait<true>(&sh.vempty[vfreed % NBAR], (vfreed / NBAR) & 1, abortp, p.error_word, 825);
+              ++vfreed;
+            }
+            if (!ok) break;
+            bar = &sh.vfull[tiles % NBAR];
+            mbar_arrive_expect_tx(bar, (uint32_t)(g.nbv * BLK));
+            for (int i = 0; i < g.nbv; ++i) p.load_v(vring + (vslot * g.nbv + i) * BLK, bar, it, step, i);
+            if (++vslot == (uint32_t)g.nv) vslot = 0;
+          }
+          if (ok && !next()) it.real = false;
+          if (ok && !it.real) {                            // tell the others, and leave
+            ++w;
+            if (mbar_wait<true>(&sh.iempty[w & 1], ((w >> 1) & 1) ^ 1, abortp, p.error_word, 826)) {
+              sh.item[w & 1].real = false;
+              mbar_arrive(&sh.ifull[w & 1]);
+            }
+          }
+        }
+      }
+    } else if (warp == 1) {
+      if (elect_one()) {
+        // ---------------- products ----------------
+        constexpr uint32_t ID_S = idesc_f16(UmmaFmt<T>::fmt, 128, 128);
+        const uint32_t id_o = idesc_f16(UmmaFmt<T>::fmt, 128, 64 * g.nbv) | (1u << 16);      // V is MN-major
+        const uint32_t q_addr = smem_u32(qbuf), k_addr = smem_u32(kring), v_addr = smem_u32(vring);
+        uint32_t tiles = 0, cnt[2] = {0, 0}, kslot = 0, vslot = 0, nq = 0;      // key tiles of the items before, steps of each tile, places in the rings
+        bool ok = true;
+        for (uint32_t w = 0; ok; ++w) {
+          ok = mbar_wait(&sh.ifull[w & 1], (w >> 1) & 1, abortp, p.error_word, 827);
+          const int n[2] = {sh.item[w & 1].n[0], sh.item[w & 1].n[1]}, most = max(n[0], n[1]);
+          if (!ok || !sh.item[w & 1].real) break;
+          mbar_arrive(&sh.iempty[w & 1]);
+          if (most <= 0) continue;
+          ok = mbar_wait(&sh.qfull, nq & 1, abortp, p.error_word, 828);
+          ++nq;
+          // S of key tile j, whose blocks start at kslot; the last tile that reads it gives them back
+          auto issue_s = [&](int t, int j) {
+            const bool last = t == (j < n[1] ? 1 : 0);
+            uint32_t slot = kslot;
+#pragma unroll 1
+            for (int i = 0; i < g.nbq; ++i) {
+              const uint64_t ad = smem_desc_sw128(q_addr + (t * g.nbq + i) * BLK), bd = smem_desc_sw128(k_addr + slot * BLK);
+#pragma unroll
+              for (int c = 0; c < 4; ++c) umma_f16(tmem + t * 128, ad + 2u * c, bd + 2u * c, ID_S, (i | c) ? 1u : 0u);
+              if (++slot == (uint32_t)g.nk) slot = 0;
+            }
             umma_commit(&sh.sfull[t]);
-            if (j == most - 1 && release) umma_commit(&sh.qempty);
-            return true;
+            if (!last) return;
+            umma_commit(&sh.kempty[(tiles + j) % NBAR]);
+            kslot = slot;
+            if (j == most - 1) umma_commit(&sh.qempty);
           };
+          auto keys = [&](int j) -> bool {
+            const bool in = mbar_wait(&sh.kfull[(tiles + j) % NBAR], ((tiles + j) / NBAR) & 1, abortp, p.error_word, 829);
+            fence_after_sync();
+            return in;
+          };
+          ok = ok && keys(0);
 #pragma unroll
           for (int t = 0; t < 2; ++t)
-            if (ok && it.n[t] > 0) ok = issue_s(t, 0);
+            if (ok && n[t] > 0) issue_s(t, 0);
 #pragma unroll 1
           for (int j = 0; ok && j < most; ++j) {
+            const uint32_t k = tiles + j, v0 = v_addr + vslot * g.nbv * BLK;
+            ok = mbar_wait(&sh.vfull[k % NBAR], (k / NBAR) & 1, abortp, p.error_word, 830);
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
-              if (!ok || j >= it.n[t]) continue;
-              if (t == it.first(j)) ok = mbar_wait(&sh.vfull[vslot], vround & 1, abortp, p.error_word, 828);
-              if (!ok || !mbar_wait(&sh.pfull[t], cnt[t] & 1, abortp, p.error_word, 829)) { ok = false; continue; }
-              fence_after_sync();
-              const uint32_t v0 = v_addr + vslot * g.nbv * BLK, pt = tmem + t * 128, ot = tmem + O_COL + t * 128;
+              if (!ok || j >= n[t]) continue;
+              const uint32_t pt = tmem + t * 128, ot = tmem + O_COL + t * 128;
 #pragma unroll
-              for (int ks = 0; ks < 8; ++ks) {      // 16 keys a step: 8 columns of p
-                const uint64_t bd = desc_mn(v0 + ks * 2048);
-                umma_ts(ot, pt + ks * 8, bd, id_o, (j | ks) ? 1u : 0u);
-                if (P::SPLIT) umma_ts(ot, pt + 64 + ks * 8, bd, id_o, 1u);
+              for (int u = 0; u < 2; ++u) {                  // the softmax hands over 64 keys at a time
+                ok = ok && mbar_wait(&sh.pfull[t][u], cnt[t] & 1, abortp, p.error_word, 831);
+                if (!ok) continue;
+                fence_after_sync();
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {                // 16 keys a step: 8 columns of p
+                  const uint64_t bd = desc_mn(v0 + (4 * u + c) * 2048);
+                  const uint32_t a = pt + u * 64 + (c >> 1) * 32 + (c & 1) * 8;
+                  umma_ts(ot, a, bd, id_o, (j | u | c) ? 1u : 0u);
+                  if (P::SPLIT) umma_ts(ot, a + 16, bd, id_o, 1u);
+                }
               }
-              if (t == it.last(j)) umma_commit(&sh.vempty[vslot]);
-              umma_commit(&sh.pvdone[t]);
+              if (!ok) continue;
               ++cnt[t];
-              if (j + 1 < it.n[t]) ok = issue_s(t, j + 1);
+              if (j + 1 < n[t]) {                            // (behind the product that reads p from its columns)
+                if (t == 0 || j + 1 >= n[0]) ok = keys(j + 1);
+                if (ok) issue_s(t, j + 1);
+              }
+              umma_commit(&sh.pvdone[t]);
             }
-            if (++vslot == (uint32_t)g.nv) { vslot = 0; ++vround; }
+            if (ok) umma_commit(&sh.vempty[k % NBAR]);
+            if (++vslot == (uint32_t)g.nv) vslot = 0;
           }
-          if (!ok) break;
+          tiles += most;
         }
-        ok = mbar_wait(&sh.wfull[w & 1], (w >> 1) & 1, abortp, p.error_word, 830) && read_work(&sh.work[w & 1], id);
-        mbar_arrive(&sh.wempty[w & 1]);
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_SOFTMAX));
-    const int t = (warp - 4) >> 2, quad = warp & 3, r = quad * 32 + lane;      // tile, TMEM lane quadrant, row of the tile
+    // ---------------- softmax ----------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(softmax_regs(GROUPS)));
+    const int grp = (warp - 4) >> 2, t = grp / GROUPS, half = grp % GROUPS, quad = warp & 3;      // tile, its columns, TMEM lane quadrant
+    const int r = quad * 32 + lane;                                                              // row of the tile
     const uint32_t lanes = tmem + (static_cast<uint32_t>(quad * 32) << 16), st = lanes + t * 128, ot = lanes + O_COL + t * 128;
-    uint32_t cnt = 0, vslot = 0, vround = 0;
+    uint32_t tiles = 0, cnt = 0, ends = 0, vslot = 0;      // key tiles of the items before, steps and items of this tile, place in the value ring
     bool ok = true;
     for (uint32_t w = 0; ok; ++w) {
-      if (p.item(id, it)) {
-        const int n = of_tile(it.n, t), most = it.most();
-        const typename P::Row row(p, it, t, r);
-        float2 l2 = make_float2(0.f, 0.f);
-        float ref = row.ref0;
-        for (int j = 0; ok && j < n; ++j) {
-          const int key0 = it.key0(j);
-          ok = warp_wait(&sh.sfull[t], cnt & 1, abortp, p.error_word, 831);
-          if (!ok) break;
-          fence_after_sync();
-          uint32_t s[4][32];
+      ok = warp_wait(&sh.ifull[w & 1], (w >> 1) & 1, abortp, p.error_word, 832);
+      if (!ok || !sh.item[w & 1].real) break;
+      const Item it = sh.item[w & 1];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.iempty[w & 1]);
+      const int n = of_tile(it.n, t), most = it.most();
+      const typename P::Row row(p, it, t, r);
+      float2 l2 = make_float2(0.f, 0.f);
+      float ref = row.ref0;
+      // A block's first turn works on nothing (step -1: no waits, no stores): it fetches the loop's instructions while the first
+      // operands are on their way, which otherwise come one after the other behind them (5 to 11 thousand clocks).
+      for (int j = w == 0 ? -1 : 0; ok && j < n; ++j) {
+        const bool dry = j < 0;
+        const int key0 = it.key0(j) + half * COLS;      // first key of this group
+        if (!dry) ok = warp_wait(&sh.sfull[t], cnt & 1, abortp, p.error_word, 833);
+        if (!ok) break;
+        fence_after_sync();
+        bool whole = key0 + COLS - 1 <= row.lim;
+        if constexpr (P::MASKED) whole = whole && (key0 >= row.lo || key0 + COLS <= row.keep);
+        whole = __all_sync(0xffffffffu, whole || dry);
+        auto seen = [&](int key) -> uint32_t {          // of 32 keys
+          uint32_t m = low_bits(row.lim - key + 1);
+          if constexpr (P::MASKED) m &= ~low_bits(row.lo - key) | low_bits(row.keep - key);
+          return m;
+        };
+        // weights of 32 keys, over their scores: hi in the first 16 columns, lo in the others
+        auto weights = [&](uint32_t (&s)[32], int c, float mref) {
+          const uint32_t y = P::CAPPED && !whole ? seen(key0 + c) : 0xffffffffu, at = st + half * COLS + c;
+          uint32_t hi[16], lo[16];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) tmem_ld32_issue(st + c * 32, s[c]);
+          for (int i = 0; i < 32; i += 4) {
+            float wt[4];
+            if constexpr (P::CAPPED) {
+              row.weights4(&s[i], wt);
+              if (!whole) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) tmem_ld32_wait(s[c]);
-          bool whole = key0 + 127 <= row.lim;
-          if constexpr (P::MASKED) whole = whole && (key0 >= row.lo || key0 + 128 <= row.keep);
-          whole = __all_sync(0xffffffffu, whole);
-          if constexpr (P::BIASED) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) row.transform(s[c], key0 + c * 32);
-          }
-          if (!whole && !P::CAPPED) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-#pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                const int key = key0 + c * 32 + i;
-                bool seen = key <= row.lim;
-                if constexpr (P::MASKED) seen = seen && (key >= row.lo || key < row.keep);
-                if (!seen) s[c][i] = 0xff800000u;      // -inf
+                for (int u = 0; u < 4; ++u)
+                  if (!(y >> (i + u) & 1u)) wt[u] = 0.f;
               }
-          }
-          if constexpr (!P::CAPPED) {
-            float mx[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              mx[c] = fmaxf(__uint_as_float(s[c][0]), __uint_as_float(s[c][1]));
-#pragma unroll
-              for (int i = 2; i < 32; i += 2) mx[c] = fmax3(mx[c], __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
-            }
-            float m = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-            if constexpr (!P::BIASED) m *= row.scale();
-            const bool moves = m > ref + P::LAZY;
-            if (__any_sync(0xffffffffu, moves)) {
-              const float fac = moves ? ex2(ref - m) : 1.f;
-              if (moves) ref = m;
-              l2.x *= fac;
-              l2.y *= fac;
-              if (j > 0) {
-                ok = warp_wait(&sh.pvdone[t], (cnt & 1) ^ 1, abortp, p.error_word, 832);
-                if (!ok) break;
-                fence_after_sync();
-#pragma unroll 1
-                for (int c = 0; c < 4 * g.nbv; ++c) {
-                  uint32_t o[16];
-                  tmem_ld16(ot + c * 16, o);
-#pragma unroll
-                  for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * fac);
-                  tmem_st16(ot + c * 16, o);
-                }
-              }
-            }
-          }
-          const float mref = ref == -INFINITY ? 0.f : ref;      // (no key seen so far: every weight is exp2(-inf))
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t hi[16], lo[16];
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              float wt[4];
-              if constexpr (P::CAPPED) {
-                row.weights4(&s[c][i], wt);
-                if (!whole) {
-#pragma unroll
-                  for (int u = 0; u < 4; ++u) {
-                    const int key = key0 + c * 32 + i + u;
-                    bool seen = key <= row.lim;
-                    if constexpr (P::MASKED) seen = seen && (key >= row.lo || key < row.keep);
-                    if (!seen) wt[u] = 0.f;
-                  }
-                }
-              } else {
-                const float sc = P::BIASED ? 1.f : row.scale();
-#pragma unroll
-                for (int u = 0; u < 4; u += 2) {
-                  float2 x = make_float2(-mref, -mref);
-                  ffma2(x, make_float2(__uint_as_float(s[c][i + u]), __uint_as_float(s[c][i + u + 1])), make_float2(sc, sc));
-                  wt[u] = ex2(x.x);
-                  wt[u + 1] = ex2(x.y);
-                }
-              }
-              l2 = fadd2(l2, fadd2(make_float2(wt[0], wt[1]), make_float2(wt[2], wt[3])));
+            } else {
+              const float sc = P::BIASED ? 1.f : row.scale();
 #pragma unroll
               for (int u = 0; u < 4; u += 2) {
-                const typename Pair<T>::V x = Pair<T>::pack(wt[u], wt[u + 1]);
-                hi[(i + u) >> 1] = *reinterpret_cast<const uint32_t*>(&x);
-                if constexpr (P::SPLIT) {
-                  const float2 f = Pair<T>::unpack(x);
-                  const typename Pair<T>::V z = Pair<T>::pack(wt[u] - f.x, wt[u + 1] - f.y);
-                  lo[(i + u) >> 1] = *reinterpret_cast<const uint32_t*>(&z);
-                }
+                float2 x = make_float2(-mref, -mref);
+                ffma2(x, make_float2(__uint_as_float(s[i + u]), __uint_as_float(s[i + u + 1])), make_float2(sc, sc));
+                wt[u] = ex2(x.x);
+                wt[u + 1] = ex2(x.y);
               }
             }
-            tmem_st16(st + c * 16, hi);
-            if constexpr (P::SPLIT) tmem_st16(st + 64 + c * 16, lo);
+            l2 = fadd2(l2, fadd2(make_float2(wt[0], wt[1]), make_float2(wt[2], wt[3])));
+#pragma unroll
+            for (int u = 0; u < 4; u += 2) {
+              const typename Pair<T>::V x = Pair<T>::pack(wt[u], wt[u + 1]);
+              hi[(i + u) >> 1] = *reinterpret_cast<const uint32_t*>(&x);
+              if constexpr (P::SPLIT) {
+                const float2 f = Pair<T>::unpack(x);
+                const typename Pair<T>::V z = Pair<T>::pack(wt[u] - f.x, wt[u + 1] - f.y);
+                lo[(i + u) >> 1] = *reinterpret_cast<const uint32_t*>(&z);
+              }
+            }
           }
-          // value rows past the sequence become zeros (0 times another sequence's values could be NaN)
-          const int left = it.keys - key0;
-          if (left < 128 && t == it.first(j)) {
-            ok = warp_wait(&sh.vfull[vslot], vround & 1, abortp, p.error_word, 833);
-            if (!ok) break;
-            for (int i = r; i < (128 - left) * 8 * g.nbv; i += 128) {
-              const int line = i >> 3, blk = line / (128 - left), key = left + line % (128 - left);
+          if (dry) return;
+          tmem_st16(at, hi);
+          if constexpr (P::SPLIT) tmem_st16(at + 16, lo);
+        };
+        // 64 keys' weights are written.  Value rows past the sequence become zeros (0 times another sequence's values could be
+        // NaN): those that the product behind this hand-over reads, whichever tile's comes first
+        auto hand_over = [&](int u) {
+          if (dry) return;
+          const int left = max(it.keys - it.key0(j) - 64 * u, 0);
+          if (left < 64) {
+            const uint32_t k = tiles + j;
+            ok = warp_wait(&sh.vfull[k % NBAR], (k / NBAR) & 1, abortp, p.error_word, 835);
+#pragma unroll 1
+            for (int i = r; ok && i < (64 - left) * 8 * g.nbv; i += 128) {
+              const int line = i >> 3, blk = line / (64 - left), key = 64 * u + left + line % (64 - left);
               *reinterpret_cast<int4*>(vring + (vslot * g.nbv + blk) * BLK + key * 128 + ((i & 7) << 4)) = make_int4(0, 0, 0, 0);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -395,56 +442,133 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
           tmem_st_wait();
           fence_before_sync();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&sh.pfull[t]);
-          ++cnt;
-          if (++vslot == (uint32_t)g.nv) { vslot = 0; ++vround; }
-        }
-        if (!ok) break;
-        for (int j = n; j < most; ++j)
-          if (++vslot == (uint32_t)g.nv) { vslot = 0; ++vround; }
-        // ---- output: four lanes share a row's 64 bytes ----
-        if (n > 0) {
-          ok = warp_wait(&sh.pvdone[t], (cnt & 1) ^ 1, abortp, p.error_word, 834);
-          if (!ok) break;
-          fence_after_sync();
-        }
-        const float inv = row.finish(p, ref, l2.x + l2.y);
-        const int rows = of_tile(it.rows, t), q0 = of_tile(it.q0, t), head = of_tile(it.head, t), r4 = r & ~3, c8 = (lane & 3) * 8;
+          if (lane == 0) mbar_arrive(&sh.pfull[t][u]);
+        };
+        if constexpr (P::CAPPED) {
 #pragma unroll 1
-        for (int c = 0; c < 64 * g.nbv; c += 32) {
-          uint32_t o[32];
-          if (n > 0) {
-            tmem_ld32_issue(ot + c, o);
-            tmem_ld32_wait(o);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = 0u;
+          for (int c = 0; c < COLS; c += 32) {
+            uint32_t s[32];
+            tmem_ld32_issue(st + half * COLS + c, s);
+            tmem_ld32_wait(s);
+            weights(s, c, 0.f);
+            if (c & 32) hand_over((half * COLS + c) >> 6);
           }
-          float f[32];
+        } else {
+          if (!whole) {
+#pragma unroll 1
+            for (int c = 0; c < 128; c += 32) {
+              uint32_t s[32];
+              tmem_ld32_issue(st + c, s);
+              const uint32_t y = seen(key0 + c);
+              tmem_ld32_wait(s);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) f[i] = inv * __uint_as_float(o[i]);
-          if constexpr (P::GATED) row.entries(p, c, f);
-          int4 v[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint32_t x[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const typename Pair<T>::V y = Pair<T>::pack(f[8 * i + 2 * u], f[8 * i + 2 * u + 1]);
-              x[u] = *reinterpret_cast<const uint32_t*>(&y);
+              for (int i = 0; i < 32; ++i)
+                if (!(y >> i & 1u)) s[i] = 0xff800000u;      // -inf
+              tmem_st32(st + c, s);
             }
-            v[i] = make_int4((int)x[0], (int)x[1], (int)x[2], (int)x[3]);
+            tmem_st_wait();
           }
-          transpose4(v, lane);
+          uint32_t s[4][32];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (r4 + i < rows && c + c8 < p.dv) st16(p.out(q0 + r4 + i, head, c + c8), v[i]);
+          for (int c = 0; c < 4; ++c) tmem_ld32_issue(st + c * 32, s[c]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tmem_ld32_wait(s[c]);
+          float m[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if constexpr (P::BIASED) row.transform(s[c], key0 + c * 32);
+            m[c] = fmaxf(__uint_as_float(s[c][0]), __uint_as_float(s[c][1]));
+#pragma unroll
+            for (int i = 2; i < 32; i += 2) m[c] = fmax3(m[c], __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
+          }
+          m[0] = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+          if constexpr (!P::BIASED) m[0] *= row.scale();
+          const bool moves = !dry && m[0] > ref + P::LAZY;
+          if (__any_sync(0xffffffffu, moves)) {
+            const float fac = moves ? ex2(ref - m[0]) : 1.f;
+            if (moves) ref = m[0];
+            l2.x *= fac;
+            l2.y *= fac;
+            if (j > 0) {
+              ok = warp_wait(&sh.pvdone[t], (cnt & 1) ^ 1, abortp, p.error_word, 834);
+              if (!ok) break;
+              fence_after_sync();
+#pragma unroll 1
+              for (int c = 0; c < 64 * g.nbv; c += 16) {
+                uint32_t o[16];
+                tmem_ld16(ot + c, o);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * fac);
+                tmem_st16(ot + c, o);
+              }
+            }
+          }
+          const float mref = ref == -INFINITY ? 0.f : ref;      // (no key seen so far: every weight is exp2(-inf))
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            weights(s[c], c * 32, mref);
+            if (c & 1) hand_over(c >> 1);
+          }
         }
-        fence_before_sync();      // (the next item's first product into O follows this warp's next arrival)
+        if (dry) {
+          l2 = make_float2(0.f, 0.f);
+          continue;
+        }
+        ++cnt;
+        if (++vslot == (uint32_t)g.nv) vslot = 0;
       }
-      ok = warp_wait(&sh.wfull[w & 1], (w >> 1) & 1, abortp, p.error_word, 835) && read_work(&sh.work[w & 1], id);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sh.wempty[w & 1]);
+      if (!ok) break;
+      vslot = (vslot + most - n) % g.nv;
+      tiles += most;
+      // ---- output: four lanes share a row's 64 bytes ----
+      float l = l2.x + l2.y;
+      if (n > 0) {
+        ok = warp_wait(&sh.pvdone[t], (cnt & 1) ^ 1, abortp, p.error_word, 836);
+        if (!ok) break;
+        fence_after_sync();
+        if constexpr (GROUPS == 2) {      // (the halves' sums: both are past the item before, whose last product waited for both)
+          sh.sum[t][half][r] = l;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh.lfull[t]);
+          ok = warp_wait(&sh.lfull[t], ends & 1, abortp, p.error_word, 839);
+          if (!ok) break;
+          l = sh.sum[t][0][r] + sh.sum[t][1][r];
+          ++ends;
+        }
+      }
+      const float inv = row.finish(p, ref, l);
+      const int rows = of_tile(it.rows, t), q0 = of_tile(it.q0, t), head = of_tile(it.head, t), r4 = r & ~3, c8 = (lane & 3) * 8;
+#pragma unroll 1
+      for (int c = half * 32; c < 64 * g.nbv; c += 32 * GROUPS) {
+        uint32_t o[32];
+        if (n > 0) {
+          tmem_ld32_issue(ot + c, o);
+          tmem_ld32_wait(o);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = 0u;
+        }
+        float f[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) f[i] = inv * __uint_as_float(o[i]);
+        if constexpr (P::GATED) row.entries(p, c, f);
+        int4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t x[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const typename Pair<T>::V y = Pair<T>::pack(f[8 * i + 2 * u], f[8 * i + 2 * u + 1]);
+            x[u] = *reinterpret_cast<const uint32_t*>(&y);
+          }
+          v[i] = make_int4((int)x[0], (int)x[1], (int)x[2], (int)x[3]);
+        }
+        transpose4(v, lane);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (r4 + i < rows && c + c8 < p.dv) st16(p.out(q0 + r4 + i, head, c + c8), v[i]);
+      }
+      fence_before_sync();      // (the next item's first product into O follows this warp's next arrival)
     }
   }
   fence_before_sync();
@@ -458,12 +582,27 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tc_kernel(const __grid_consta
 // ---- host ----------------------------------------------------------------------------------------------
 // Rings for rows of nbq and nbv blocks: two value tiles (one where the queries take over half of the shared memory), the rest
 // key blocks.  With two key blocks a row that is three key tiles and two value tiles; with three, 4 key blocks and two value tiles.
+static_assert(14 * BLK + SLACK + sizeof(Shared) <= 232448, "14 blocks of operands");
 static inline Rings rings_of(int nbq, int nbv) {
   const int blocks = (232448 - SLACK - (int)sizeof(Shared)) / BLK - 2 * nbq;
   Rings g{nbq, nbv, 0, nbq > 3 ? 1 : 2};
   g.nk = blocks - g.nv * nbv;
-  if (g.nk > MAXRING) g.nk = MAXRING;
+  if (g.nk > (NBAR - 1) * nbq) g.nk = (NBAR - 1) * nbq;
   return g;
+}
+
+// Pairs, unless every tile can have an SM to itself (an estimate from the rows of all sequences: the counts are on the device): a
+// launch that short is one tile's latency, which the second tile of a pair only adds to.
+// Prompts, single tiles / pairs: 1 x 100 tokens, 32 heads: 10.3 / 12.1 us; 4 of up to 400, 8 heads: 20.3 / 22.1; 16 of up to 100,
+// 16 heads (about 256 tiles by this count): 51.5 / 32.5.
+static inline int pick_mode(int heads, int B, int total_q, bool heads_share, bool even) {
+  if ((int64_t)heads * (total_q / 128 + B) <= 148) return SINGLE;
+  return heads_share && even ? PAIR_HEADS : PAIR_ROWS;
+}
+static inline dim3 grid_of(int mode, int heads, int B, int max_q, int& levels) {
+  const int rows = mode == PAIR_ROWS ? 256 : 128;
+  levels = (max_q + rows - 1) / rows;
+  return dim3(mode == PAIR_HEADS ? heads / 2 : heads, B, levels);
 }
 
 template <class P>
@@ -471,7 +610,7 @@ static int launch_attn(const P& p, dim3 grid, cudaStream_t st, const char* what)
   const int smem = (2 * p.rings.nbq + p.rings.nk + p.rings.nv * p.rings.nbv) * BLK + (int)sizeof(Shared) + SLACK;
   cudaError_t e = cudaFuncSetAttribute(attn_tc_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) { set_error("%s: %s", what, cudaGetErrorString(e)); return ZP_ERR_CUDA; }
-  attn_tc_kernel<P><<<grid, THREADS, smem, st>>>(p);
+  attn_tc_kernel<P><<<grid, threads_of(P::GROUPS), smem, st>>>(p);
   return check_launch(what);
 }
 

@@ -16,6 +16,7 @@ using namespace attn;
 template <typename T_> struct PrefillTc {
   using T = T_;
   static constexpr bool SPLIT = false, MASKED = false, CAPPED = false, BIASED = false, GATED = false;
+  static constexpr int GROUPS = 1;
   // weights up to 2^LAZY: bf16 has fp32's range; fp16 ends at 2^16
   static constexpr float LAZY = UmmaFmt<T>::fmt == 1 ? 40.f : 12.f;
   CUtensorMap tmQ, tmK, tmV;
@@ -23,22 +24,26 @@ template <typename T_> struct PrefillTc {
   void* o;
   int* error_word;
   Rings rings;
-  int NBmax, Hq, Hkv, BS, levels, dv;
-  bool pair_heads;
+  int NBmax, Hq, Hkv, BS, levels, dv, mode;
   float scale_log2e;
 
+  __device__ __forceinline__ void prefetch() const {
+    prefetch_tensormap(&tmQ);
+    prefetch_tensormap(&tmK);
+    prefetch_tensormap(&tmV);
+  }
   __device__ __forceinline__ bool item(dim3 id, Item& it) const {
     const int b = id.y, level = levels - 1 - (int)id.z;
     const int q0 = cu_q[b], lq = cu_q[b + 1] - q0, lk = cu_k[b + 1] - cu_k[b];
-    const int first = level * (pair_heads ? 128 : 256);
+    const int first = level * level_rows(mode);
     if (first >= lq) return false;
     it.b = b;
     it.keys = lk;
     it.kept = it.t0 = 0;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-      const int qi = first + (pair_heads ? 0 : t * 128), rows = min(128, lq - qi);
-      it.head[t] = pair_heads ? 2 * (int)id.x + t : (int)id.x;
+      const int qi = item_row(mode, first, t), rows = item_rows(mode, lq - qi, t);
+      it.head[t] = item_head(mode, id.x, t);
       it.q0[t] = q0 + qi;
       it.rows[t] = rows;
       it.pos[t] = qi + lk - lq;
@@ -51,12 +56,17 @@ template <typename T_> struct PrefillTc {
   __device__ __forceinline__ void load_q(unsigned char* dst, uint64_t* bar, const Item& it, int t) const {
     for (int i = 0; i < 2; ++i) tma_load_5d(dst + i * BLK, &tmQ, bar, i * 64, it.head[t], it.q0[t], 0, 0);
   }
-  __device__ __forceinline__ void load_kv(unsigned char* dst, const CUtensorMap* tm, uint64_t* bar, const Item& it, int key0, int i) const {
-    if (table) tma_load_5d(dst, tm, bar, i * 64, it.hk, key0 % BS, table[(int64_t)it.b * NBmax + key0 / BS], 0);
-    else tma_load_5d(dst, tm, bar, i * 64, it.hk, cu_k[it.b] + key0, 0, 0);
+  struct Step {
+    int row, page;
+    __device__ __forceinline__ Step(const PrefillTc& p, const Item& it, int key0)
+        : row(p.table ? key0 % p.BS : p.cu_k[it.b] + key0), page(p.table ? p.table[(int64_t)it.b * p.NBmax + key0 / p.BS] : 0) {}
+  };
+  __device__ __forceinline__ void load_k(unsigned char* dst, uint64_t* bar, const Item& it, const Step& s, int i) const {
+    tma_load_5d(dst, &tmK, bar, i * 64, it.hk, s.row, s.page, 0);
   }
-  __device__ __forceinline__ void load_k(unsigned char* dst, uint64_t* bar, const Item& it, int key0, int i) const { load_kv(dst, &tmK, bar, it, key0, i); }
-  __device__ __forceinline__ void load_v(unsigned char* dst, uint64_t* bar, const Item& it, int key0, int i) const { load_kv(dst, &tmV, bar, it, key0, i); }
+  __device__ __forceinline__ void load_v(unsigned char* dst, uint64_t* bar, const Item& it, const Step& s, int i) const {
+    tma_load_5d(dst, &tmV, bar, i * 64, it.hk, s.row, s.page, 0);
+  }
   __device__ __forceinline__ T* out(int row, int head, int c) const { return reinterpret_cast<T*>(o) + ((int64_t)row * Hq + head) * 128 + c; }
 
   struct Row {
@@ -85,10 +95,9 @@ static int launch_prefill_tc(const void* q, const void* k, const void* v, Prefil
   if (int rc = make_tensor_map_5d(&p.tmV, UmmaFmt<T>::tm, v, dims, strides, box, sizeof(T))) return rc;
   p.rings = rings_of(2, 2);
   p.dv = 128;
-  p.pair_heads = p.Hq / p.Hkv % 2 == 0;
-  const int tile = p.pair_heads ? 128 : 256;
-  p.levels = (max_seqlen_q + tile - 1) / tile;
-  return launch_attn(p, dim3(p.pair_heads ? p.Hq / 2 : p.Hq, B, p.levels), st, "zp_varlen_prefill(tcgen05)");
+  p.mode = pick_mode(p.Hq, B, total_q, true, p.Hq / p.Hkv % 2 == 0);
+  const dim3 grid = grid_of(p.mode, p.Hq, B, max_seqlen_q, p.levels);
+  return launch_attn(p, grid, st, "zp_varlen_prefill(tcgen05)");
 }
 
 // Called by zp_varlen_prefill_ex (zp_prefill.cu).
