@@ -125,6 +125,26 @@ __device__ __forceinline__ float ld_cluster(const float* p, uint32_t rank) {
 }
 
 // 16-byte vector copy helpers
+// ---- kernels that begin while the one before them ends ----------------------------------------------
+// A kernel launched by `launch_early` may start as soon as every block of the kernel before it on the stream has called
+// `let_next_begin` or is done.  All of its threads call `wait_for_previous` first: before it, nothing may be read that an
+// earlier kernel writes, and nothing written; and what earlier kernels wrote is not read through the read-only path (no
+// __restrict__ const pointers).  `let_next_begin` comes after the wait, so at most two kernels of a stream overlap, and
+// a kernel launched the ordinary way still waits for everything before it.  It hides the launch and the first latencies of a
+// step's small kernels: a step of 4 sequences and 4 layers as a graph 197 -> 176 us, a step's attention for 192 sequences 285 -> 282.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+static inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 __device__ __forceinline__ int4 ld16(const void* p) { return *reinterpret_cast<const int4*>(p); }
 __device__ __forceinline__ void st16(void* p, int4 v) { *reinterpret_cast<int4*>(p) = v; }
 

@@ -35,6 +35,8 @@ __global__ void __launch_bounds__(DM_THREADS) paged_decode_mma_kernel(const DmAr
   const int G = a.Hq / a.Hkv;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, tq = lane & 3;  // fragment row / column-pair index
+  wait_for_previous();
+  let_next_begin();
   const int n = a.seqlens[b];
   const int per = ((n + a.nsplit - 1) / a.nsplit + DM_TILE - 1) / DM_TILE * DM_TILE;   // whole tiles: page sizes are multiples of one
   const int k_begin = min(split * per, n);
@@ -272,16 +274,18 @@ static int launch_decode_mma(const DmArgs& a, cudaStream_t st) {
     cfg.blockDim = dim3(DM_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = attr.val.clusterDim.y = 1; attr.val.clusterDim.z = a.nsplit;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = a.nsplit;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     e = cudaLaunchKernelEx(&cfg, kern, a);
     if (e != cudaSuccess) { set_error("zp_paged_decode: %s", cudaGetErrorString(e)); return ZP_ERR_CUDA; }
     return check_launch("zp_paged_decode(mma, clusters)");
   }
-  kern<<<dim3(a.B, a.Hkv, a.nsplit), DM_THREADS, smem, st>>>(a);
+  launch_early(kern, dim3(a.B, a.Hkv, a.nsplit), DM_THREADS, smem, st, a);
   int rc = check_launch("zp_paged_decode(mma)");
   if (rc || a.nsplit == 1) return rc;
   decode_mma_merge_kernel<T><<<dim3(a.B, (a.Hq + 3) / 4), 128, 0, st>>>(a);

@@ -58,7 +58,7 @@ template <typename T> struct Vec16 {   // one 16-byte vector of T
 // ---------------------------------------------------------------------------------------------
 template <typename T, int VPT>
 __global__ void __launch_bounds__(256)
-rms_norm_kernel(const T* x, const T* residual, const T* __restrict__ weight,
+rms_norm_kernel(const T* x, const T* residual, const T* weight,
                 T* out, T* residual_out, int H, int64_t x_stride, int64_t out_stride, float eps) {
   __shared__ float red[32];
   constexpr int EPV = Vec16<T>::N;
@@ -68,6 +68,8 @@ rms_norm_kernel(const T* x, const T* residual, const T* __restrict__ weight,
   const int nvec = H / EPV;
   float s[VPT][EPV];
   float ss = 0.f;
+  wait_for_previous();
+  let_next_begin();
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int v = threadIdx.x + i * 256;
@@ -124,7 +126,9 @@ __device__ __forceinline__ float silu_f32(float g) {
 // 8192 rows of 12288, bf16: 88 us = 6.9 TB/s (a grid-stride loop with 64-bit indices 119).
 template <typename T, typename Index>
 __global__ void __launch_bounds__(256)
-silu_and_mul_kernel(const T* __restrict__ x, T* __restrict__ out, int I, Index total_vec) {
+silu_and_mul_kernel(const T* x, T* out, int I, Index total_vec) {
+  wait_for_previous();
+  let_next_begin();
   constexpr int EPV = Vec16<T>::N;
   const Index vec_per_row = I / EPV, v0 = (Index)blockIdx.x * 512 + threadIdx.x;
   Vec16<T> a[2], b[2];
@@ -238,6 +242,8 @@ __global__ void __launch_bounds__(256) qk_norm_rope_store_kernel(const QkArgs a)
   const int lane = threadIdx.x & 31, l8 = lane & 7, hg = lane >> 3;   // 4 heads per warp at a time
   const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), part = blockIdx.y;
   const bool is_q = part < a.nq, is_v = part >= a.nq + a.nk, window = item >= a.n_tokens;
+  wait_for_previous();
+  let_next_begin();
   if (item >= a.n_tokens + a.n_triples || (window && !is_q)) return;
   int n = item, qid = 0, idx = 0;
   if (window) {
@@ -613,10 +619,10 @@ extern "C" int zp_rms_norm(const void* x, const void* residual, const void* weig
   ZP_DISPATCH_DTYPE(dtype, T, {
     const T* xp = (const T*)x; const T* rp = (const T*)residual; const T* wp = (const T*)weight;
     T* op = (T*)out; T* rop = (T*)residual_out;
-    if (nvec <= 256) zp::rms_norm_kernel<T, 1><<<n_rows, 256, 0, st>>>(xp, rp, wp, op, rop, hidden, x_stride, out_stride, eps);
-    else if (nvec <= 512) zp::rms_norm_kernel<T, 2><<<n_rows, 256, 0, st>>>(xp, rp, wp, op, rop, hidden, x_stride, out_stride, eps);
-    else if (nvec <= 1024) zp::rms_norm_kernel<T, 4><<<n_rows, 256, 0, st>>>(xp, rp, wp, op, rop, hidden, x_stride, out_stride, eps);
-    else zp::rms_norm_kernel<T, 8><<<n_rows, 256, 0, st>>>(xp, rp, wp, op, rop, hidden, x_stride, out_stride, eps);
+    if (nvec <= 256) zp::launch_early(zp::rms_norm_kernel<T, 1>, dim3(n_rows), 256, 0, st, xp, rp, wp, op, rop, hidden, x_stride, out_stride, eps);
+    else if (nvec <= 512) zp::launch_early(zp::rms_norm_kernel<T, 2>, dim3(n_rows), 256, 0, st, xp, rp, wp, op, rop, hidden, x_stride, out_stride, eps);
+    else if (nvec <= 1024) zp::launch_early(zp::rms_norm_kernel<T, 4>, dim3(n_rows), 256, 0, st, xp, rp, wp, op, rop, hidden, x_stride, out_stride, eps);
+    else zp::launch_early(zp::rms_norm_kernel<T, 8>, dim3(n_rows), 256, 0, st, xp, rp, wp, op, rop, hidden, x_stride, out_stride, eps);
   });
   return zp::check_launch("zp_rms_norm");
 }
@@ -633,9 +639,9 @@ extern "C" int zp_silu_and_mul(const void* x, void* out, int n_rows, int inter, 
   ZP_REQUIRE(blocks <= 0x7fffffff, "zp_silu_and_mul: too many rows");
   ZP_DISPATCH_DTYPE(dtype, T, {
     if (total_vec < (1ll << 31))
-      zp::silu_and_mul_kernel<T, uint32_t><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const T*)x, (T*)out, inter, (uint32_t)total_vec);
+      zp::launch_early(zp::silu_and_mul_kernel<T, uint32_t>, dim3((unsigned)blocks), 256, 0, (cudaStream_t)stream, (const T*)x, (T*)out, inter, (uint32_t)total_vec);
     else
-      zp::silu_and_mul_kernel<T, int64_t><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const T*)x, (T*)out, inter, total_vec);
+      zp::launch_early(zp::silu_and_mul_kernel<T, int64_t>, dim3((unsigned)blocks), 256, 0, (cudaStream_t)stream, (const T*)x, (T*)out, inter, total_vec);
   });
   return zp::check_launch("zp_silu_and_mul");
 }
@@ -676,8 +682,8 @@ extern "C" int zp_qk_norm_rope_store(const void* qkv, const int64_t* positions, 
   a.nk = (Hkv + a.per - 1) / a.per;
   const dim3 grid((n_tokens + n_triples + 7) / 8, a.nq + 2 * a.nk);   // eight warps per block, one token each
   ZP_DISPATCH_DTYPE(dtype, T, {
-    if (D == 128) zp::qk_norm_rope_store_kernel<T, 128><<<grid, 256, 0, st>>>(a);
-    else zp::qk_norm_rope_store_kernel<T, 64><<<grid, 256, 0, st>>>(a);
+    if (D == 128) zp::launch_early(zp::qk_norm_rope_store_kernel<T, 128>, grid, 256, 0, st, a);
+    else zp::launch_early(zp::qk_norm_rope_store_kernel<T, 64>, grid, 256, 0, st, a);
   });
   return zp::check_launch("zp_qk_norm_rope_store");
 }
