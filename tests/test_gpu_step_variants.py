@@ -71,6 +71,39 @@ def test_sampler_takes_the_best_of_all_draws(dtype, rows, V, spread):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows", [1, 2, 7, 8])
+@pytest.mark.parametrize("n_out,k,bias", [(16, 32, False), (40, 96, True), (1000, 1024, True), (256, 2048 + 32, False)])
+def test_small_linear(dtype, rows, n_out, k, bias):
+    from zipage_b200.layers.step_ops import linear
+    g = _gen(rows + k)
+    layer = torch.nn.Linear(k, n_out, bias=bias, device="cuda", dtype=dtype)
+    x = torch.randn(rows, 2 * k, device="cuda", generator=g).to(dtype)[:, :k]      # (a column view)
+    with torch.no_grad():
+        out = linear(layer, x)
+        w, b = layer.weight.double(), layer.bias.double() if bias else 0.0
+    ref, mag = x.double() @ w.T + b, x.double().abs() @ w.abs().T
+    # fp32 sums of k products, then one rounding to 8 or 11 significant bits
+    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert ((out.double() - ref).abs() <= unit * ref.abs() + 2.0 ** -24 * k * mag + 1e-7).all()
+
+
+def test_linear_leaves_the_rest_to_the_layer():
+    from zipage_b200 import kernel as K
+    from zipage_b200.layers.step_ops import SMALL_ROWS, linear
+    layer = torch.nn.Linear(64, 48, device="cuda", dtype=torch.bfloat16)
+    x = torch.randn(SMALL_ROWS + 1, 64, device="cuda", dtype=torch.bfloat16)
+    before = K.LAUNCHES
+    y = linear(layer, x[:4])                          # gradients wanted
+    assert y.requires_grad
+    with torch.no_grad():
+        assert torch.equal(linear(layer, x), layer(x))
+        handle = layer.register_forward_hook(lambda m, i, o: o * 0)
+        assert not linear(layer, x[:4]).any()
+        handle.remove()
+    assert K.LAUNCHES == before
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("B,heads,kv_heads,width", [(1, 8, 8, 16), (2, 16, 1, 9), (5, 32, 8, 16), (3, 4, 2, 17), (70, 8, 1, 4)])
 def test_paged_decode_splits(dtype, B, heads, kv_heads, width):
     """Short tables split within a cluster, longer ones (17 pages) through scratch."""
@@ -92,3 +125,70 @@ def test_paged_decode_splits(dtype, B, heads, kv_heads, width):
         w = torch.softmax(torch.einsum("hd,shd->hs", q[b, 0].double(), k) * D ** -0.5, -1)
         ref, mag = torch.einsum("hs,shd->hd", w, v), torch.einsum("hs,shd->hd", w, v.abs())
         assert ((out[b, 0].double() - ref).abs() <= 2 * unit * mag + 1e-6).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("q_rank,R,rot,heads,dim", [(2048, 1024, 64, 5, 8), (2056, 1024, 64, 1, 128), (8, 8, 8, 33, 64), (1536, 512, 24, 16, 0)])
+def test_latent_rows_in_vectors(dtype, q_rank, R, rot, heads, dim):
+    from zipage_b200.layers.latent_attention import latent_prepare, latent_rotate_q, rotary_turns
+    g, N, KP = _gen(q_rank + rot), 13, (R + rot + 15) // 16 * 16
+    n = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    y, wq, wk = n(N, q_rank + R + rot).to(dtype), n(q_rank), n(R)
+    pos, turns = torch.arange(N, device="cuda") * 4099, rotary_turns(rot, 10000.0, "cuda")
+    cache, dense = torch.zeros(1, 16, 1, KP, dtype=dtype, device="cuda"), torch.full((N, KP), 7.0, dtype=dtype, device="cuda")
+    slots = torch.arange(N, dtype=torch.int32, device="cuda")
+    cq = latent_prepare(y, pos, turns, wq, wk, cache, slots, q_rank, R, rot, 1e-5, dense)
+    norm = lambda x, w: x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5) * w.double()
+    angle = pos[:, None].double() * 10000.0 ** (-torch.arange(0, rot, 2, device="cuda").double() / rot)
+    c, s = angle.cos(), angle.sin()
+
+    def turn(x):
+        a, b = x[..., ::2].double(), x[..., 1::2].double()
+        cc, ss = (c, s) if x.dim() == 2 else (c[:, None], s[:, None])
+        return torch.stack([a * cc - b * ss, a * ss + b * cc], -1).flatten(-2)
+
+    # one rounding to T (half a unit in the last place) and fp32 arithmetic before it, also where a rotation's two parts cancel
+    close = lambda got, want: ((got.double() - want).abs() <= torch.finfo(dtype).eps / 2 * want.abs() + 4e-6).all()
+    assert close(cq, norm(y[:, :q_rank], wq))
+    want = torch.cat([norm(y[:, q_rank:q_rank + R], wk), turn(y[:, q_rank + R:])], -1)
+    assert close(dense[:, :R + rot], want) and (dense[:, R + rot:] == 0).all() and torch.equal(cache.view(16, KP)[:N], dense)
+    q = n(N, heads * (dim + rot)).to(dtype)
+    want, ql = turn(q.view(N, heads, -1)[..., dim:]), torch.full((N, heads, KP), 7.0, dtype=dtype, device="cuda")
+    latent_rotate_q(q, pos, turns, heads, dim, rot, ql, R)
+    assert close(ql[..., R:R + rot], want) and (ql[..., R + rot:] == 0).all() and (ql[..., :R] == 7).all()
+    before = q.clone()
+    latent_rotate_q(q, pos, turns, heads, dim, rot)
+    assert close(q.view(N, heads, -1)[..., dim:], want) and torch.equal(q.view(N, heads, -1)[..., :dim], before.view(N, heads, -1)[..., :dim])
+
+
+@pytest.mark.parametrize("rows,width", [(1, 256), (4, 1024), (8, 2048)])
+def test_kernels_that_begin_early_see_what_came_before(rows, width):
+    from zipage_b200.layers.step_ops import linear, rms_norm, silu_and_mul
+    g = _gen(width)
+    n = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    x0, r0, norm, ws = n(rows, width), n(rows, width), n(width), [n(2 * width, width) * width ** -0.5 for _ in range(2)]
+    layer = torch.nn.Linear(width, 2 * width, bias=False, device="cuda", dtype=torch.bfloat16)
+    x, r = x0.clone(), r0.clone()
+
+    @torch.no_grad()
+    def chain(after):
+        x.copy_(x0), r.copy_(r0)
+        for i in range(30):
+            layer.weight.copy_(ws[i % 2]), after()          # the weight changes right before it is read
+            h, rr = rms_norm(x, norm, 1e-5, r)
+            after()
+            y = linear(layer, h)
+            after()
+            x.copy_(silu_and_mul(y)) if i % 3 else x.copy_(rms_norm(silu_and_mul(y), norm, 1e-5))
+            r.copy_(rr), after()
+        return torch.cat([x, r])
+
+    want = chain(torch.cuda.synchronize).clone()
+    assert want.isfinite().all()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = chain(lambda: None)
+    for _ in range(5):
+        assert torch.equal(chain(lambda: None), want)
+        graph.replay()
+        assert torch.equal(out, want)

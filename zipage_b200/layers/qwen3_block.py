@@ -2,7 +2,7 @@
 
 Same module tree and forward contracts as third_party/nanovllm/models/qwen3.py:14-170
 (`Qwen3Attention`, `Qwen3MLP`, `Qwen3DecoderLayer`, `Qwen3Model`): the projections are plain
-`nn.Linear` (cuBLAS), everything between them is one of this library's kernels.  In
+`nn.Linear` (cuBLAS; the few rows of a small decode step: this library's), everything between them is one of this library's kernels.  In
 `Qwen3Attention.forward` the q/k head normalisation, the rotation and the two cache writes
 (qwen3.py:75-79 and zipage/layers/attention.py:72-77) are one launch, so `Attention.attend` is
 called instead of `Attention.forward`.
@@ -20,7 +20,7 @@ from torch import nn
 
 from ..utils.context import get_context
 from .attention import Attention
-from .step_ops import RMSNorm, SiluAndMul, qk_norm_rope_store, rope_cos_sin_cache
+from .step_ops import RMSNorm, SiluAndMul, linear, qk_norm_rope_store, rope_cos_sin_cache
 
 
 def reduce_add_norm(comm, norm, partial, residual):
@@ -52,7 +52,7 @@ class Qwen3Attention(nn.Module):
         self.k_norm = RMSNorm(self.head_dim, eps=rms_norm_eps)
 
     def forward(self, positions, hidden_states):
-        qkv = self.qkv_proj(hidden_states)
+        qkv = linear(self.qkv_proj, hidden_states)
         if self._cos_sin is None or self._cos_sin.device != qkv.device:
             self._cos_sin = rope_cos_sin_cache(self.head_dim, self.max_position, self.rope_theta, qkv.device)
         context = get_context()
@@ -69,7 +69,7 @@ class Qwen3Attention(nn.Module):
             return_k=context.is_prefill and context.block_tables is None,
             query_slot_count=context.query_slot_count if have_q else None)
         o = attn.attend(q, k, v)
-        return self.o_proj(o.flatten(1, -1))
+        return linear(self.o_proj, o.flatten(1, -1))
 
 
 class Qwen3MLP(nn.Module):
@@ -84,7 +84,7 @@ class Qwen3MLP(nn.Module):
         self.act_fn = SiluAndMul()
 
     def forward(self, x):
-        return self.down_proj(self.act_fn(self.gate_up_proj(x)))
+        return linear(self.down_proj, self.act_fn(linear(self.gate_up_proj, x)))
 
 
 class Qwen3DecoderLayer(nn.Module):

@@ -50,6 +50,30 @@ class RMSNorm(nn.Module):
         return rms_norm(x, self.weight, self.eps, residual)
 
 
+# Rows, and entries of the weight, up to which `linear` takes this library's kernel.  At 8 rows it takes 0.55 to 0.8 of cuBLAS's time
+# for weights of up to 2^23 entries (2048 x 1024: 2.7 us for 4.8; 6144 x 1024: 4.2 for 5.2); larger weights go either way
+# (8192 x 2048: 7.9 for 8.0; 5120 x 2048: 7.1 for 6.5; 12288 x 4096: 26 for 19), and so do 9 to 32 rows (4096 x 4096: 11.4 for 9.5).
+SMALL_ROWS, SMALL_WEIGHT = 8, 1 << 23
+
+
+def linear(layer, x):
+    """layer(x) for an nn.Linear: the few rows of a small decode step through `zp_small_linear`, everything else
+    (more rows, fp32, odd sizes, gradients, subclasses, hooks) through the layer itself."""
+    w, b = layer.weight, layer.bias
+    if (type(layer) is nn.Linear and type(x) is torch.Tensor and type(w) is nn.Parameter and x.dim() == 2 and 0 < x.shape[0] <= SMALL_ROWS
+            and w.numel() <= SMALL_WEIGHT and x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype
+            and w.device == x.device and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 8 == 0 and w.shape[1] % 32 == 0
+            and (w.data_ptr() | x.data_ptr()) % 16 == 0 and (b is None or b.dtype == x.dtype and b.is_contiguous())
+            and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda")
+            and not (layer._forward_hooks or layer._forward_pre_hooks or nn.modules.module._has_any_global_hook())):
+        out = torch.empty((x.shape[0], w.shape[0]), dtype=x.dtype, device=x.device)
+        L.check(L.load().zp_small_linear(L.ptr(x), x.stride(0), L.ptr(w), L.ptr(b), L.ptr(out), x.shape[0], w.shape[0], w.shape[1],
+                                         L.dtype_code(x), L.stream_ptr()), "small_linear")
+        _count(1)
+        return out
+    return layer(x)
+
+
 def silu_and_mul(x):
     L.require_cuda(x)
     two_i = x.shape[-1]
