@@ -326,6 +326,13 @@ int zp_qk_norm_rope_store(const void* qkv, const int64_t* positions, const float
 int zp_sample(const void* logits, const float* temperatures, const float* noise,
               int64_t* tokens_out, int n_rows, int vocab, uint64_t seed, int dtype, void* stream);
 
+/* Rows 0 .. n of input_ids (int64), num_tokens, query_ids and block_tables [n, width] (row stride given) into the buffers that a captured
+ * decode step reads: [max_n] and [max_n, max_width] contiguous.  Past n and width num_tokens becomes 0, query_ids and tables -1;
+ * input_ids keep what they hold.  (What model_runner.py:709-724 copies into the captured graph's variables.) */
+int zp_decode_inputs(const int64_t* input_ids, const int32_t* num_tokens, const int32_t* block_tables, int64_t table_stride,
+                     const int32_t* query_ids, int n, int width, int64_t* input_ids_out, int32_t* num_tokens_out,
+                     int32_t* block_tables_out, int32_t* query_ids_out, int max_n, int max_width, void* stream);
+
 /* Replaces the host loop of ModelRunner.prepare_decode, zipage/engine/model_runner.py:633-675
  * (with get_query_slot_mapping, :319-350), from device-resident state, so that a decode step
  * needs no host-built lists: num_tokens [B] (len(seq)), block_tables [B, table_width] (-1 padded,

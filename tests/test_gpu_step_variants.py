@@ -12,7 +12,7 @@ def _gen(seed):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("heads,kv_heads,D", [(32, 8, 128), (5, 1, 128), (18, 6, 64)])
 def test_qk_norm_rope_is_the_same_for_few_and_many_tokens(dtype, heads, kv_heads, D):
-    """1100 tokens in one call (16 heads a warp) and in halves (four heads a warp): the same arithmetic, the same bits."""
+    """1100 tokens in one call (32 heads a warp) and in halves (four heads a warp): the same arithmetic, the same bits."""
     from zipage_b200.layers import step_ops as P
     g, N, dev = _gen(heads), 1100, "cuda"
     qkv = torch.randn(N, (heads + 2 * kv_heads) * D, device=dev, generator=g).to(dtype)
@@ -192,3 +192,18 @@ def test_kernels_that_begin_early_see_what_came_before(rows, width):
         assert torch.equal(chain(lambda: None), want)
         graph.replay()
         assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("n,width", [(1, 1), (3, 70), (8, 129), (7, 129), (8, 0)])
+def test_decode_inputs(n, width):
+    from zipage_b200.layers.step_ops import decode_inputs
+    g = _gen(n + width)
+    n32 = lambda *s: torch.randint(0, 1000, s, device="cuda", generator=g, dtype=torch.int32)
+    ids, num, tab, qid = n32(n).long(), n32(n), n32(n, width + 3)[:, :width], n32(n)
+    buffers = (torch.full((8,), 5, dtype=torch.int64, device="cuda"), n32(8), n32(8, 129), n32(8))
+    assert decode_inputs(ids, num, tab, qid, buffers)
+    want = torch.full((8, 129), -1, dtype=torch.int32, device="cuda")
+    want[:n, :width] = tab
+    assert torch.equal(buffers[2], want) and torch.equal(buffers[0][:n], ids) and (buffers[0][n:] == 5).all()
+    assert torch.equal(buffers[1][:n], num) and (buffers[1][n:] == 0).all() and torch.equal(buffers[3][:n], qid) and (buffers[3][n:] == -1).all()
+    assert not decode_inputs(ids, num.long(), tab, qid, buffers) and not decode_inputs(ids, num, tab.cpu(), qid, buffers)

@@ -14,7 +14,7 @@ from __future__ import annotations
 
 import torch
 
-from ..layers.step_ops import prepare_decode
+from ..layers.step_ops import decode_inputs, prepare_decode
 from ..utils.context import reset_context, set_context
 
 
@@ -71,6 +71,8 @@ class DecodeGraphRunner:
     def _fill(self, input_ids, num_tokens, block_tables, query_ids):
         bs = input_ids.shape[0]
         assert bs <= self.max_bs and block_tables.shape[1] <= self.block_tables.shape[1]
+        if decode_inputs(input_ids, num_tokens, block_tables, query_ids, (self.input_ids, self.num_tokens, self.block_tables, self.query_ids)):
+            return bs
         self.input_ids[:bs] = input_ids
         self.num_tokens.zero_()
         self.num_tokens[:bs] = num_tokens

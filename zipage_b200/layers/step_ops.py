@@ -161,6 +161,21 @@ class Sampler(nn.Module):
         return sample(logits, temperatures, noise, self.seed)
 
 
+def decode_inputs(input_ids, num_tokens, block_tables, query_ids, buffers):
+    """The inputs of a decode step into the runner's buffers (ids, counts, tables, query ids), the rest cleared: one launch, or False
+    where the tensors are not such that the kernel can read them."""
+    ids, num, tab, qid = buffers
+    given = ((input_ids, ids), (num_tokens, num), (block_tables, tab), (query_ids, qid))
+    if not all(type(x) is torch.Tensor and x.device == y.device and x.dtype == y.dtype and x.dim() == y.dim() and (x.shape[-1] <= 1 or x.stride(-1) == 1)
+               for x, y in given) or not tab.is_cuda or not len(input_ids) == len(num_tokens) == len(block_tables) == len(query_ids):
+        return False
+    L.check(L.load().zp_decode_inputs(L.ptr(input_ids), L.ptr(num_tokens), L.ptr(block_tables), block_tables.stride(0), L.ptr(query_ids),
+                                      len(input_ids), block_tables.shape[1], L.ptr(ids), L.ptr(num), L.ptr(tab), L.ptr(qid),
+                                      len(ids), tab.shape[1], L.stream_ptr()), "decode_inputs")
+    _count(1)
+    return True
+
+
 def prepare_decode(num_tokens, block_tables, query_ids, query_cache_len, block_size=256):
     """Device tensors in, device tensors out: positions [B] i64, context_lens [B] i32,
     slot_mapping [B] i32, triples [B,3] i32 with n_triples [1] i32 valid rows."""
