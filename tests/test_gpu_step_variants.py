@@ -100,6 +100,9 @@ def test_linear_leaves_the_rest_to_the_layer():
         handle = layer.register_forward_hook(lambda m, i, o: o * 0)
         assert not linear(layer, x[:4]).any()
         handle.remove()
+        for k in (32, 96):                            # the layer refuses an input of another width
+            with pytest.raises(RuntimeError):
+                linear(layer, torch.randn(4, k, device="cuda", dtype=torch.bfloat16))
     assert K.LAUNCHES == before
 
 

@@ -56,16 +56,24 @@ class RMSNorm(nn.Module):
 SMALL_ROWS, SMALL_WEIGHT = 8, 1 << 23
 
 
+def _small_linear_takes(layer, x):
+    """Whether `zp_small_linear` computes layer(x), for x on the current CUDA device.  The kernel takes its sizes from the weight, so
+    they are compared here."""
+    w, b = layer.weight, layer.bias
+    return (type(layer) is nn.Linear and type(w) is nn.Parameter and x.dim() == w.dim() == 2 and 0 < x.shape[0] <= SMALL_ROWS
+            and x.shape[1] == w.shape[1] > 0 and w.numel() <= SMALL_WEIGHT and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype
+            and w.device == x.device and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 8 == 0 and w.shape[1] % 32 == 0
+            and (w.data_ptr() | x.data_ptr()) % 16 == 0
+            and (b is None or b.shape == w.shape[:1] and b.dtype == x.dtype and b.device == x.device and b.is_contiguous())
+            and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda")
+            and not (layer._forward_hooks or layer._forward_pre_hooks or nn.modules.module._has_any_global_hook()))
+
+
 def linear(layer, x):
     """layer(x) for an nn.Linear: the few rows of a small decode step through `zp_small_linear`, everything else
-    (more rows, fp32, odd sizes, gradients, subclasses, hooks) through the layer itself."""
-    w, b = layer.weight, layer.bias
-    if (type(layer) is nn.Linear and type(x) is torch.Tensor and type(w) is nn.Parameter and x.dim() == 2 and 0 < x.shape[0] <= SMALL_ROWS
-            and w.numel() <= SMALL_WEIGHT and x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype
-            and w.device == x.device and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 8 == 0 and w.shape[1] % 32 == 0
-            and (w.data_ptr() | x.data_ptr()) % 16 == 0 and (b is None or b.dtype == x.dtype and b.is_contiguous())
-            and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda")
-            and not (layer._forward_hooks or layer._forward_pre_hooks or nn.modules.module._has_any_global_hook())):
+    (more rows, fp32, odd sizes, sizes that do not fit, gradients, subclasses, hooks) through the layer itself."""
+    if type(x) is torch.Tensor and x.is_cuda and x.device.index == torch.cuda.current_device() and _small_linear_takes(layer, x):
+        w, b = layer.weight, layer.bias
         out = torch.empty((x.shape[0], w.shape[0]), dtype=x.dtype, device=x.device)
         L.check(L.load().zp_small_linear(L.ptr(x), x.stride(0), L.ptr(w), L.ptr(b), L.ptr(out), x.shape[0], w.shape[0], w.shape[1],
                                          L.dtype_code(x), L.stream_ptr()), "small_linear")
