@@ -100,6 +100,11 @@ def test_linear_leaves_the_rest_to_the_layer():
         handle = layer.register_forward_hook(lambda m, i, o: o * 0)
         assert not linear(layer, x[:4]).any()
         handle.remove()
+        with torch.autocast("cuda", torch.float16):
+            assert linear(layer, x[:4]).dtype == torch.float16
+        layer.forward = lambda v: v * 0
+        assert not linear(layer, x[:4]).any()
+        del layer.forward
         for k in (32, 96):                            # the layer refuses an input of another width
             with pytest.raises(RuntimeError):
                 linear(layer, torch.randn(4, k, device="cuda", dtype=torch.bfloat16))

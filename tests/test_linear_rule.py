@@ -40,3 +40,40 @@ def test_other_sizes_are_the_layers():
     assert not _small_linear_takes(_layer(k=0), _x(4, 0))
     assert not _small_linear_takes(_layer(), _x(0)) and not _small_linear_takes(_layer(), _x(SMALL_ROWS + 1))
     assert not _small_linear_takes(_layer(), _x()[0]) and not _small_linear_takes(_layer(), _x()[None])
+
+
+@torch.no_grad()
+def test_a_call_that_something_looks_at_is_the_layers():
+    layer, x = _layer(), _x()
+    layer.forward = lambda v: v                                  # (offloading and adapter libraries replace it so)
+    assert not _small_linear_takes(layer, x)
+    del layer.forward
+    assert _small_linear_takes(layer, x)
+    for register in (layer.register_forward_hook, layer.register_forward_pre_hook, nn.modules.module.register_module_forward_hook):
+        handle = register(lambda *a: None)
+        assert not _small_linear_takes(layer, x)
+        handle.remove()
+
+    class Function(torch.overrides.TorchFunctionMode):
+        def __torch_function__(self, f, types, args=(), kwargs=None):
+            return f(*args, **(kwargs or {}))
+
+    class Dispatch(torch.utils._python_dispatch.TorchDispatchMode):
+        def __torch_dispatch__(self, f, types, args=(), kwargs=None):
+            return f(*args, **(kwargs or {}))
+
+    for context in (Function(), Dispatch(), torch.enable_grad(), torch.autograd.forward_ad.dual_level()):
+        with context:
+            assert not _small_linear_takes(layer, x)
+    seen = []
+    torch.vmap(lambda v: seen.append(_small_linear_takes(layer, v)) or v)(x[:, None])
+    assert seen == [False]
+    with torch.device("cpu"):
+        assert _small_linear_takes(layer, x)
+    assert _small_linear_takes(layer, x)
+
+
+@torch.no_grad()
+def test_a_patched_class_is_the_layers(monkeypatch):
+    monkeypatch.setattr(nn.Linear, "forward", lambda self, v: v)
+    assert not _small_linear_takes(_layer(), _x())

@@ -13,6 +13,9 @@ from __future__ import annotations
 
 import torch
 from torch import nn
+from torch.autograd import forward_ad
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from .. import _lib as L
 from ..kernel import _count
@@ -56,22 +59,39 @@ class RMSNorm(nn.Module):
 SMALL_ROWS, SMALL_WEIGHT = 8, 1 << 23
 
 
+_linear_forward = nn.Linear.forward
+
+
+def _plain_call(layer):
+    """Whether layer(x) is nn.Linear's product and nothing around it looks at the call: no hooks, no forward or compiled call of the layer's
+    own, no function or dispatch mode (a default device is one, but leaves products alone), no transform (vmap, forward-mode
+    derivatives), no gradients, autocast, tracing or compilation."""
+    modes = _get_current_function_mode_stack() if torch._C._len_torch_function_stack() else ()
+    return (type(layer) is nn.Linear and nn.Linear.forward is _linear_forward and "forward" not in layer.__dict__
+            and layer._compiled_call_impl is None
+            and not (layer._forward_hooks or layer._forward_pre_hooks or nn.modules.module._has_any_global_hook())
+            and all(type(m) is DeviceContext for m in modes) and not torch._C._len_torch_dispatch_stack()
+            and torch._C._functorch.peek_interpreter_stack() is None and forward_ad._current_level < 0
+            and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda")
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+
+
 def _small_linear_takes(layer, x):
     """Whether `zp_small_linear` computes layer(x), for x on the current CUDA device.  The kernel takes its sizes from the weight, so
     they are compared here."""
+    if not _plain_call(layer):
+        return False
     w, b = layer.weight, layer.bias
-    return (type(layer) is nn.Linear and type(w) is nn.Parameter and x.dim() == w.dim() == 2 and 0 < x.shape[0] <= SMALL_ROWS
+    return (type(w) is nn.Parameter and x.layout is w.layout is torch.strided and x.dim() == w.dim() == 2 and 0 < x.shape[0] <= SMALL_ROWS
             and x.shape[1] == w.shape[1] > 0 and w.numel() <= SMALL_WEIGHT and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype
             and w.device == x.device and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 8 == 0 and w.shape[1] % 32 == 0
             and (w.data_ptr() | x.data_ptr()) % 16 == 0
-            and (b is None or b.shape == w.shape[:1] and b.dtype == x.dtype and b.device == x.device and b.is_contiguous())
-            and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda")
-            and not (layer._forward_hooks or layer._forward_pre_hooks or nn.modules.module._has_any_global_hook()))
+            and (b is None or b.shape == w.shape[:1] and b.dtype == x.dtype and b.device == x.device and b.is_contiguous()))
 
 
 def linear(layer, x):
     """layer(x) for an nn.Linear: the few rows of a small decode step through `zp_small_linear`, everything else
-    (more rows, fp32, odd sizes, sizes that do not fit, gradients, subclasses, hooks) through the layer itself."""
+    (more rows, fp32, odd sizes, sizes that do not fit, gradients, subclasses, hooks, modes) through the layer itself."""
     if type(x) is torch.Tensor and x.is_cuda and x.device.index == torch.cuda.current_device() and _small_linear_takes(layer, x):
         w, b = layer.weight, layer.bias
         out = torch.empty((x.shape[0], w.shape[0]), dtype=x.dtype, device=x.device)
