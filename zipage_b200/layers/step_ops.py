@@ -79,10 +79,10 @@ def _plain_call(layer):
 def _small_linear_takes(layer, x):
     """Whether `zp_small_linear` computes layer(x), for x on the current CUDA device.  The kernel takes its sizes from the weight, so
     they are compared here."""
-    if not _plain_call(layer):
+    if x.dim() != 2 or x.shape[0] > SMALL_ROWS or not _plain_call(layer):      # (what tells most other calls apart comes first)
         return False
     w, b = layer.weight, layer.bias
-    return (type(w) is nn.Parameter and x.layout is w.layout is torch.strided and x.dim() == w.dim() == 2 and 0 < x.shape[0] <= SMALL_ROWS
+    return (type(w) is nn.Parameter and x.layout is w.layout is torch.strided and w.dim() == 2 and x.shape[0] > 0
             and x.shape[1] == w.shape[1] > 0 and w.numel() <= SMALL_WEIGHT and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype
             and w.device == x.device and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 8 == 0 and w.shape[1] % 32 == 0
             and (w.data_ptr() | x.data_ptr()) % 16 == 0
