@@ -337,11 +337,13 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
               }
               if (!ok) continue;
               ++cnt[t];
+              // (before the next scores are reported: the softmax's wait compares parities, and after those scores it could otherwise
+              // take the product two steps back for the last one)
+              umma_commit(&sh.pvdone[t]);
               if (j + 1 < n[t]) {                            // (behind the product that reads p from its columns)
                 if (t == 0 || j + 1 >= n[0]) ok = keys(j + 1);
                 if (ok) issue_s(t, j + 1);
               }
-              umma_commit(&sh.pvdone[t]);
             }
             if (ok) umma_commit(&sh.vempty[k % NBAR]);
             if (++vslot == (uint32_t)g.nv) vslot = 0;
