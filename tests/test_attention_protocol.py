@@ -3,7 +3,9 @@
 The issuer of products, the tensor pipe (which works the issued products and commits off in order) and the softmax warps of both
 tiles are replayed as coroutines over models of the mbarriers, under random schedules and random numbers of key tiles per item.  Checked:
 no deadlock; a softmax warp reads the scores of its own step; the product reads the weights of its own step; and the output of
-an item is read from that item's accumulator, although the next item's first product overwrites all of it.  A wait for a product compares the parity of its barrier, so that the product
+an item is read from that item's accumulator, although the next item's first product overwrites all of it.  With two groups of warps a
+tile that last point needs both groups' hand-over before an item's first product: the variant that waits for one of them alone
+reads the next item's accumulator within a few items.  A wait for a product compares the parity of its barrier, so that the product
 before has to be reported before the next scores are: the other order takes the one for the other.
 """
 import random
@@ -16,7 +18,7 @@ from test_slot_protocol import Bar, Violation
 WARPS = 4                              # of a group
 
 
-def run(seed, groups, done_before_scores=True, n_items=25):
+def run(seed, groups, first_waits_for_both=True, done_before_scores=True, n_items=25):
     rnd = random.Random(seed)
     items = [(rnd.randint(0, 3), rnd.randint(0, 3)) for _ in range(n_items)]      # key tiles of the two query tiles
     sfull, pvdone = [Bar(1), Bar(1)], [Bar(1), Bar(1)]
@@ -40,6 +42,8 @@ def run(seed, groups, done_before_scores=True, n_items=25):
                     if j >= n[t]:
                         continue
                     for u in range(2):
+                        if groups == 2 and first_waits_for_both and j == 0 and u == 0:
+                            yield from wait(pfull[t][1], cnt[t] & 1)
                         yield from wait(pfull[t][u], cnt[t] & 1)
                         pipe.append(("product", t, (w, j), u))
                         yield
@@ -116,13 +120,24 @@ def run(seed, groups, done_before_scores=True, n_items=25):
             raise Violation("deadlock")
 
 
-@pytest.mark.parametrize("groups", [1])
+@pytest.mark.parametrize("groups", [1, 2])
 @pytest.mark.parametrize("seed", range(20))
 def test_an_items_output_is_its_own(seed, groups):
     run(seed, groups)
 
 
-@pytest.mark.parametrize("groups", [1])
+def test_waiting_for_one_of_two_groups_is_unsafe():
+    failures = 0
+    for seed in range(10):
+        try:
+            run(seed, 2, first_waits_for_both=False)
+        except Violation as e:
+            assert "output" in str(e)
+            failures += 1
+    assert failures > 0
+
+
+@pytest.mark.parametrize("groups", [1, 2])
 def test_reporting_a_product_after_the_next_scores_is_unsafe(groups):
     failures = 0
     for seed in range(10):

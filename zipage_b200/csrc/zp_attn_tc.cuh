@@ -324,7 +324,10 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
               const uint32_t pt = tmem + t * 128, ot = tmem + O_COL + t * 128;
 #pragma unroll
               for (int u = 0; u < 2; ++u) {                  // the softmax hands over 64 keys at a time
-                ok = ok && mbar_wait(&sh.pfull[t][u], cnt[t] & 1, abortp, p.error_word, 831);
+                // an item's first product overwrites all of O: both groups have to be past the item before, whose output they read there
+                const bool first = GROUPS == 2 && j == 0;
+                if (first && u == 0) ok = ok && mbar_wait(&sh.pfull[t][1], cnt[t] & 1, abortp, p.error_word, 840);
+                if (!first || u == 0) ok = ok && mbar_wait(&sh.pfull[t][u], cnt[t] & 1, abortp, p.error_word, 831);
                 if (!ok) continue;
                 fence_after_sync();
 #pragma unroll
@@ -570,7 +573,7 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
         for (int i = 0; i < 4; ++i)
           if (r4 + i < rows && c + c8 < p.dv) st16(p.out(q0 + r4 + i, head, c + c8), v[i]);
       }
-      fence_before_sync();      // (the next item's first product into O follows this warp's next arrival)
+      fence_before_sync();      // (the next item's first product into O follows the next arrival of every softmax warp of this tile)
     }
   }
   fence_before_sync();
