@@ -130,3 +130,50 @@ def test_latent_prefill_edges(many, dim, rot, vdim, rank):
         ref, mag = _softmax(q[a:a + x].view(x, heads, dim + rot), k, kv[b:b + y, heads * dim:].view(y, heads, vdim), (dim + rot) ** -0.5, seen)
         assert ((out[a:a + x].view(x, heads, vdim).double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * mag + 1e-6).all()
         a, b = a + x, b + y
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.04])
+@pytest.mark.parametrize("kind", ["prompts", "prompts_fp16", "windows_64", "windows_128", "windows_biased", "windows_capped", "latents"])
+@pytest.mark.parametrize("copies", [1, 40])              # launches of few and of many query tiles
+def test_factors_of_zero_and_below(kind, scale, copies):
+    """The mean of the visible values, or weights that fall with the product; masked keys stay unseen."""
+    from zipage_b200.layers import attention as A
+    from zipage_b200.layers.latent_attention import latent_prefill
+    heads, kv_heads, dtype = 4, 2, torch.float16 if kind == "prompts_fp16" else torch.bfloat16
+    lens_q, lens_k = [1, 129, 250] * copies, [70, 129, 400] * copies
+    g = torch.Generator(device="cuda").manual_seed(copies)
+    n = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dtype)
+    rows, keys, cap, slopes = sum(lens_q), sum(lens_k), 0.0, None
+    if kind == "latents":
+        kv_heads = heads
+        q, kv, lat, out = n(rows, heads * D), n(keys, heads * (64 + 128)), n(keys, 64 + 64), torch.empty(rows, heads * 128, dtype=dtype, device="cuda")
+        latent_prefill(q, kv, lat, _cu(lens_q), _cu(lens_k), max(lens_q), out, heads, 64, 64, 128, 64, scale)
+        q, v = q.view(rows, heads, D), kv[:, heads * 64:].view(keys, heads, 128)
+        k = torch.cat([kv[:, :heads * 64].view(keys, heads, 64), lat[:, None, 64:].expand(-1, heads, -1)], -1)
+    elif kind.startswith("prompts"):
+        q, k, v = n(rows, heads, D), n(keys, kv_heads, D), n(keys, kv_heads, D)
+        out = A.varlen_prefill_attention(q, k, v, max(lens_q), _cu(lens_q), max(lens_k), _cu(lens_k), softmax_scale=scale)
+    else:
+        d = 64 if kind == "windows_64" else 128
+        q, k, v = n(rows, heads, d), n(keys, kv_heads, d), n(keys, kv_heads, d)
+        need = [(m + 63) // 64 for m in lens_k]
+        table = torch.full((len(need), max(need)), -1, dtype=torch.int32, device="cuda")
+        for b, part in enumerate(torch.arange(sum(need), dtype=torch.int32, device="cuda").split(need)):
+            table[b, :need[b]] = part
+        cap, slopes = 30.0 if kind == "windows_capped" else 0.0, torch.rand(heads, device="cuda", generator=g) * 0.05 if kind == "windows_biased" else None
+        out = A.window_attention(q.flatten(1), _paged(k, lens_k, 64, table), _paged(v, lens_k, 64, table), torch.tensor(lens_k, dtype=torch.int32, device="cuda"),
+                                 table, heads, d, d, scale, 0, cap, cu_seqlens_q=_cu(lens_q), max_seqlen_q=max(lens_q), slopes=slopes)
+    _no_device_error()
+    # as in the tests above: weights of prompts are rounded to T, the others carry 16 bits; one rounding of the result
+    unit = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * 1.1
+    for b in (0, 1, 2, len(lens_q) - 1):
+        x, y, r0, k0 = lens_q[b], lens_k[b], sum(lens_q[:b]), sum(lens_k[:b])
+        p, j = torch.arange(y - x, y, device="cuda")[:, None], torch.arange(y, device="cuda")[None]
+        kk, vv = (t[k0:k0 + y].double().repeat_interleave(heads // kv_heads, 1) for t in (k, v))
+        s = torch.einsum("thd,shd->hts", q[r0:r0 + x].double(), kk) * scale
+        s = cap * torch.tanh(s / cap) if cap else s
+        s = s if slopes is None else s - slopes.double()[:, None, None] * (p - j)
+        w = torch.softmax(s.masked_fill(j > p, float("-inf")), -1)
+        ref, mag = torch.einsum("hts,shd->thd", w, vv), torch.einsum("hts,shd->thd", w, vv.abs())
+        err = (out[r0:r0 + x].view(x, heads, -1).double() - ref).abs()
+        assert (err <= (unit * 2 * mag if kind.startswith("prompts") else 2.0 ** -8 * ref.abs() + 1e-4 * mag) + 1e-6).all()

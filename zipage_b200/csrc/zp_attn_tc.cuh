@@ -143,6 +143,12 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, error_word, where));
 }
 
+// The factor of the raw products as a positive number and what is left of it: masked products become -inf before they meet the factor.
+struct Factor {
+  float mag, sign;
+  __device__ __forceinline__ explicit Factor(float s) : mag(s > 0.f || s < 0.f ? fabsf(s) : 1.f), sign(s > 0.f ? 1.f : s < 0.f ? -1.f : s) {}
+};
+
 // What P has to bring:
 //   T                            element type;  SPLIT: weights as hi + lo (T = bf16);  MASKED: rows have a first visible key too
 //   GROUPS                       1, or 2 where the reference is fixed (halves of a row need no common maximum then)
@@ -154,8 +160,8 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
 //   load_k(dst, bar, it, step, i), load_v(dst, bar, it, step, i): TMA loads of one block each
 //   Row(p, it, t, r)             one query row, with lim (last visible key) and, where MASKED, lo and keep (keys j < lo are not seen
 //                                unless j < keep), ref0 (first reference; -inf unless CAPPED), and
-//     scale()                    what a raw product is multiplied by to become the exponent of 2, or
-//     transform(s, key0)         (P::BIASED) raw products of 32 keys to exponents of 2, or
+//     fac                        what a raw product is multiplied by to become the exponent of 2 (its magnitude by the pipeline, or by
+//     transform(s, key0)         (P::BIASED) that makes exponents of 2 of the raw products of 32 keys), or
 //     weights4(s, w)             (CAPPED) four raw products to four weights
 //     finish(p, ref, l)          factor of the row's sums (1 / l, gates)
 //     entries(p, c, v)           (P::GATED) factors of 32 entries
@@ -383,6 +389,7 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
         fence_after_sync();
         bool whole = key0 + COLS - 1 <= row.lim;
         if constexpr (P::MASKED) whole = whole && (key0 >= row.lo || key0 + COLS <= row.keep);
+        if constexpr (!P::CAPPED) whole = whole && row.fac.sign == 1.f;
         whole = __all_sync(0xffffffffu, whole || dry);
         auto seen = [&](int key) -> uint32_t {          // of 32 keys
           uint32_t m = low_bits(row.lim - key + 1);
@@ -404,7 +411,7 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
                   if (!(y >> (i + u) & 1u)) wt[u] = 0.f;
               }
             } else {
-              const float sc = P::BIASED ? 1.f : row.scale();
+              const float sc = P::BIASED ? 1.f : row.fac.mag;
 #pragma unroll
               for (int u = 0; u < 4; u += 2) {
                 float2 x = make_float2(-mref, -mref);
@@ -466,6 +473,10 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
               tmem_ld32_issue(st + c, s);
               const uint32_t y = seen(key0 + c);
               tmem_ld32_wait(s);
+              if (row.fac.sign != 1.f) {                     // (a factor that is negative or zero)
+#pragma unroll
+                for (int i = 0; i < 32; ++i) s[i] = __float_as_uint(__uint_as_float(s[i]) * row.fac.sign);
+              }
 #pragma unroll
               for (int i = 0; i < 32; ++i)
                 if (!(y >> i & 1u)) s[i] = 0xff800000u;      // -inf
@@ -487,7 +498,7 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
             for (int i = 2; i < 32; i += 2) m[c] = fmax3(m[c], __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
           }
           m[0] = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
-          if constexpr (!P::BIASED) m[0] *= row.scale();
+          if constexpr (!P::BIASED) m[0] *= row.fac.mag;
           const bool moves = !dry && m[0] > ref + P::LAZY;
           if (__any_sync(0xffffffffu, moves)) {
             const float fac = moves ? ex2(ref - m[0]) : 1.f;

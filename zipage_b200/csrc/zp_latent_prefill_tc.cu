@@ -74,10 +74,10 @@ struct LatentPrefillTc {
 
   struct Row {
     int lim;
-    float ref0, sc;
+    float ref0;
+    Factor fac;
     __device__ __forceinline__ Row(const LatentPrefillTc& p, const Item& it, int t, int r)
-        : lim(min(it.keys - 1, of_tile(it.pos, t) + r)), ref0(-INFINITY), sc(p.scale_log2e) {}
-    __device__ __forceinline__ float scale() const { return sc; }
+        : lim(min(it.keys - 1, of_tile(it.pos, t) + r)), ref0(-INFINITY), fac(p.scale_log2e) {}
     __device__ __forceinline__ float finish(const LatentPrefillTc&, float, float l) const { return l > 0.f ? 1.f / l : 0.f; }
   };
 };
@@ -113,7 +113,8 @@ extern "C" int zp_latent_prefill(const void* q, int64_t q_stride, const void* kv
     set_error("zp_latent_prefill: needs bf16, head sizes that are multiples of 8 (values at most 128) and 16-byte aligned rows");
     return ZP_ERR_UNSUPPORTED;
   }
-  if ((int64_t)H * (total_q / 128 + B) <= LATENT_SHORT)
+  // (the other kernel masks products before it scales them: factors above zero only)
+  if (scale > 0.f && (int64_t)H * (total_q / 128 + B) <= LATENT_SHORT)
     return latent_prefill_tc_short(q, q_stride, kv, latent, cu_seqlens_q, cu_seqlens_k, out, out_stride, B, max_seqlen_q, total_q, total_k, H, dim,
                                    rot, vdim, kv_rank, KP, scale, (cudaStream_t)stream);
   LatentPrefillTc p;

@@ -71,10 +71,10 @@ template <typename T_> struct PrefillTc {
 
   struct Row {
     int lim;
-    float ref0, sc;
+    float ref0;
+    Factor fac;
     __device__ __forceinline__ Row(const PrefillTc& p, const Item& it, int t, int r)
-        : lim(min(it.keys - 1, of_tile(it.pos, t) + r)), ref0(-INFINITY), sc(p.scale_log2e) {}
-    __device__ __forceinline__ float scale() const { return sc; }
+        : lim(min(it.keys - 1, of_tile(it.pos, t) + r)), ref0(-INFINITY), fac(p.scale_log2e) {}
     __device__ __forceinline__ float finish(const PrefillTc&, float, float l) const { return l > 0.f ? 1.f / l : 0.f; }
   };
 };

@@ -100,10 +100,11 @@ struct WindowTc {
   struct Row {
     int lim, lo, keep, row, head;
     bool real;
-    float ref0, sc, y, m2c, off, slope;
+    float ref0, y, m2c, off, slope;
+    Factor fac;
     __device__ __forceinline__ Row(const WindowTc& p, const Item& it, int t, int r)
         : lim(of_tile(it.pos, t) + r), lo(win_first(p.a, lim)), keep(p.a.keep), row(of_tile(it.q0, t) + r), head(of_tile(it.head, t)),
-          real(r < of_tile(it.rows, t)), ref0(-INFINITY), sc(p.a.scale * LOG2E) {
+          real(r < of_tile(it.rows, t)), ref0(-INFINITY), fac(p.a.scale * LOG2E) {
       if constexpr (CAPPED) {
         y = 2.f * LOG2E * p.a.scale / p.a.softcap;
         m2c = -2.f * p.a.softcap * LOG2E;
@@ -112,13 +113,12 @@ struct WindowTc {
       }
       if constexpr (BIASED) slope = win_slope2(p.a, head);
     }
-    __device__ __forceinline__ float scale() const { return sc; }
     __device__ __forceinline__ void transform(uint32_t (&s)[32], int key0) const {
       const float at = slope * (float)(key0 - lim);      // bias of the first column (lim is the row's position)
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
         float2 x = make_float2(fmaf(slope, (float)i, at), fmaf(slope, (float)(i + 1), at));
-        ffma2(x, make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), make_float2(sc, sc));
+        ffma2(x, make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), make_float2(fac.mag, fac.mag));
         s[i] = __float_as_uint(x.x);
         s[i + 1] = __float_as_uint(x.y);
       }
@@ -188,7 +188,8 @@ constexpr int64_t WINDOW_SHORT = 704;
 int window_prefill_tc_short(const WinArgs& a, int max_q, int total_q, cudaStream_t st);
 
 int window_prefill_tc(const WinArgs& a, int max_q, int total_q, cudaStream_t st) {
-  if ((int64_t)a.Hq * (total_q / 128 + a.B) <= WINDOW_SHORT) return window_prefill_tc_short(a, max_q, total_q, st);
+  // (the other kernel masks products before it scales them: factors above zero only)
+  if ((a.scale > 0.f || a.softcap > 0.f) && (int64_t)a.Hq * (total_q / 128 + a.B) <= WINDOW_SHORT) return window_prefill_tc_short(a, max_q, total_q, st);
   if (a.softcap > 0.f) return launch_window_tc<WindowTc<true, false>>(a, max_q, total_q, st);
   if (a.slopes) return launch_window_tc<WindowTc<false, true>>(a, max_q, total_q, st);
   return launch_window_tc<WindowTc<false, false>>(a, max_q, total_q, st);
