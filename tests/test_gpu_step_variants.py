@@ -135,6 +135,37 @@ def test_paged_decode_splits(dtype, B, heads, kv_heads, width):
         assert ((out[b, 0].double() - ref).abs() <= 2 * unit * mag + 1e-6).all()
 
 
+@pytest.mark.parametrize("offset", [0, 4, 8])
+def test_paged_decode_takes_scratch_of_exactly_the_needed_size(offset):
+    """Wherever floats may lie: all splits run, so that the bits are those of a call with plenty, and nothing is noted."""
+    from zipage_b200 import _lib as L
+    lib, B, heads, kv_heads, D, width = L.load(), 2, 8, 2, 128, 20
+    g = _gen(offset)
+    kc, vc = (torch.randn(B * width, 256, kv_heads, D, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    table = torch.arange(B * width, dtype=torch.int32, device="cuda").view(B, width)
+    lens, q = torch.tensor([width * 256, 4000], dtype=torch.int32, device="cuda"), torch.randn(B, heads, D, device="cuda", generator=g).to(torch.bfloat16)
+
+    def call(ws, size):
+        out = torch.empty_like(q)
+        rc = lib.zp_paged_decode(L.ptr(q), L.ptr(kc), L.ptr(vc), L.ptr(lens), L.ptr(table), L.ptr(out), B, width, heads, kv_heads, D, 256, kc.stride(0),
+                                 D ** -0.5, L.dtype_code(q), ws, size, L.stream_ptr())
+        torch.cuda.synchronize()
+        assert rc == 0
+        return out
+    splits = min(width, 32)                               # (148 * 4 blocks over 2 x 2 would be more)
+    exact = B * kv_heads * splits * 4 * (D + 2) * 4       # groups of 4 heads
+    plenty = torch.empty(2 * exact, dtype=torch.uint8, device="cuda")
+    ws = torch.empty(exact + offset, dtype=torch.uint8, device="cuda")
+    want = call(plenty.data_ptr(), plenty.numel())
+    call(0, 0)
+    unsplit = lib.zp_last_error()
+    assert b"unsplit" in unsplit
+    assert lib.zp_rms_norm(*[None] * 5, 4, 4096, 4096, 4096, 1e-6, 0, None) != 0       # (another note)
+    other = lib.zp_last_error()
+    assert torch.equal(call(ws.data_ptr() + offset, exact), want) and lib.zp_last_error() == other
+    assert lib.zp_paged_decode_workspace_bytes(B, heads, D, 32) >= exact
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("q_rank,R,rot,heads,dim", [(2048, 1024, 64, 5, 8), (2056, 1024, 64, 1, 128), (8, 8, 8, 33, 64), (1536, 512, 24, 16, 0)])
 def test_latent_rows_in_vectors(dtype, q_rank, R, rot, heads, dim):

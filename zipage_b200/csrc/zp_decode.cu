@@ -256,9 +256,9 @@ extern "C" int zp_paged_decode(const void* q, const void* k_cache, const void* v
   const bool mma = (dtype == ZP_DTYPE_BF16 || dtype == ZP_DTYPE_F16) && D == 128 && BS % 64 == 0 && G <= 16;
   a.nsplit = zp::pick_splits(B, Hkv, NBmax);
   a.part = nullptr;
-  if (const size_t off = (uintptr_t)workspace % 8; workspace && off) {      // (partial results are read in pairs)
-    workspace = (char*)workspace + (8 - off);
-    workspace_bytes = workspace_bytes > 8 - off ? workspace_bytes - (8 - off) : 0;
+  if (const size_t off = (uintptr_t)workspace % 4; workspace && off) {      // (partial results are floats)
+    workspace = (char*)workspace + (4 - off);
+    workspace_bytes = workspace_bytes > 4 - off ? workspace_bytes - (4 - off) : 0;
   }
   if (mma && (int64_t)NBmax * BS <= zp::DEC_CLUSTER_KEYS) a.nsplit = zp::pick_cluster(B, Hkv, NBmax, BS);
   else if (a.nsplit > 1) {

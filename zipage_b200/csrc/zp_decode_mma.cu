@@ -228,16 +228,18 @@ __global__ void __launch_bounds__(DM_THREADS) paged_decode_mma_kernel(const DmAr
 // A warp per query head.  The splits' maxima and sums are read by one lane each (at most 32 splits), so that their latency is
 // paid once; then every lane adds up four entries with the splits' loads in flight together.  1 sequence of 16000 keys, 32 heads:
 // 8.1 us; 4 of them: 6.8 (a block per key/value head that walked its splits one after the other: 34.2 and 24.7).
-template <typename T>
+// PAIRS: the scratch is 8-byte aligned (its rows are 130 floats), so that it is read in pairs.
+template <typename T, bool PAIRS>
 __global__ void __launch_bounds__(128) decode_mma_merge_kernel(const DmArgs a) {
   const int b = blockIdx.x, hq = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (hq >= a.Hq) return;
   const int G = a.Hq / a.Hkv, h = hq / G, row = hq % G;
   const float* base = a.part + (((int64_t)b * a.Hkv + h) * a.nsplit * a.gp + row) * 130;
   const int64_t pitch = (int64_t)a.gp * 130;
+  auto ld2 = [](const float* p) { return PAIRS ? *reinterpret_cast<const float2*>(p) : make_float2(p[0], p[1]); };
   float m = -INFINITY, l = 0.f;
   if (lane < a.nsplit) {
-    const float2 ml = *reinterpret_cast<const float2*>(base + lane * pitch + 128);
+    const float2 ml = ld2(base + lane * pitch + 128);
     m = ml.x; l = ml.y;
   }
   const float M = warp_max(m);
@@ -247,8 +249,8 @@ __global__ void __launch_bounds__(128) decode_mma_merge_kernel(const DmArgs a) {
 #pragma unroll 8
   for (int s = 0; s < a.nsplit; ++s) {
     const float ws = __shfl_sync(0xffffffffu, w, s);
-    const float2* rr = reinterpret_cast<const float2*>(base + s * pitch + lane * 4);   // (rows of 130 floats: 8-byte aligned)
-    const float2 x = rr[0], y = rr[1];
+    const float* rr = base + s * pitch + lane * 4;
+    const float2 x = ld2(rr), y = ld2(rr + 2);
     num.x = fmaf(ws, x.x, num.x); num.y = fmaf(ws, x.y, num.y);
     num.z = fmaf(ws, y.x, num.z); num.w = fmaf(ws, y.y, num.w);
   }
@@ -288,7 +290,8 @@ static int launch_decode_mma(const DmArgs& a, cudaStream_t st) {
   launch_early(kern, dim3(a.B, a.Hkv, a.nsplit), DM_THREADS, smem, st, a);
   int rc = check_launch("zp_paged_decode(mma)");
   if (rc || a.nsplit == 1) return rc;
-  decode_mma_merge_kernel<T><<<dim3(a.B, (a.Hq + 3) / 4), 128, 0, st>>>(a);
+  const auto merge = (uintptr_t)a.part % 8 == 0 ? decode_mma_merge_kernel<T, true> : decode_mma_merge_kernel<T, false>;
+  merge<<<dim3(a.B, (a.Hq + 3) / 4), 128, 0, st>>>(a);
   return check_launch("zp_paged_decode(mma) merge");
 }
 
