@@ -241,8 +241,8 @@ int zp_paged_decode(const void* q, const void* k_cache, const void* v_cache,
  * memory to the KV cache, a latency-critical thread that cannot take cudaMalloc's implicit
  * synchronisation).  The split-KV partial results go to a 4 MiB array built into the library
  * (every GPU that loads the library holds it until exit); the call performs no allocation of any
- * kind.  Batches whose split scratch exceeds zp_paged_decode_noalloc_max_scratch_bytes() are
- * rejected with ZP_ERR_WORKSPACE.  The first call on each device looks up the array's device
+ * kind.  Batches whose split scratch, counted for splits of whole pages whatever kernel runs, exceeds
+ * zp_paged_decode_noalloc_max_scratch_bytes() are rejected with ZP_ERR_WORKSPACE.  The first call on each device looks up the array's device
  * address (cudaGetSymbolAddress) and should therefore be made before any stream capture starts.
  * All calls on a device share the array: it keeps the last call's partials (every entry a call
  * reads is written by that call first, so nothing needs clearing), and two calls whose kernels

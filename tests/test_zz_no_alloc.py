@@ -88,3 +88,23 @@ def test_noalloc_decode_rejects_batches_beyond_the_builtin_scratch():
     rc_ref, ref = _call(lib, False, *c, ws)
     torch.cuda.synchronize()
     assert rc_new == 0 and rc_ref == 0 and torch.equal(new, ref)
+
+
+def test_noalloc_decode_of_long_tables_uses_the_builtin_array():
+    """16-bit caches split short tables without scratch; beyond 4096 keys the partial results go to the array."""
+    from oracle import zipage_oracle as O
+    from zipage_b200 import _lib as L
+    dev, lib, B, Hq, Hkv, D, width = torch.device("cuda:0"), L.load(), 2, 8, 2, 128, 17
+    g = torch.Generator().manual_seed(9)
+    kc, vc = (torch.randn(B * width, BS, Hkv, D, generator=g).to(torch.bfloat16) for _ in range(2))
+    table, lens = torch.randperm(B * width, generator=g).to(torch.int32).view(B, width), torch.tensor([width * BS, 300], dtype=torch.int32)
+    q = torch.randn(B, Hq, D, generator=g).to(torch.bfloat16)
+    args = [t.to(dev) for t in (q, kc, vc, lens, table)]
+    ws = torch.empty(lib.zp_paged_decode_workspace_bytes(B, Hq, D, 32), dtype=torch.uint8, device=dev)
+    rc, ref = _call(lib, False, *args, ws)
+    for _ in range(2):
+        rc_new, new = _call(lib, True, *args)
+        torch.cuda.synchronize()
+        assert rc == 0 and rc_new == 0 and torch.equal(new, ref)
+    want = O.paged_decode_attention(q.unsqueeze(1), kc, vc, lens, table).squeeze(1).float()
+    assert (new.cpu().float() - want).abs().max() <= 2e-2 * want.abs().max()

@@ -307,7 +307,8 @@ extern "C" int zp_paged_decode_noalloc(const void* q, const void* k_cache, const
                                        void* stream) {
   if (B == 0) return ZP_OK;
   ZP_REQUIRE(Hkv > 0 && Hq % Hkv == 0, "zp_paged_decode_noalloc: Hq must be a multiple of Hkv");
-  // the same split choice as zp_paged_decode makes when given scratch
+  // The splits of whole pages, which zp_paged_decode makes of tables beyond a cluster's keys and of fp32 caches.  Shorter tables of the
+  // tensor-core form need no scratch, but the limit counts them alike: it depends on the batch, not on the kernel that runs.
   const int nsplit = zp::pick_splits(B, Hkv, NBmax);
   const size_t need = nsplit > 1
       ? (size_t)B * Hkv * nsplit * zp::gp_of(Hq / Hkv) * (D + 2) * sizeof(float) : 0;
