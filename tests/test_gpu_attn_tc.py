@@ -177,3 +177,101 @@ def test_factors_of_zero_and_below(kind, scale, copies):
         ref, mag = torch.einsum("hts,shd->thd", w, vv), torch.einsum("hts,shd->thd", w, vv.abs())
         err = (out[r0:r0 + x].view(x, heads, -1).double() - ref).abs()
         assert (err <= (unit * 2 * mag if kind.startswith("prompts") else 2.0 ** -8 * ref.abs() + 1e-4 * mag) + 1e-6).all()
+
+
+def _climb(q, k, lens, at):
+    """Scores that climb from 128 keys to the next by about 45 powers of two (a steeper step every third time), for the heads whose
+    queries look at entry `at`: one head up, one down, the others not.  q, k [rows, heads, d]; scale d^-0.5."""
+    step = 45.0 / 1.4427 * q.shape[2] ** 0.5 / 8
+    k[:, :, at] = torch.cat([(torch.arange(n, device="cuda") // 128 * 1.0 + torch.arange(n, device="cuda") // 384) * step for n in lens])[:, None].to(k.dtype)
+    q[:, :, at] = 0
+    q[:, 0, at], q[:, -1, at] = 8, -8
+
+
+# scores reach some 700 powers of two; the accumulators keep 2^-22 of their raw products, which moves weight and sum by 1.2e-4 each
+CLIMB_ERROR = 4e-4
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("heads,kv_heads", [(4, 2), (3, 1)])
+def test_prompts_whose_reference_moves(dtype, heads, kv_heads):
+    """The reference moves by more than the lazy bound at almost every key tile, and the accumulator with it."""
+    from zipage_b200.layers.attention import varlen_prefill_attention
+    lens_q, lens_k = [1000, 130, 700], [1300, 1100, 700]
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    n = lambda rows, h: torch.randn(rows, h, D, device="cuda", generator=g).to(dtype)
+    q, k, v = n(sum(lens_q), heads), n(sum(lens_k), kv_heads), n(sum(lens_k), kv_heads)
+    _climb(q, k, lens_k, 5)
+    out = varlen_prefill_attention(q, k, v, max(lens_q), _cu(lens_q), max(lens_k), _cu(lens_k))
+    _no_device_error()
+    unit = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * 1.1      # as in test_prefill_edges
+    a = b = 0
+    for x, y in zip(lens_q, lens_k):
+        seen = torch.arange(y, device="cuda")[None] <= torch.arange(x, device="cuda")[:, None] + y - x
+        ref, mag = _softmax(q[a:a + x], k[b:b + y], v[b:b + y], D ** -0.5, seen)
+        assert ((out[a:a + x].double() - ref).abs() <= (unit * 2 + CLIMB_ERROR) * mag + 1e-6).all()
+        a, b = a + x, b + y
+
+
+@pytest.mark.parametrize("many", [False, True])          # launches of few and of many query tiles
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(8, 4, 128, 128), (6, 2, 48, 16), (3, 3, 72, 104)])
+@pytest.mark.parametrize("softcap,steep,window", [(30.0, False, 300), (0.0, True, 0), (0.0, True, 300)])
+@pytest.mark.parametrize("gated", ["entry", None])
+def test_windows_of_views(many, heads, kv_heads, dim, vdim, softcap, steep, window, gated):
+    """Columns of wider rows for queries, gates and results, a gate per entry, a factor, climbing scores, several items per block."""
+    from zipage_b200.layers.attention import window_attention
+    copies = 1 + 2000 // (10 * heads) if many else 1
+    lens_q, lens_k = [1, 129, 400, 250] * copies, [513, 129, 700, 1000] * copies
+    g = torch.Generator(device="cuda").manual_seed(heads + dim)
+    n = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    rows, keys = sum(lens_q), sum(lens_k)
+    q, k, v = n(rows, heads, dim), n(keys, kv_heads, dim), n(keys, kv_heads, vdim)
+    if steep:
+        _climb(q, k, lens_k, 5)
+    wide, gate = n(rows, heads * dim + 24), n(rows, 8 + heads * vdim + 16)[:, 8:8 + heads * vdim]
+    wide[:, 16:-8] = q.flatten(1)
+    pad = lambda t: torch.nn.functional.pad(t, (0, -t.shape[2] % 16))
+    need = [(m + 63) // 64 for m in lens_k]
+    ids, table = torch.randperm(sum(need), device="cuda", generator=g).to(torch.int32), torch.full((len(need), max(need)), -1, dtype=torch.int32, device="cuda")
+    for b, part in enumerate(ids.split(need)):
+        table[b, :need[b]] = part
+    results = torch.full((rows, heads * vdim + 16), 3.0, dtype=torch.bfloat16, device="cuda")
+    window_attention(wide[:, 16:-8], _paged(pad(k), lens_k, 64, table), _paged(pad(v), lens_k, 64, table), torch.tensor(lens_k, dtype=torch.int32, device="cuda"),
+                     table, heads, dim, vdim, dim ** -0.5, window, softcap, cu_seqlens_q=_cu(lens_q), max_seqlen_q=max(lens_q), out=results[:, 8:-8],
+                     impl="auto" if many else "tcgen05", gate=gate if gated else None, gate_mode=gated, out_scale=0.7)
+    _no_device_error()
+    assert (results[:, :8] == 3).all() and (results[:, -8:] == 3).all()
+    for i in [*range(4), *range(len(lens_q) - 4, len(lens_q))]:
+        x, y, a, b = lens_q[i], lens_k[i], sum(lens_q[:i]), sum(lens_k[:i])
+        p, j = torch.arange(y - x, y, device="cuda")[:, None], torch.arange(y, device="cuda")[None]
+        seen = (j <= p) & (p - j < window) if window else j <= p
+        kk, vv = (t[b:b + y].double().repeat_interleave(heads // kv_heads, 1) for t in (k, v))
+        s = torch.einsum("thd,shd->hts", q[a:a + x].double(), kk) * dim ** -0.5
+        s = softcap * torch.tanh(s / softcap) if softcap else s
+        w = torch.softmax(s.masked_fill(~seen[None], float("-inf")), -1) * 0.7
+        f = torch.sigmoid(gate[a:a + x].double()).view(x, heads, vdim) if gated else 1.0
+        ref, mag = torch.einsum("hts,shd->thd", w, vv) * f, torch.einsum("hts,shd->thd", w, vv.abs()) * f
+        # as in test_window_edges
+        assert ((results[a:a + x, 8:-8].view(x, heads, vdim).double() - ref).abs() <= 2.0 ** -8 * ref.abs() + (CLIMB_ERROR if steep else 1e-4) * mag + 1e-6).all()
+
+
+@pytest.mark.parametrize("many", [False, True])
+@pytest.mark.parametrize("dim,rot", [(128, 64), (64, 0)])
+def test_latents_whose_reference_moves(many, dim, rot):
+    from zipage_b200.layers.latent_attention import latent_prefill
+    copies = 60 if many else 1
+    heads, vdim, rank, lens_q, lens_k = 3, 128, 64, [1, 300, 513] * copies, [900, 301, 1300] * copies
+    g = torch.Generator(device="cuda").manual_seed(dim + rot)
+    n = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    rows, keys = sum(lens_q), sum(lens_k)
+    q, k, v, lat = n(rows, heads, dim + rot), n(keys, heads, dim), n(keys, heads, vdim), n(keys, rank + rot)
+    _climb(q, k, lens_k, 5)
+    kv, out = torch.cat([k.flatten(1), v.flatten(1)], -1), torch.empty(rows, heads * vdim, dtype=torch.bfloat16, device="cuda")
+    latent_prefill(q.flatten(1), kv, lat, _cu(lens_q), _cu(lens_k), max(lens_q), out, heads, dim, rot, vdim, rank, (dim + rot) ** -0.5)
+    _no_device_error()
+    for i in [*range(3), *range(len(lens_q) - 3, len(lens_q))]:
+        x, y, a, b = lens_q[i], lens_k[i], sum(lens_q[:i]), sum(lens_k[:i])
+        kk = torch.cat([k[b:b + y], lat[b:b + y, None, rank:].expand(-1, heads, -1)], -1)
+        seen = torch.arange(y, device="cuda")[None] <= torch.arange(x, device="cuda")[:, None] + y - x
+        ref, mag = _softmax(q[a:a + x], kk, v[b:b + y], (dim + rot) ** -0.5, seen)
+        assert ((out[a:a + x].view(x, heads, vdim).double() - ref).abs() <= 2.0 ** -8 * ref.abs() + CLIMB_ERROR * mag + 1e-6).all()
