@@ -53,3 +53,11 @@ def test_other_step_ops_reject_bad_arguments():
     assert lib.zp_prepare_decode(p, p, p, 3, 9, 32, 256, p, p, p, p, None, None) == INVALID
     assert lib.zp_prepare_decode(None, p, p, 3, 9, 32, 256, p, p, p, p, p, None) == INVALID
     assert lib.zp_prepare_decode(p, p, p, 3, 9, 300, 256, p, p, p, p, p, None) == INVALID  # window longer than a page
+
+
+def test_latent_rows_reject_unknown_types():
+    lib, p = L.load(), C.c_void_p(4096)
+    for dtype in (3, 7, -1):
+        assert lib.zp_latent_prepare(p, 640, p, p, p, p, p, p, None, p, 5, 64, 512, 64, 576, 100, 1e-6, dtype, None) == INVALID
+        assert "dtype" in _err(lib)
+        assert lib.zp_latent_rotate_q(p, 640, p, p, None, 5, 4, 96, 64, 0, 0, dtype, None) == INVALID

@@ -243,7 +243,7 @@ extern "C" int zp_latent_prepare(const void* y, int64_t row_stride, const int64_
   const int epv = 16 / (int)zp::dtype_size(dtype);
   const int vec_q = q_rank % epv == 0 && row_stride % epv == 0 && ((uintptr_t)y | (uintptr_t)cq) % 16 == 0;
   const int vec_kv = vec_q && kv_rank % epv == 0 && KP % epv == 0 && ((uintptr_t)cache | (uintptr_t)dense) % 16 == 0;
-  if (dtype != ZP_DTYPE_F32 && vec_q && (vec_kv || kv_rank == 0) && q_rank <= 256 * zp::LP_NQ && kv_rank <= 256 * zp::LP_NK && rot <= 64 &&
+  if ((dtype == ZP_DTYPE_BF16 || dtype == ZP_DTYPE_F16) && vec_q && (vec_kv || kv_rank == 0) && q_rank <= 256 * zp::LP_NQ && kv_rank <= 256 * zp::LP_NK && rot <= 64 &&
       ((uintptr_t)q_weight | (uintptr_t)kv_weight) % 16 == 0) {
     auto run = [&](auto t) {
       using T = decltype(t);
