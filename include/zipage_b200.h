@@ -291,7 +291,7 @@ int zp_rms_norm(const void* x, const void* residual, const void* weight, void* o
 int zp_silu_and_mul(const void* x, void* out, int n_rows, int inter, int dtype, void* stream);
 
 /* out [rows, n_out] = T(x weight^T + bias) for up to 8 rows: x [rows, k] (row stride, a multiple of 8), weight [n_out, k] contiguous,
- * bias [n_out] or NULL, out contiguous; 16-bit T, fp32 accumulation, k a multiple of 32, x and weight 16-byte aligned.  (No counterpart
+ * bias [n_out] or NULL, out contiguous; 16-bit T, fp32 accumulation, k a multiple of 32 and at most 2^24, n_out at most 2^30, x and weight 16-byte aligned.  (No counterpart
  * in the reference, whose projections are torch's: third_party/nanovllm/layers/linear.py:54-153.) */
 int zp_small_linear(const void* x, int64_t x_stride, const void* weight, const void* bias, void* out, int rows, int n_out, int k,
                     int dtype, void* stream);

@@ -61,3 +61,13 @@ def test_latent_rows_reject_unknown_types():
         assert lib.zp_latent_prepare(p, 640, p, p, p, p, p, p, None, p, 5, 64, 512, 64, 576, 100, 1e-6, dtype, None) == INVALID
         assert "dtype" in _err(lib)
         assert lib.zp_latent_rotate_q(p, 640, p, p, None, 5, 4, 96, 64, 0, 0, dtype, None) == INVALID
+
+
+def test_small_linear_rejects_bad_arguments():
+    lib, p = L.load(), C.c_void_p(4096)
+    call = lambda x=p, stride=64, w=p, out=p, rows=4, n=48, k=64, dtype=0: lib.zp_small_linear(x, stride, w, None, out, rows, n, k, dtype, None)
+    assert call(rows=0) == 0 and call(n=0) == 0
+    for bad in (dict(x=None), dict(w=None), dict(out=None), dict(rows=9), dict(rows=-1), dict(n=-1), dict(k=0), dict(k=48), dict(stride=65),
+                dict(x=C.c_void_p(4100)), dict(w=C.c_void_p(4100)), dict(k=1 << 27), dict(n=2 ** 31 - 1)):
+        assert call(**bad) == INVALID, bad
+    assert call(dtype=7) != 0

@@ -72,7 +72,9 @@ extern "C" int zp_small_linear(const void* x, int64_t x_stride, const void* weig
                                int dtype, void* stream) {
   if (rows == 0 || n_out == 0) return ZP_OK;
   ZP_REQUIRE(x && weight && out, "zp_small_linear: null pointer");
-  ZP_REQUIRE(rows > 0 && rows <= 8 && n_out > 0 && k > 0 && k % 32 == 0 && x_stride % 8 == 0, "zp_small_linear: sizes not supported");
+  // (sizes up to which the bytes of a block's rows and the number of blocks are counted in 32 bits)
+  ZP_REQUIRE(rows > 0 && rows <= 8 && n_out > 0 && n_out <= 1 << 30 && k > 0 && k <= 1 << 24 && k % 32 == 0 && x_stride % 8 == 0,
+             "zp_small_linear: sizes not supported");
   ZP_REQUIRE(((uintptr_t)x | (uintptr_t)weight) % 16 == 0, "zp_small_linear: x and weight must be 16-byte aligned");
   auto run = [&](auto t) {
     using T = decltype(t);
