@@ -275,3 +275,39 @@ def test_latents_whose_reference_moves(many, dim, rot):
         seen = torch.arange(y, device="cuda")[None] <= torch.arange(x, device="cuda")[:, None] + y - x
         ref, mag = _softmax(q[a:a + x], kk, v[b:b + y], (dim + rot) ** -0.5, seen)
         assert ((out[a:a + x].view(x, heads, vdim).double() - ref).abs() <= 2.0 ** -8 * ref.abs() + CLIMB_ERROR * mag + 1e-6).all()
+
+
+def _kernels(call):
+    """Names of the kernels that `call` launches."""
+    from torch.profiler import ProfilerActivity, profile
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    if not names:
+        pytest.skip("the profiler records no kernels here")
+    return " ".join(names)
+
+
+@pytest.mark.parametrize("rows,context,short", [(128, 512, True), (100, 400, True), (128, 500, False), (129, 2000, False), (128, 0, False)])
+def test_latents_of_single_tiles(rows, context, short):
+    """Portions of one tile behind a context of at least four times their length leave the pairs of the shared pipeline half empty."""
+    from zipage_b200.layers.latent_attention import latent_prefill
+    heads, B, dim, rot, vdim, rank = 8, 40, 64, 64, 128, 64
+    lens_q, lens_k = [rows] * B, [rows + context] * B
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    n = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    q, kv, lat = n(rows * B, heads * (dim + rot)), n((rows + context) * B, heads * (dim + vdim)), n((rows + context) * B, rank + rot)
+    out, cq, ck = torch.empty(rows * B, heads * vdim, dtype=torch.bfloat16, device="cuda"), _cu(lens_q), _cu(lens_k)
+    names = _kernels(lambda: latent_prefill(q, kv, lat, cq, ck, rows, out, heads, dim, rot, vdim, rank, D ** -0.5))
+    _no_device_error()
+    assert ("short" in names) == short
+    for b in (0, B - 1):
+        a, x, y = b * rows, rows, rows + context
+        part = kv[b * y:b * y + y]
+        k = torch.cat([part[:, :heads * dim].view(y, heads, dim), lat[b * y:b * y + y, None, rank:].expand(-1, heads, -1)], -1)
+        seen = torch.arange(y, device="cuda")[None] <= torch.arange(x, device="cuda")[:, None] + y - x
+        ref, mag = _softmax(q[a:a + x].view(x, heads, D), k, part[:, heads * dim:].view(y, heads, vdim), D ** -0.5, seen)
+        assert ((out[a:a + x].view(x, heads, vdim).double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * mag + 1e-6).all()

@@ -87,6 +87,13 @@ struct LatentPrefillTc {
 // 47 / 22 to 39; 448, equal portions 32 / 40, continued ones 67 / 58; 512: 48 to 76 / 57 to 75, 128-token portions 64 / 48; 560: 52 to
 // 98 / 73 to 112; 1216: 122 to 178 / 187 to 236.
 constexpr int64_t LATENT_SHORT = 512;
+// Portions of up to one tile leave the second tile of every item empty, which costs the more the longer the work on the first lasts: with
+// a context of four times the portions such launches go there too, whatever their number.  32 portions of 128, 100, 64, 32 tokens,
+// 32 heads (us, this file / short): no context 59 / 74, 61 / 76, 59 / 70, 61 / 64; after 256 keys 105 / 107, 106 / 109, 107 / 102, 107 / 96; after
+// 512 145 / 139, 146 / 143, 147 / 135, 148 / 131; after 2000 (128, 100, 64) 381 / 340, 383 / 338, 383 / 332.
+static bool latent_takes_short(int H, int B, int max_seqlen_q, int total_q, int total_k) {
+  return (int64_t)H * (total_q / 128 + B) <= LATENT_SHORT || (max_seqlen_q <= 128 && total_k >= (int64_t)5 * total_q);
+}
 int latent_prefill_tc_short(const void* q, int64_t q_stride, const void* kv, const void* latent, const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k,
                             void* out, int64_t out_stride, int B, int max_seqlen_q, int total_q, int total_k, int H, int dim, int rot, int vdim,
                             int kv_rank, int KP, float scale, cudaStream_t st);
@@ -114,7 +121,7 @@ extern "C" int zp_latent_prefill(const void* q, int64_t q_stride, const void* kv
     return ZP_ERR_UNSUPPORTED;
   }
   // (the other kernel masks products before it scales them: factors above zero only)
-  if (scale > 0.f && (int64_t)H * (total_q / 128 + B) <= LATENT_SHORT)
+  if (scale > 0.f && latent_takes_short(H, B, max_seqlen_q, total_q, total_k))
     return latent_prefill_tc_short(q, q_stride, kv, latent, cu_seqlens_q, cu_seqlens_k, out, out_stride, B, max_seqlen_q, total_q, total_k, H, dim,
                                    rot, vdim, kv_rank, KP, scale, (cudaStream_t)stream);
   LatentPrefillTc p;
