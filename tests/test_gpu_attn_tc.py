@@ -238,7 +238,7 @@ def test_windows_of_views(many, heads, kv_heads, dim, vdim, softcap, steep, wind
     results = torch.full((rows, heads * vdim + 16), 3.0, dtype=torch.bfloat16, device="cuda")
     window_attention(wide[:, 16:-8], _paged(pad(k), lens_k, 64, table), _paged(pad(v), lens_k, 64, table), torch.tensor(lens_k, dtype=torch.int32, device="cuda"),
                      table, heads, dim, vdim, dim ** -0.5, window, softcap, cu_seqlens_q=_cu(lens_q), max_seqlen_q=max(lens_q), out=results[:, 8:-8],
-                     impl="auto" if many else "tcgen05", gate=gate if gated else None, gate_mode=gated, out_scale=0.7)
+                     impl="tcgen05", gate=gate if gated else None, gate_mode=gated, out_scale=0.7)
     _no_device_error()
     assert (results[:, :8] == 3).all() and (results[:, -8:] == 3).all()
     for i in [*range(4), *range(len(lens_q) - 4, len(lens_q))]:
@@ -311,3 +311,43 @@ def test_latents_of_single_tiles(rows, context, short):
         seen = torch.arange(y, device="cuda")[None] <= torch.arange(x, device="cuda")[:, None] + y - x
         ref, mag = _softmax(q[a:a + x].view(x, heads, D), k, part[:, heads * dim:].view(y, heads, vdim), D ** -0.5, seen)
         assert ((out[a:a + x].view(x, heads, vdim).double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * mag + 1e-6).all()
+
+
+def _plain_windows(heads, kv_heads, d, lens, context, window, softcap):
+    """Windows over random portions behind `context` keys: the names of the kernels, and the check of the first and last portion."""
+    from zipage_b200.layers.attention import window_attention
+    lens_k = [n + context for n in lens]
+    g = torch.Generator(device="cuda").manual_seed(len(lens) + d)
+    n = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    q, k, v = n(sum(lens), heads, d), n(sum(lens_k), kv_heads, d), n(sum(lens_k), kv_heads, d)
+    need = [(m + 63) // 64 for m in lens_k]
+    table = torch.full((len(need), max(need)), -1, dtype=torch.int32, device="cuda")
+    for b, part in enumerate(torch.arange(sum(need), dtype=torch.int32, device="cuda").split(need)):
+        table[b, :need[b]] = part
+    args = (q.flatten(1), _paged(k, lens_k, 64, table), _paged(v, lens_k, 64, table), torch.tensor(lens_k, dtype=torch.int32, device="cuda"), table, heads, d, d,
+            d ** -0.5, window, softcap)
+    cu = _cu(lens)
+    out = window_attention(*args, cu_seqlens_q=cu, max_seqlen_q=max(lens))
+    names = _kernels(lambda: window_attention(*args, cu_seqlens_q=cu, max_seqlen_q=max(lens)))
+    _no_device_error()
+    for i in (0, len(lens) - 1):
+        x, y, a, b = lens[i], lens_k[i], sum(lens[:i]), sum(lens_k[:i])
+        p, j = torch.arange(y - x, y, device="cuda")[:, None], torch.arange(y, device="cuda")[None]
+        seen = (j <= p) & (p - j < window) if window else j <= p
+        kk, vv = (t[b:b + y].double().repeat_interleave(heads // kv_heads, 1) for t in (k, v))
+        s = torch.einsum("thd,shd->hts", q[a:a + x].double(), kk) * d ** -0.5
+        s = softcap * torch.tanh(s / softcap) if softcap else s
+        w = torch.softmax(s.masked_fill(~seen[None], float("-inf")), -1)
+        ref, mag = torch.einsum("hts,shd->thd", w, vv), torch.einsum("hts,shd->thd", w, vv.abs())
+        assert ((out[a:a + x].view(x, heads, d).double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * mag + 1e-6).all()
+    return "short" if "tc_short" in names else "pairs" if "attn_tc" in names else "mma" if "window_prefill_mma" in names else names
+
+
+@pytest.mark.parametrize("heads,kv_heads,lens,context,window,softcap,kernel", [
+    (32, 8, [128] * 13, 0, 0, 0.0, "short"), (32, 8, [128] * 14, 0, 0, 0.0, "pairs"),                  # 416 and 448 tiles
+    (32, 8, [200] * 11, 1100, 0, 30.0, "short"), (32, 8, [200] * 12, 1100, 0, 30.0, "pairs"),          # 704 and 768, far, capped
+    (32, 8, [200] * 11, 700, 0, 30.0, "pairs"), (32, 8, [200] * 11, 1100, 0, 0.0, "pairs"), (32, 8, [200] * 11, 1100, 512, 30.0, "short"),
+    (8, 8, [128] * 60, 0, 0, 0.0, "pairs"), (8, 8, [128] * 60, 64, 0, 0.0, "short"), (8, 8, [128] * 60, 0, 100, 0.0, "short"),
+])
+def test_which_windows_go_in_pairs(heads, kv_heads, lens, context, window, softcap, kernel):
+    assert _plain_windows(heads, kv_heads, 128, lens, context, window, softcap) == kernel

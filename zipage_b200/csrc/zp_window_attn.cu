@@ -133,7 +133,7 @@ int window_decode_mma(const WinArgs& a, int dtype, cudaStream_t st);
 int window_decode_splits(int B, int Hkv, int span);
 // tcgen05 prefill kernel (zp_window_attn_tc.cu)
 bool window_tc_supports(const WinArgs& a, int total_q, int dtype);
-int window_prefill_tc(const WinArgs& a, int max_q, int total_q, cudaStream_t st);
+int window_prefill_tc(const WinArgs& a, int max_q, int total_q, bool forced, cudaStream_t st);
 
 }  // namespace zp
 
@@ -193,7 +193,7 @@ extern "C" int zp_window_attention(const void* q, const void* k_cache, const voi
     return ZP_ERR_UNSUPPORTED;
   }
   if (tc && (impl == ZP_IMPL_TCGEN05 || (impl == ZP_IMPL_AUTO && max_seqlen_q >= 96)))
-    return zp::window_prefill_tc(a, max_seqlen_q, total_q, st);
+    return zp::window_prefill_tc(a, max_seqlen_q, total_q, impl == ZP_IMPL_TCGEN05, st);
   if (half && impl != ZP_IMPL_SIMT && zp::window_mma_supports(a)) {
     if (cu_seqlens_q) return zp::window_prefill_mma(a, max_seqlen_q, dtype, st);
     int span = NBmax * BS;

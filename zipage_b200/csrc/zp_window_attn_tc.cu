@@ -13,6 +13,8 @@
 // A tile of its own per block, all softmax warps on it, left the tensor cores idle during each of its softmax turns.  Four portions of
 // 500 to 3000 tokens, 32 heads on 8, window 1024, cap 30: 302 us (344 so).  Uniform portions, no window: 4 x 2000 tokens 236 us (320),
 // 4 x 1000 85 (112); cap 30 and window 512: 86 (107).
+#include <algorithm>
+
 #include "zp_attn_tc.cuh"
 #include "zp_window_attn.cuh"
 
@@ -179,17 +181,40 @@ static int launch_window_tc(const WinArgs& a, int max_q, int total_q, cudaStream
   return launch_attn(p, grid, st, "zp_window_attention(tcgen05)");
 }
 
-// Launches of up to so many 128-row query tiles (about: the counts are on the device) take the kernel of zp_window_attn_tc_short.cu.
-// A pair of tiles as the unit of work leaves coarser last waves, and its code is longer to fetch.  Kernel times of the two over head sizes
-// 64 and 128, with and without window, cap and earlier context (us, this file / short): 32 tiles 15.6 / 11.7; 112: 18 to 37 / 12 to 26;
-// 352: 24 to 48 / 20 to 35; 448, equal portions 27 to 35 / 35 to 40, continued ones 62 / 45; 672: 56 to 57 / 66 to 67, continued under a
-// window 86 / 76, the widest loss at this line; 800: 56 to 63 / 76, 94 / 88; 1216: 100 to 177 / 124 to 190.
-constexpr int64_t WINDOW_SHORT = 704;
+// Launches of few 128-row query tiles take the kernel of zp_window_attn_tc_short.cu (single tiles, whose waves are finer and whose code is
+// shorter to fetch).  Times of this file's kernel over that one's, heads of 128, portions of 96 to 2560 tokens, 32 heads on 8 unless noted; the
+// lines lie where no column is above 1 by more than a few percent:
+//   tiles        no context, no cap   cap   | window 512 or 1024, context 2000: no cap   cap   | no window, context 2000: no cap   cap
+//   320 .. 416   0.86 .. 1.00   0.91 .. 1.03 | 1.05 .. 1.14   1.12 .. 1.20                     | 0.95 .. 1.18   1.13 .. 1.26
+//   448 .. 576   0.70 .. 0.76   0.72 .. 0.82 | 0.83 .. 0.90   0.90 .. 0.97                     | 0.82 .. 0.96   0.90 .. 0.99
+//   608 .. 736   0.75 .. 0.84   0.76 .. 0.96 | 0.91 .. 0.98   1.02 .. 1.06                     | 0.91 .. 1.01   1.02 .. 1.15
+//   768 ..       0.60 .. 0.83   0.63 .. 0.82 | 0.80 .. 0.94   0.84 .. 0.99                     | 0.78 .. 0.92   0.84 .. 1.01 (one 1.09)
+// (Caps: two waves of pairs last as long as three to four of single tiles, so 608 to 736 tiles, three waves for five, lose.)  With an odd
+// number of heads per key/value head a pair is two row blocks of one head: half empty for portions of one tile (1.14 to 1.35 with a context
+// of 500 to 2000 keys), and under a window or behind a context each of its tiles also walks keys that only the other one sees (16 heads on
+// 16, 12 portions of 30 to 1500 tokens after 1000, window 512: 1.07 to 1.11; 48 of 10 to 200: 1.24 to 1.28).  Without either it
+// is 0.67 to 1.00.
+constexpr int64_t WINDOW_SHORT = 704;      // in heads x (rows / 128 + portions), at most twice the number of tiles
+constexpr int64_t WINDOW_TILES = 432, WINDOW_TILES_CAP = 768;
 int window_prefill_tc_short(const WinArgs& a, int max_q, int total_q, cudaStream_t st);
 
-int window_prefill_tc(const WinArgs& a, int max_q, int total_q, cudaStream_t st) {
+static bool window_takes_short(const WinArgs& a, int max_q, int total_q, bool forced) {
+  if ((int64_t)a.Hq * (total_q / 128 + a.B) <= WINDOW_SHORT) return true;
+  if (forced) return false;
+  const int64_t keys = (int64_t)a.NBmax * a.BS;      // that a sequence's table has room for
+  if (a.Hq / a.Hkv % 2) return a.window > 0 || a.chunk > 0 || 2 * keys >= (int64_t)3 * max_q;
+  // tiles: half a tile more per portion than its rows fill, at most what the longest portion has (the counts are on the device)
+  const int64_t tiles = a.Hq * std::min((int64_t)a.B * ((max_q + 127) / 128), std::max((int64_t)a.B, (int64_t)total_q / 128 + (a.B + 1) / 2));
+  if (tiles < WINDOW_TILES) return true;
+  const int64_t span = std::min({keys, a.window > 0 ? (int64_t)a.window : keys, a.chunk > 0 ? (int64_t)a.chunk : keys});
+  const bool far = span < keys ? span >= 512 : span > 1024;      // a row sees so many keys
+  return a.softcap > 0.f && far && tiles < WINDOW_TILES_CAP;
+}
+
+// forced: the caller asked for tcgen05 (lines that depend on more than the number of tiles are for the others)
+int window_prefill_tc(const WinArgs& a, int max_q, int total_q, bool forced, cudaStream_t st) {
   // (the other kernel masks products before it scales them: factors above zero only)
-  if ((a.scale > 0.f || a.softcap > 0.f) && (int64_t)a.Hq * (total_q / 128 + a.B) <= WINDOW_SHORT) return window_prefill_tc_short(a, max_q, total_q, st);
+  if ((a.scale > 0.f || a.softcap > 0.f) && window_takes_short(a, max_q, total_q, forced)) return window_prefill_tc_short(a, max_q, total_q, st);
   if (a.softcap > 0.f) return launch_window_tc<WindowTc<true, false>>(a, max_q, total_q, st);
   if (a.slopes) return launch_window_tc<WindowTc<false, true>>(a, max_q, total_q, st);
   return launch_window_tc<WindowTc<false, false>>(a, max_q, total_q, st);
