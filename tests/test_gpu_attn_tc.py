@@ -351,3 +351,11 @@ def _plain_windows(heads, kv_heads, d, lens, context, window, softcap):
 ])
 def test_which_windows_go_in_pairs(heads, kv_heads, lens, context, window, softcap, kernel):
     assert _plain_windows(heads, kv_heads, 128, lens, context, window, softcap) == kernel
+
+
+@pytest.mark.parametrize("lens,context,kernel", [
+    ([96] + [64] * 30, 0, "mma"), ([300] + [40] * 30, 500, "mma"), ([96] + [80] * 30, 0, "pairs"), ([300] + [110] * 30, 0, "pairs"), ([96] + [64] * 3, 0, "short"),
+    ([96] * 11, 0, "mma"), ([96] * 11, 600, "short"), ([96] * 28, 0, "pairs"), ([140] * 11, 0, "short"),
+])
+def test_which_windows_of_small_heads_take_tcgen05(lens, context, kernel):
+    assert _plain_windows(16, 4, 64, lens, context, 0, 0.0) == kernel

@@ -4,6 +4,8 @@
 //
 // Cache rows are padded to KP / VP elements (multiples of 16; the padding stays zero), so that every
 // row starts on a 16-byte boundary whatever the head sizes.
+#include <algorithm>
+
 #include "zp_window_attn.cuh"
 
 namespace zp {
@@ -184,15 +186,23 @@ extern "C" int zp_window_attention(const void* q, const void* k_cache, const voi
   a.gate_stride = gate_stride; a.gate_mode = gate_mode; a.out_scale = out_scale;
   cudaStream_t st = (cudaStream_t)stream;
   const bool half = dtype == ZP_DTYPE_BF16 || dtype == ZP_DTYPE_F16;
-  // Portions long enough to fill 128-row query tiles.  Heads of 64 too (us, tcgen05 / mma.sync): 1 portion of 130 tokens 9.4 / 9.6, 8 of
-  // 128 7.9 / 9.5, 3 of 300 to 100 and 3 of 500 after up to 1000 earlier keys 26 / 43 and 46 / 74, 4 of 1000 140 / 254; of 32: 138 / 309.
+  // Portions long enough to fill 128-row query tiles.  Small heads too (us, tcgen05 / mma.sync): heads of 64, 1 portion of 130 tokens 9.4 / 9.6, 8
+  // of 128 7.9 / 9.5, 3 of 300 to 100 and 3 of 500 after up to 1000 earlier keys 26 / 43 and 46 / 74, 4 of 1000 140 / 254; of 32: 138 / 309.
+  // But a portion of up to 64 tokens is one tile of either kernel, and mma.sync's is the shorter: where small heads have mostly
+  // such portions and more of them than SMs, tcgen05 takes (portions after 0, 1000, 1000 keys; the last with window 256 and cap) 1.4 to 2.4, 0.8 to 1.3
+  // and 1.2 to 1.6 of its time.  With 80 tokens and from 450 tiles on it is 0.6 to 0.9, 0.5 to 0.6, 0.7 to 1.0, so the line is a mean of 80; of 112
+  // where a portion of several tiles is among them (1000 tokens and twenty of 40: 0.8 to 1.0, 0.7 to 1.0, 1.1 to 1.5).  Two or three waves of
+  // single tiles with few keys are mma.sync's too (176 and 352 tiles of 80 or 96 tokens: 1.0 to 1.4, 0.5 to 0.9, 0.8 to 1.2).
   const bool tc = cu_seqlens_q && zp::window_tc_supports(a, total_q, dtype);
   if (impl == ZP_IMPL_TCGEN05 && !tc) {
     zp::set_error("zp_window_attention: the tcgen05 kernel needs bf16 portions, head sizes that are multiples of 8 up to 128, 16-byte "
                   "aligned rows and no soft cap or one of at most 69 without slopes");
     return ZP_ERR_UNSUPPORTED;
   }
-  if (tc && (impl == ZP_IMPL_TCGEN05 || (impl == ZP_IMPL_AUTO && max_seqlen_q >= 96)))
+  const int64_t heads = (int64_t)Hq * B, keys = (int64_t)NBmax * BS, span = std::min({keys, window > 0 ? (int64_t)window : keys, chunk > 0 ? (int64_t)chunk : keys});
+  const bool few_keys = max_seqlen_q <= 128 && heads < 448 && span <= 512;
+  const bool fills = max_seqlen_q >= 96 && (KP + VP > 128 || heads <= 148 || (total_q >= (int64_t)(max_seqlen_q <= 192 ? 80 : 112) * B && !few_keys));
+  if (tc && (impl == ZP_IMPL_TCGEN05 || (impl == ZP_IMPL_AUTO && fills)))
     return zp::window_prefill_tc(a, max_seqlen_q, total_q, impl == ZP_IMPL_TCGEN05, st);
   if (half && impl != ZP_IMPL_SIMT && zp::window_mma_supports(a)) {
     if (cu_seqlens_q) return zp::window_prefill_mma(a, max_seqlen_q, dtype, st);
