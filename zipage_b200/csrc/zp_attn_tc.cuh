@@ -611,9 +611,10 @@ static inline Rings rings_of(int nbq, int nbv) {
 // launch that short is one tile's latency, which the second tile of a pair only adds to.
 // Prompts, single tiles / pairs: 1 x 100 tokens, 32 heads: 10.3 / 12.1 us; 4 of up to 400, 8 heads: 20.3 / 22.1; 16 of up to 100,
 // 16 heads (about 256 tiles by this count): 51.5 / 32.5.
-static inline int pick_mode(int heads, int B, int total_q, bool heads_share, bool even) {
-  if ((int64_t)heads * (total_q / 128 + B) <= 148) return SINGLE;
-  return heads_share && even ? PAIR_HEADS : PAIR_ROWS;
+// (Windows and latents of few tiles have kernels of their own, and no single tiles here.)
+static inline int pick_pair(int heads_per_kv) { return heads_per_kv % 2 == 0 ? PAIR_HEADS : PAIR_ROWS; }
+static inline int pick_mode(int heads, int heads_per_kv, int B, int total_q) {
+  return (int64_t)heads * (total_q / 128 + B) <= 148 ? SINGLE : pick_pair(heads_per_kv);
 }
 static inline dim3 grid_of(int mode, int heads, int B, int max_q, int& levels) {
   const int rows = mode == PAIR_ROWS ? 256 : 128;

@@ -128,7 +128,7 @@ extern "C" int zp_latent_prefill(const void* q, int64_t q_stride, const void* kv
   p.cu_q = cu_seqlens_q; p.cu_k = cu_seqlens_k; p.o = (__nv_bfloat16*)out; p.dv = vdim;
   p.nbn = (dim + 63) / 64;
   p.rings = rings_of(p.nbn + (rot + 63) / 64, (vdim + 63) / 64);
-  p.mode = pick_mode(H, B, total_q, false, false);
+  p.mode = PAIR_ROWS;      // (every head has keys of its own)
   const dim3 grid = grid_of(p.mode, H, B, max_seqlen_q, p.levels);
   p.out_stride = out_stride; p.scale_log2e = scale * LOG2E;
   p.error_word = device_error_word();

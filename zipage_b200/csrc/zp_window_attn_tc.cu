@@ -176,7 +176,7 @@ static int launch_window_tc(const WinArgs& a, int max_q, int total_q, cudaStream
   }
   p.rings = rings_of((a.D + 63) / 64, (a.DV + 63) / 64);
   p.dv = a.DV;
-  p.mode = pick_mode(a.Hq, a.B, total_q, true, a.Hq / a.Hkv % 2 == 0);
+  p.mode = pick_pair(a.Hq / a.Hkv);
   const dim3 grid = grid_of(p.mode, a.Hq, a.B, max_q, p.levels);
   return launch_attn(p, grid, st, "zp_window_attention(tcgen05)");
 }
