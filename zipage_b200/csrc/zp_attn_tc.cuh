@@ -103,46 +103,9 @@ __device__ __forceinline__ bool read_work(const uint4* answer, dim3& id) {
   return ok != 0;
 }
 
-// ---- operands --------------------------------------------------------------------------------------
-// MN-major tile, 128-byte swizzle: 64 contiguous elements per K row, 8-row groups 1024 bytes apart along K, the next 64
-// elements along MN a block away
-__device__ __forceinline__ uint64_t desc_mn(uint32_t addr) {
-  const uint32_t lo = ((addr >> 4) & 0x3FFFu) | ((uint32_t)(BLK >> 4) << 16);
-  const uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);
-  return (static_cast<uint64_t>(hi) << 32) | lo;
-}
-// A operand from TMEM (one row per lane, two 16-bit elements per column)
-__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d), "r"(a), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-  uint32_t x[16], y[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) { x[i] = r[i]; y[i] = r[16 + i]; }
-  tmem_st16(taddr, x);
-  tmem_st16(taddr + 16, y);
-}
+// ---- masks and waits ---------------------------------------------------------------------------------
 // the lowest n bits, n from below 0 to above 32
 __device__ __forceinline__ uint32_t low_bits(int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u; }
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-// the same answer in all lanes of the warp
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* error_word, int where) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, error_word, where));
-}
-
 // The factor of the raw products as a positive number and what is left of it: masked products become -inf before they meet the factor.
 struct Factor {
   float mag, sign;
@@ -338,7 +301,7 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
                 fence_after_sync();
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {                // 16 keys a step: 8 columns of p
-                  const uint64_t bd = desc_mn(v0 + (4 * u + c) * 2048);
+                  const uint64_t bd = smem_desc_mn(v0 + (4 * u + c) * 2048);
                   const uint32_t a = pt + u * 64 + (c >> 1) * 32 + (c & 1) * 8;
                   umma_ts(ot, a, bd, id_o, (j | u | c) ? 1u : 0u);
                   if (P::SPLIT) umma_ts(ot, a + 16, bd, id_o, 1u);
@@ -370,7 +333,7 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
     uint32_t tiles = 0, cnt = 0, ends = 0, vslot = 0;      // key tiles of the items before, steps and items of this tile, place in the value ring
     bool ok = true;
     for (uint32_t w = 0; ok; ++w) {
-      ok = warp_wait(&sh.ifull[w & 1], (w >> 1) & 1, abortp, p.error_word, 832);
+      ok = mbar_wait_warp(&sh.ifull[w & 1], (w >> 1) & 1, abortp, p.error_word, 832);
       if (!ok || !sh.item[w & 1].real) break;
       const Item it = sh.item[w & 1];
       __syncwarp();
@@ -384,7 +347,7 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
       for (int j = w == 0 ? -1 : 0; ok && j < n; ++j) {
         const bool dry = j < 0;
         const int key0 = it.key0(j) + half * COLS;      // first key of this group
-        if (!dry) ok = warp_wait(&sh.sfull[t], cnt & 1, abortp, p.error_word, 833);
+        if (!dry) ok = mbar_wait_warp(&sh.sfull[t], cnt & 1, abortp, p.error_word, 833);
         if (!ok) break;
         fence_after_sync();
         bool whole = key0 + COLS - 1 <= row.lim;
@@ -416,8 +379,8 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
               for (int u = 0; u < 4; u += 2) {
                 float2 x = make_float2(-mref, -mref);
                 ffma2(x, make_float2(__uint_as_float(s[i + u]), __uint_as_float(s[i + u + 1])), make_float2(sc, sc));
-                wt[u] = ex2(x.x);
-                wt[u + 1] = ex2(x.y);
+                wt[u] = ex2_approx(x.x);
+                wt[u + 1] = ex2_approx(x.y);
               }
             }
             l2 = fadd2(l2, fadd2(make_float2(wt[0], wt[1]), make_float2(wt[2], wt[3])));
@@ -443,7 +406,7 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
           const int left = max(it.keys - it.key0(j) - 64 * u, 0);
           if (left < 64) {
             const uint32_t k = tiles + j;
-            ok = warp_wait(&sh.vfull[k % NBAR], (k / NBAR) & 1, abortp, p.error_word, 835);
+            ok = mbar_wait_warp(&sh.vfull[k % NBAR], (k / NBAR) & 1, abortp, p.error_word, 835);
 #pragma unroll 1
             for (int i = r; ok && i < (64 - left) * 8 * g.nbv; i += 128) {
               const int line = i >> 3, blk = line / (64 - left), key = 64 * u + left + line % (64 - left);
@@ -501,12 +464,12 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
           if constexpr (!P::BIASED) m[0] *= row.fac.mag;
           const bool moves = !dry && m[0] > ref + P::LAZY;
           if (__any_sync(0xffffffffu, moves)) {
-            const float fac = moves ? ex2(ref - m[0]) : 1.f;
+            const float fac = moves ? ex2_approx(ref - m[0]) : 1.f;
             if (moves) ref = m[0];
             l2.x *= fac;
             l2.y *= fac;
             if (j > 0) {
-              ok = warp_wait(&sh.pvdone[t], (cnt & 1) ^ 1, abortp, p.error_word, 834);
+              ok = mbar_wait_warp(&sh.pvdone[t], (cnt & 1) ^ 1, abortp, p.error_word, 834);
               if (!ok) break;
               fence_after_sync();
 #pragma unroll 1
@@ -539,14 +502,14 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
       // ---- output: four lanes share a row's 64 bytes ----
       float l = l2.x + l2.y;
       if (n > 0) {
-        ok = warp_wait(&sh.pvdone[t], (cnt & 1) ^ 1, abortp, p.error_word, 836);
+        ok = mbar_wait_warp(&sh.pvdone[t], (cnt & 1) ^ 1, abortp, p.error_word, 836);
         if (!ok) break;
         fence_after_sync();
         if constexpr (GROUPS == 2) {      // (the halves' sums: both are past the item before, whose last product waited for both)
           sh.sum[t][half][r] = l;
           __syncwarp();
           if (lane == 0) mbar_arrive(&sh.lfull[t]);
-          ok = warp_wait(&sh.lfull[t], ends & 1, abortp, p.error_word, 839);
+          ok = mbar_wait_warp(&sh.lfull[t], ends & 1, abortp, p.error_word, 839);
           if (!ok) break;
           l = sh.sum[t][0][r] + sh.sum[t][1][r];
           ++ends;

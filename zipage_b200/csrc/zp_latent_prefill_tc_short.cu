@@ -36,49 +36,6 @@ struct LfParams {
   int* error_word;
 };
 
-__device__ __forceinline__ uint64_t lf_desc_mn(uint32_t addr) {   // MN-major, one 64-entry block
-  const uint32_t lo = ((addr >> 4) & 0x3FFFu) | ((uint32_t)(LF_BLK >> 4) << 16);
-  const uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);
-  return (static_cast<uint64_t>(hi) << 32) | lo;
-}
-__device__ __forceinline__ void lf_umma_ts(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d), "r"(a), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
-}
-__device__ __forceinline__ void lf_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ void lf_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-  uint32_t a[16], b[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) { a[i] = r[i]; b[i] = r[16 + i]; }
-  lf_st16(taddr, a);
-  lf_st16(taddr + 16, b);
-}
-__device__ __forceinline__ float lf_ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-__device__ __forceinline__ bool lf_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* error_word, int where) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, error_word, where));
-}
-// meeting of the 128 threads of a lane quadrant (barriers 1-4); true when any of them brings true
-__device__ __forceinline__ bool lf_meet_any(int q, bool v) {
-  uint32_t out;
-  asm volatile(
-      "{\n\t.reg .pred p, r;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "barrier.cta.red.or.pred r, %2, 128, p;\n\t"
-      "selp.u32 %0, 1, 0, r;\n\t}"
-      : "=r"(out) : "r"((uint32_t)v), "r"(q + 1) : "memory");
-  return out != 0;
-}
-
 __global__ void __launch_bounds__(LF_THREADS, 1)
 latent_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQn, const __grid_constant__ CUtensorMap tmQr,
                          const __grid_constant__ CUtensorMap tmKn, const __grid_constant__ CUtensorMap tmKr,
@@ -171,9 +128,9 @@ latent_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQn, const _
           const uint32_t v_addr = r_addr + s * LF_BLK;
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks) {      // 16 keys per step: 8 columns of P
-            const uint64_t bd = lf_desc_mn(v_addr + ks * 2048);
-            lf_umma_ts(tmem + LF_O + i * 64, tmem + LF_PHI + ks * 8, bd, ID_O, (j | ks) ? 1u : 0u);
-            lf_umma_ts(tmem + LF_O + i * 64, tmem + LF_PLO + ks * 8, bd, ID_O, 1u);
+            const uint64_t bd = smem_desc_mn(v_addr + ks * 2048);
+            umma_ts(tmem + LF_O + i * 64, tmem + LF_PHI + ks * 8, bd, ID_O, (j | ks) ? 1u : 0u);
+            umma_ts(tmem + LF_O + i * 64, tmem + LF_PLO + ks * 8, bd, ID_O, 1u);
           }
           umma_commit(&sh.empty[s]);
         }
@@ -195,7 +152,7 @@ latent_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQn, const _
       const int sb = j & 1, key0 = j * 128 + cq * 32;
       const bool whole = key0 + 31 <= lim;
       float mx = -INFINITY;
-      if (ok) ok = lf_wait(&sh.sfull[sb], (j >> 1) & 1, abortp, p.error_word, 927);
+      if (ok) ok = mbar_wait_warp(&sh.sfull[sb], (j >> 1) & 1, abortp, p.error_word, 927);
       if (ok) {
         fence_after_sync();
         tmem_ld32_issue(lane_base + sb * 128 + cq * 32, ra);
@@ -212,16 +169,16 @@ latent_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQn, const _
         for (int i = 0; i < 32; i += 2) mx = fmax3(mx, __uint_as_float(ra[i]), __uint_as_float(ra[i + 1]));
         mx *= sl2;
       }
-      if (lf_meet_any(q, mx > ref + LF_LAZY)) {           // some row's reference moves
+      if (meet_any(q, mx > ref + LF_LAZY)) {           // some row's reference moves
         sh.stat[cq][r] = mx;
-        lf_meet_any(q, false);
+        meet_any(q, false);
         const float m = fmaxf(fmaxf(sh.stat[0][r], sh.stat[1][r]), fmaxf(sh.stat[2][r], sh.stat[3][r]));
         float fac = 1.f;
-        if (m > ref + LF_LAZY) { fac = lf_ex2(ref - m); ref = m; }
+        if (m > ref + LF_LAZY) { fac = ex2_approx(ref - m); ref = m; }
         l0 *= fac;
         l1 *= fac;
         if (j > 0) {
-          if (ok) ok = lf_wait(&sh.pempty, (j & 1) ^ 1, abortp, p.error_word, 928);
+          if (ok) ok = mbar_wait_warp(&sh.pempty, (j & 1) ^ 1, abortp, p.error_word, 928);
           if (ok && cq * 32 < p.nbv * 64) {
             fence_after_sync();
             uint32_t o[32];
@@ -229,11 +186,11 @@ latent_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQn, const _
             tmem_ld32_wait(o);
 #pragma unroll
             for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * fac);
-            lf_st32(lane_base + LF_O + cq * 32, o);
+            tmem_st32(lane_base + LF_O + cq * 32, o);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           }
         }
-        lf_meet_any(q, false);                            // stat may be rewritten
+        meet_any(q, false);                            // stat may be rewritten
       }
       if (ok) {
         uint32_t hi[16], lw[16];
@@ -241,7 +198,7 @@ latent_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQn, const _
           const float mref = ref == -INFINITY ? 0.f : ref;   // (a row without queries: every weight is exp2(-inf))
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            const float w0 = lf_ex2(fmaf(__uint_as_float(ra[i]), sl2, -mref)), w1 = lf_ex2(fmaf(__uint_as_float(ra[i + 1]), sl2, -mref));
+            const float w0 = ex2_approx(fmaf(__uint_as_float(ra[i]), sl2, -mref)), w1 = ex2_approx(fmaf(__uint_as_float(ra[i + 1]), sl2, -mref));
             l0 += w0;
             l1 += w1;
             const __nv_bfloat162 x = __floats2bfloat162_rn(w0, w1);
@@ -259,16 +216,16 @@ latent_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQn, const _
         if (first < 128) {
           for (int i = 0; ok && i < p.nbv; ++i) {
             const int t = j * per + nbq + i, s = t % p.ring;
-            ok = lf_wait(&sh.full[s], (t / p.ring) & 1, abortp, p.error_word, 929);
+            ok = mbar_wait_warp(&sh.full[s], (t / p.ring) & 1, abortp, p.error_word, 929);
             for (int idx = threadIdx.x - 64; ok && idx < (128 - first) * 8; idx += 512)
               *reinterpret_cast<int4*>(ring + s * LF_BLK + (first + (idx >> 3)) * 128 + ((idx & 7) << 4)) = make_int4(0, 0, 0, 0);
           }
         }
-        if (ok) ok = lf_wait(&sh.pempty, (j & 1) ^ 1, abortp, p.error_word, 930);
+        if (ok) ok = mbar_wait_warp(&sh.pempty, (j & 1) ^ 1, abortp, p.error_word, 930);
         if (ok) {
           fence_after_sync();
-          lf_st16(lane_base + LF_PHI + cq * 16, hi);
-          lf_st16(lane_base + LF_PLO + cq * 16, lw);
+          tmem_st16(lane_base + LF_PHI + cq * 16, hi);
+          tmem_st16(lane_base + LF_PLO + cq * 16, lw);
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           if (first < 128) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
@@ -278,8 +235,8 @@ latent_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQn, const _
       if (lane == 0) mbar_arrive(&sh.pfull);
     }
     sh.stat[cq][r] = l0 + l1;
-    lf_meet_any(q, false);
-    if (ok) ok = lf_wait(&sh.ofull, 0, abortp, p.error_word, 931);
+    meet_any(q, false);
+    if (ok) ok = mbar_wait_warp(&sh.ofull, 0, abortp, p.error_word, 931);
     if (ok && cq * 32 < p.nbv * 64) {
       const float l = (sh.stat[0][r] + sh.stat[1][r]) + (sh.stat[2][r] + sh.stat[3][r]);
       fence_after_sync();

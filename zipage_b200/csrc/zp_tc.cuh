@@ -179,6 +179,57 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "memory");
 }
 
+// ---- the A operand in TMEM, an MN-major B operand -------------------------------------------------
+// MN-major tile, 128-byte swizzle: 64 contiguous elements per K row, 8-row groups 1024 bytes apart along K, the next 64
+// elements along MN `lbo` bytes away (blocks of 128 rows: 16 KB)
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t lbo = 16384) {
+  const uint32_t lo = ((addr >> 4) & 0x3FFFu) | ((lbo >> 4) << 16);
+  const uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);
+  return (static_cast<uint64_t>(hi) << 32) | lo;
+}
+// A operand from TMEM (one row per lane, two 16-bit elements per column)
+__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d), "r"(a), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+  uint32_t x[16], y[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) { x[i] = r[i]; y[i] = r[16 + i]; }
+  tmem_st16(taddr, x);
+  tmem_st16(taddr + 16, y);
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// 2^x and 1 / x to about 2^-22
+__device__ __forceinline__ float ex2_approx(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float rcp_approx(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+// meeting of the 128 threads of a lane quadrant (barriers 1 to 4); true when any of them brings true
+__device__ __forceinline__ bool meet_any(int q, bool v) {
+  uint32_t out;
+  asm volatile(
+      "{\n\t.reg .pred p, r;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.or.pred r, %2, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, r;\n\t}"
+      : "=r"(out) : "r"((uint32_t)v), "r"(q + 1) : "memory");
+  return out != 0;
+}
+// the same answer in all lanes of the warp
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* error_word, int where) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, error_word, where));
+}
+
 // ---- packed fp32 pairs and 3-input max (sm_100) ----
 __device__ __forceinline__ void ffma2(float2& d, float2 a, float2 b) {  // d += a * b, both lanes
   asm("{\n\t.reg .b64 ra, rb, rc;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"

@@ -16,28 +16,11 @@
 #include <algorithm>
 
 #include "zp_attn_tc.cuh"
-#include "zp_window_attn.cuh"
+#include "zp_window_tc.cuh"
 
 namespace zp {
 
 using namespace attn;
-
-__device__ __forceinline__ float rcp_(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-
-// four raw products -> exp2(-2c / (1 + exp2(y s)) + off).  The exponent is held at 30: beyond, 1 / (1 + E) is below
-// 2^-30 and the weight is 1 to fp32 accuracy, and the product of four stays finite.
-__device__ __forceinline__ void weights4(const uint32_t* s, float y, float m2c, float off, float (&p)[4]) {
-  const float2 yy = make_float2(y, y), one = make_float2(1.f, 1.f);
-  const float2 u = fmul2(make_float2(__uint_as_float(s[0]), __uint_as_float(s[1])), yy), v = fmul2(make_float2(__uint_as_float(s[2]), __uint_as_float(s[3])), yy);
-  const float2 ab = fadd2(make_float2(ex2(fminf(u.x, 30.f)), ex2(fminf(u.y, 30.f))), one), cd = fadd2(make_float2(ex2(fminf(v.x, 30.f)), ex2(fminf(v.y, 30.f))), one);
-  const float2 prod = fmul2(make_float2(ab.x, cd.x), make_float2(ab.y, cd.y));
-  const float r = rcp_(prod.x * prod.y) * m2c;
-  const float2 rr = fmul2(make_float2(prod.y, prod.x), make_float2(r, r));      // m2c / ab, m2c / cd
-  float2 lo = make_float2(off, off), hi = lo;
-  ffma2(lo, make_float2(rr.x, rr.x), make_float2(ab.y, ab.x));
-  ffma2(hi, make_float2(rr.y, rr.y), make_float2(cd.y, cd.x));
-  p[0] = ex2(lo.x); p[1] = ex2(lo.y); p[2] = ex2(hi.x); p[3] = ex2(hi.y);
-}
 
 template <bool CAPPED_, bool BIASED_>   // (not both)
 struct WindowTc {
@@ -128,7 +111,7 @@ struct WindowTc {
     __device__ __forceinline__ void weights4(const uint32_t* s, float (&w)[4]) const { zp::weights4(s, y, m2c, off, w); }
     __device__ __forceinline__ float finish(const WindowTc& p, float ref, float l) const {
       if (!real) return 0.f;
-      if (p.a.sink) l += ex2(win_sink2(p.a, head) - ref);
+      if (p.a.sink) l += ex2_approx(win_sink2(p.a, head) - ref);
       return l > 0.f ? win_head_factor<T>(p.a, row, head) / l : 0.f;
     }
     __device__ __forceinline__ void entries(const WindowTc& p, int c, float (&v)[32]) const {

@@ -6,8 +6,7 @@
 // Roles (576 threads, one block per SM): warp 0 = TMA producer and TMEM owner, warp 1 = MMA issuer, warps 2-17 = softmax.
 // Shared memory: the Q tile and a ring of five 32 KB K/V stages; TMEM: two S accumulators, O, P_hi and P_lo.
 // Every wait is bounded; after it the block raises the device error word and leaves.
-#include "zp_tc.cuh"
-#include "zp_window_attn.cuh"
+#include "zp_window_tc.cuh"
 
 namespace zp {
 
@@ -26,65 +25,6 @@ struct __align__(16) WtShared {
   int abort_flag;
 };
 
-// MN-major operand tile, 128-byte swizzle: 64 contiguous elements per K row, 8-row groups `sbo` bytes
-// apart along K, the next 64 elements along MN `lbo` bytes away
-__device__ __forceinline__ uint64_t desc_mn(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
-  const uint32_t lo = ((smem_addr >> 4) & 0x3FFFu) | ((lbo >> 4) << 16);
-  const uint32_t hi = (sbo >> 4) | (1u << 14) | (2u << 29);
-  return (static_cast<uint64_t>(hi) << 32) | lo;
-}
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ float ex2_(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-__device__ __forceinline__ float rcp_(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-
-// four raw products -> exp2(-2c / (1 + exp2(y s)) + off).  The exponent is held at 30: beyond, 1 / (1 + E) is below
-// 2^-30 and the weight is 1 to fp32 accuracy, and the product of four stays finite.
-__device__ __forceinline__ void weights4(const uint32_t* s, float y, float m2c, float off, float (&p)[4]) {
-  const float2 yy = make_float2(y, y), one = make_float2(1.f, 1.f);
-  const float2 u = fmul2(make_float2(__uint_as_float(s[0]), __uint_as_float(s[1])), yy), v = fmul2(make_float2(__uint_as_float(s[2]), __uint_as_float(s[3])), yy);
-  const float2 ab = fadd2(make_float2(ex2_(fminf(u.x, 30.f)), ex2_(fminf(u.y, 30.f))), one), cd = fadd2(make_float2(ex2_(fminf(v.x, 30.f)), ex2_(fminf(v.y, 30.f))), one);
-  const float2 prod = fmul2(make_float2(ab.x, cd.x), make_float2(ab.y, cd.y));
-  const float r = rcp_(prod.x * prod.y) * m2c;
-  const float2 rr = fmul2(make_float2(prod.y, prod.x), make_float2(r, r));      // m2c / ab, m2c / cd
-  float2 lo = make_float2(off, off), hi = lo;
-  ffma2(lo, make_float2(rr.x, rr.x), make_float2(ab.y, ab.x));
-  ffma2(hi, make_float2(rr.y, rr.y), make_float2(cd.y, cd.x));
-  p[0] = ex2_(lo.x); p[1] = ex2_(lo.y); p[2] = ex2_(hi.x); p[3] = ex2_(hi.y);
-}
-
-// meeting of the 128 threads of a lane quadrant (barriers 1-4); true when any of them brings true
-__device__ __forceinline__ bool wt_meet_any(int q, bool v) {
-  uint32_t out;
-  asm volatile(
-      "{\n\t.reg .pred p, r;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "barrier.cta.red.or.pred r, %2, 128, p;\n\t"
-      "selp.u32 %0, 1, 0, r;\n\t}"
-      : "=r"(out) : "r"((uint32_t)v), "r"(q + 1) : "memory");
-  return out != 0;
-}
-__device__ __forceinline__ void wt_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-  uint32_t x[16], y[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) { x[i] = r[i]; y[i] = r[16 + i]; }
-  tmem_st16(taddr, x);
-  tmem_st16(taddr + 16, y);
-}
 constexpr float WT_LAZY = 40.f;    // log2 units
 
 struct WtParams { WinArgs a; int* error_word; };
@@ -186,7 +126,7 @@ window_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQ, const __
         const uint32_t v_addr = smem_u32(ring + s * WT_TILE);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {      // 16 keys per step: 8 columns of P
-          const uint64_t bd = desc_mn(v_addr + ks * 2048, WT_BLK, 1024);
+          const uint64_t bd = smem_desc_mn(v_addr + ks * 2048);
           umma_ts(tmem_base + WT_O, tmem_base + WT_PHI + ks * 8, bd, IDESC_PV, (j | ks) ? 1u : 0u);
           umma_ts(tmem_base + WT_O, tmem_base + WT_PLO + ks * 8, bd, IDESC_PV, 1u);
         }
@@ -238,12 +178,12 @@ window_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQ, const __
           for (int i = 0; i < 32; i += 2) mx = fmax3(mx, __uint_as_float(ra[i]), __uint_as_float(ra[i + 1]));
           if constexpr (!SLOPED) mx *= sl2;
         }
-        if (wt_meet_any(q, mx > ref + WT_LAZY)) {           // some row's reference moves
+        if (meet_any(q, mx > ref + WT_LAZY)) {           // some row's reference moves
           sh.stat[cq][r] = mx;
-          wt_meet_any(q, false);
+          meet_any(q, false);
           const float m = fmaxf(fmaxf(sh.stat[0][r], sh.stat[1][r]), fmaxf(sh.stat[2][r], sh.stat[3][r]));
           float fac = 1.f;
-          if (m > ref + WT_LAZY) { fac = ex2_(ref - m); ref = m; }
+          if (m > ref + WT_LAZY) { fac = ex2_approx(ref - m); ref = m; }
           l0 *= fac;
           l1 *= fac;
           if (j > 0) {
@@ -255,11 +195,11 @@ window_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQ, const __
               tmem_ld32_wait(o);
 #pragma unroll
               for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * fac);
-              wt_st32(lane_base + WT_O + cq * 32, o);
+              tmem_st32(lane_base + WT_O + cq * 32, o);
               asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             }
           }
-          wt_meet_any(q, false);                            // stat may be rewritten
+          meet_any(q, false);                            // stat may be rewritten
         }
         if (ok) {
           uint32_t hi[16], lw[16];
@@ -267,8 +207,8 @@ window_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQ, const __
             const float mref = ref == -INFINITY ? 0.f : ref;   // (a row without keys so far: every weight is exp2(-inf))
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
-              const float w0 = ex2_(SLOPED ? __uint_as_float(ra[i]) - mref : fmaf(__uint_as_float(ra[i]), sl2, -mref));
-              const float w1 = ex2_(SLOPED ? __uint_as_float(ra[i + 1]) - mref : fmaf(__uint_as_float(ra[i + 1]), sl2, -mref));
+              const float w0 = ex2_approx(SLOPED ? __uint_as_float(ra[i]) - mref : fmaf(__uint_as_float(ra[i]), sl2, -mref));
+              const float w1 = ex2_approx(SLOPED ? __uint_as_float(ra[i + 1]) - mref : fmaf(__uint_as_float(ra[i + 1]), sl2, -mref));
               l0 += w0;
               l1 += w1;
               const __nv_bfloat162 x = __floats2bfloat162_rn(w0, w1);
@@ -371,7 +311,7 @@ window_prefill_tc_short_kernel(const __grid_constant__ CUtensorMap tmQ, const __
     }
     if (ok) {
       l = (sh.stat[0][r] + sh.stat[1][r]) + (sh.stat[2][r] + sh.stat[3][r]);
-      if (a.sink) l += ex2_(win_sink2(a, h) - ref);
+      if (a.sink) l += ex2_approx(win_sink2(a, h) - ref);
       fence_after_sync();
       tmem_ld32_issue(lane_base + WT_O + cq * 32, ra);
       tmem_ld32_wait(ra);

@@ -63,12 +63,6 @@ struct __align__(16) WtShared {
 constexpr size_t WT_SMEM_BYTES = WT_NS * WT_PAGE_BYTES + 2 * WT_QBLOCK_BYTES + sizeof(WtShared);
 static_assert(WT_SMEM_BYTES <= 232448, "window-score kernel: shared memory budget");
 
-__device__ __forceinline__ float ex2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // a - c in fp32 with a a 16-bit value: one instruction, no separate widening of a (sm_100)
 template <typename T> struct MixedSub;
 template <> struct MixedSub<__nv_bfloat16> {
