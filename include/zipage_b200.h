@@ -267,7 +267,9 @@ int zp_varlen_prefill(const void* q, const void* k, const void* v, const int32_t
  * zeros instead of memory behind it), and a choice of kernel family: ZP_IMPL_AUTO picks the
  * tcgen05 kernel for 16-bit tensors with head_dim 128 (pages: a multiple of 128 keys) and the
  * kernels of zp_varlen_prefill otherwise; ZP_IMPL_SIMT always takes the latter; ZP_IMPL_TCGEN05
- * fails with ZP_ERR_UNSUPPORTED where the tcgen05 kernel cannot run. */
+ * fails with ZP_ERR_UNSUPPORTED where the tcgen05 kernel cannot run.  A row's weights are relative to a score that its
+ * largest may exceed by 2^40 (fp16: 2^12) before the sums are scaled, so values of n keys stay finite up to 2^(88 - log2 n) in magnitude
+ * (zp_window_attention's and zp_latent_prefill's tcgen05 kernels alike). */
 int zp_varlen_prefill_ex(const void* q, const void* k, const void* v, const int32_t* cu_seqlens_q,
                          const int32_t* cu_seqlens_k, const int32_t* block_table, void* out, int B,
                          int max_seqlen_q, int NBmax, int Hq, int Hkv, int D, int BS,

@@ -124,7 +124,6 @@ __device__ __forceinline__ float ld_cluster(const float* p, uint32_t rank) {
   return v;
 }
 
-// 16-byte vector copy helpers
 // ---- kernels that begin while the one before them ends ----------------------------------------------
 // A kernel launched by `launch_early` may start as soon as every block of the kernel before it on the stream has called
 // `let_next_begin` or is done.  All of its threads call `wait_for_previous` first: before it, nothing may be read that an
@@ -145,6 +144,7 @@ static inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int thre
   return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
+// ---- 16-byte vector copies ------------------------------------------------------------------
 __device__ __forceinline__ int4 ld16(const void* p) { return *reinterpret_cast<const int4*>(p); }
 __device__ __forceinline__ void st16(void* p, int4 v) { *reinterpret_cast<int4*>(p) = v; }
 

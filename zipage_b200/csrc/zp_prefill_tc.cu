@@ -5,8 +5,9 @@
 // A work item is two heads of one key/value head over the same 128 queries, so that a key tile is fetched once for
 // both; where a key/value head has an odd number of heads it is two neighbouring query tiles of one head.
 //
-// Measured (32 / 8 heads, bf16; causal count): 1 x 16384 tokens 1.93 ms = 1140 TFLOP/s, 12 prompts of 60 to 1500 tokens 155 us. One
-// query tile a block with a pass for the row maxima and one for the weights (what stood here before): 3.35 ms and 292 us.
+// Measured (32 / 8 heads, bf16; causal count), single calls and SM clock under load: 1 x 16384 tokens 2.11 to 2.17 ms at 1.72 GHz = 1030 TFLOP/s,
+// 4 x 4096 0.63 to 0.65 ms, 12 prompts of 60 to 1500 tokens 155 us at 1.86 GHz. One query tile a block with a pass for the row maxima and one for
+// the weights (what stood here before): 3.46 ms at 1.78 GHz, 1.09 ms, 282 us at 1.96 GHz.
 #include "zp_attn_tc.cuh"
 
 namespace zp {
