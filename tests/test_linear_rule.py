@@ -39,6 +39,8 @@ def test_other_sizes_are_the_layers():
     assert not _small_linear_takes(one, _x())
     assert not _small_linear_takes(_layer(k=0), _x(4, 0))
     assert not _small_linear_takes(_layer(), _x(0)) and not _small_linear_takes(_layer(), _x(SMALL_ROWS + 1))
+    assert _small_linear_takes(_layer(k=4096, n=64), _x(4, 4096)) and not _small_linear_takes(_layer(k=4096 + 32, n=64), _x(4, 4096 + 32))
+    assert _small_linear_takes(_layer(k=64, n=1 << 15), _x()) and not _small_linear_takes(_layer(k=64, n=(1 << 15) + 16), _x())
     assert not _small_linear_takes(_layer(), _x()[0]) and not _small_linear_takes(_layer(), _x()[None])
 
 

@@ -53,10 +53,12 @@ class RMSNorm(nn.Module):
         return rms_norm(x, self.weight, self.eps, residual)
 
 
-# Rows, and entries of the weight, up to which `linear` takes this library's kernel.  At 8 rows it takes 0.55 to 0.8 of cuBLAS's time
+# Rows, entries and sides of the weight up to which `linear` takes this library's kernel.  At 8 rows it takes 0.55 to 0.8 of cuBLAS's time
 # for weights of up to 2^23 entries (2048 x 1024: 2.7 us for 4.8; 6144 x 1024: 4.2 for 5.2); larger weights go either way
 # (8192 x 2048: 7.9 for 8.0; 5120 x 2048: 7.1 for 6.5; 12288 x 4096: 26 for 19), and so do 9 to 32 rows (4096 x 4096: 11.4 for 9.5).
-SMALL_ROWS, SMALL_WEIGHT = 8, 1 << 23
+# A block walks 16 whole rows of the weight, so long ones leave SMs idle (256 x 4096: 7.7 for 8.3; 256 x 8192: 17.9 for 13.1; 32 x 65536: 145 for
+# 13.6), and very many short ones are blocks of no work (32768 x 256: 6.7 for 7.2; 65536 x 128: 9.0 for 7.7).
+SMALL_ROWS, SMALL_WEIGHT, SMALL_K, SMALL_N = 8, 1 << 23, 4096, 1 << 15
 
 
 _linear_forward = nn.Linear.forward
@@ -83,7 +85,7 @@ def _small_linear_takes(layer, x):
         return False
     w, b = layer.weight, layer.bias
     return (type(w) is nn.Parameter and x.layout is w.layout is torch.strided and w.dim() == 2 and x.shape[0] > 0
-            and x.shape[1] == w.shape[1] > 0 and w.numel() <= SMALL_WEIGHT and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype
+            and 0 < x.shape[1] == w.shape[1] <= SMALL_K and w.shape[0] <= SMALL_N and w.numel() <= SMALL_WEIGHT and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype
             and w.device == x.device and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 8 == 0 and w.shape[1] % 32 == 0
             and (w.data_ptr() | x.data_ptr()) % 16 == 0
             and (b is None or b.shape == w.shape[:1] and b.dtype == x.dtype and b.device == x.device and b.is_contiguous()))
