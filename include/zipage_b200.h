@@ -228,7 +228,7 @@ int zp_update_tables(const int32_t* target_table, int32_t* new_table, int32_t* c
  * cache_seqlens [B]; block_table [B, NBmax] (-1 padded).  Scratch from
  * zp_paged_decode_workspace_bytes.  With too little scratch for the split-KV form the call still
  * succeeds, runs one block per (sequence, kv head) and leaves a note in zp_last_error (16-bit caches with
- * head_dim 128 whose tables hold up to 4096 keys split without scratch). */
+ * head_dim 128 whose tables hold up to 4096 keys split without scratch, where B * Hkv is at most 444). */
 size_t zp_paged_decode_workspace_bytes(int B, int Hq, int D, int max_splits);
 int zp_paged_decode(const void* q, const void* k_cache, const void* v_cache,
                     const int32_t* cache_seqlens, const int32_t* block_table, void* out, int B,

@@ -135,6 +135,24 @@ def test_paged_decode_splits(dtype, B, heads, kv_heads, width):
         assert ((out[b, 0].double() - ref).abs() <= 2 * unit * mag + 1e-6).all()
 
 
+@pytest.mark.parametrize("B,kv_heads,width", [(55, 8, 3), (56, 8, 3), (444, 1, 2), (445, 1, 2), (75, 8, 2), (3, 2, 1)])
+def test_paged_decode_of_as_many_splits_as_fit(B, kv_heads, width):
+    """Clusters up to 444 (sequence, key/value head) pairs, two splits with scratch up to 591, none beyond; one page is never split."""
+    from zipage_b200.layers.attention import paged_decode_attention
+    g, D, heads = _gen(B), 128, 2 * kv_heads
+    lens = torch.randint(1, width * 256 + 1, (B,), device="cuda", generator=g, dtype=torch.int32)
+    kc, vc = (torch.randn(40, 256, kv_heads, D, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    table = torch.randint(0, 40, (B, width), device="cuda", generator=g, dtype=torch.int32)      # (pages may be shared)
+    q = torch.randn(B, 1, heads, D, device="cuda", generator=g).to(torch.bfloat16)
+    out = paged_decode_attention(q, kc, vc, lens, table)
+    for b in (0, 1, B // 2, B - 1):
+        n = int(lens[b])
+        k, v = (c[table[b].long()].flatten(0, 1)[:n].double().repeat_interleave(2, 1) for c in (kc, vc))
+        w = torch.softmax(torch.einsum("hd,shd->hs", q[b, 0].double(), k) * D ** -0.5, -1)
+        ref, mag = torch.einsum("hs,shd->hd", w, v), torch.einsum("hs,shd->hd", w, v.abs())
+        assert ((out[b, 0].double() - ref).abs() <= 2.0 ** -8 * 1.1 * 2 * mag + 1e-6).all()      # as in test_paged_decode_splits
+
+
 @pytest.mark.parametrize("offset", [0, 4, 8])
 def test_paged_decode_takes_scratch_of_exactly_the_needed_size(offset):
     """Wherever floats may lie: all splits run, so that the bits are those of a call with plenty, and nothing is noted."""

@@ -186,13 +186,19 @@ static int pick_splits(int B, int Hkv, int NBmax) {
 
 // The mma.sync kernel splits between any two 64-key tiles, and up to 8 splits of a sequence are a cluster that needs no scratch and no
 // second launch.  A cluster takes contexts of up to DEC_CLUSTER_KEYS, where its splits have at most as many keys as two pages;
-// beyond, a small batch needs more than 8 splits to fill the SMs.
-// 4 sequences of 700 to 2304 keys, 16 heads on 8, a layer: 11.7 us (whole pages a split, scratch and a merge kernel: 15.7).
+// beyond, a small batch needs more than 8 splits to fill the SMs.  The splits of all sequences fit the SMs at once (three blocks each):
+// clusters of a second wave cost more than they share out.  A table of one page is not split, and from that many (sequence, key/value head) pairs
+// on the splits are those with scratch: two while they fit four blocks an SM, none beyond.
+// A layer with cold caches (us; 1, 2, 4, 8 splits as clusters; whole pages a split, scratch and a merge of its own before): 4 sequences of
+// 2200 keys, 32 heads on 8: 33, 21, 15.7, 15.7 (25); 8: 34, 23, 21, 30 (35); 16: 40, 36, 44, 48 (47); 32: 60, 77, 71, 88 (70); 64: 129, 117, 117, 151 (116; with
+// scratch 114).  64 of 10 keys, one page: 9.9, 21, 34, 74 (9.9).
 constexpr int64_t DEC_CLUSTER_KEYS = 4096;
+constexpr int64_t DEC_CLUSTER_BLOCKS = 148 * 3;
+static bool takes_cluster(int B, int Hkv, int NBmax, int BS) { return (int64_t)NBmax * BS <= DEC_CLUSTER_KEYS && (int64_t)B * Hkv <= DEC_CLUSTER_BLOCKS; }
 static int pick_cluster(int B, int Hkv, int NBmax, int BS) {
-  const int64_t keys = (int64_t)NBmax * BS, want = (148 * 6 + B * Hkv - 1) / (B * Hkv);      // two rounds of three blocks an SM
+  const int64_t keys = (int64_t)NBmax * BS;
   int s = 1;
-  while (s < 8 && s < want && keys / (2 * s) >= 128) s *= 2;
+  while (s < 8 && keys > 256 && 2 * s * (int64_t)B * Hkv <= DEC_CLUSTER_BLOCKS && keys / (2 * s) >= 128) s *= 2;
   return s;
 }
 
@@ -260,7 +266,7 @@ extern "C" int zp_paged_decode(const void* q, const void* k_cache, const void* v
     workspace = (char*)workspace + (4 - off);
     workspace_bytes = workspace_bytes > 4 - off ? workspace_bytes - (4 - off) : 0;
   }
-  if (mma && (int64_t)NBmax * BS <= zp::DEC_CLUSTER_KEYS) a.nsplit = zp::pick_cluster(B, Hkv, NBmax, BS);
+  if (mma && zp::takes_cluster(B, Hkv, NBmax, BS)) a.nsplit = zp::pick_cluster(B, Hkv, NBmax, BS);
   else if (a.nsplit > 1) {
     const size_t need = (size_t)B * Hkv * a.nsplit * zp::gp_of(G) * (D + 2) * sizeof(float);
     if (!workspace || workspace_bytes < need) {
@@ -307,8 +313,8 @@ extern "C" int zp_paged_decode_noalloc(const void* q, const void* k_cache, const
                                        void* stream) {
   if (B == 0) return ZP_OK;
   ZP_REQUIRE(Hkv > 0 && Hq % Hkv == 0, "zp_paged_decode_noalloc: Hq must be a multiple of Hkv");
-  // The splits of whole pages, which zp_paged_decode makes of tables beyond a cluster's keys and of fp32 caches.  Shorter tables of the
-  // tensor-core form need no scratch, but the limit counts them alike: it depends on the batch, not on the kernel that runs.
+  // The splits of whole pages, which zp_paged_decode makes of tables beyond a cluster's keys, of batches beyond its blocks and of fp32
+  // caches.  The others need no scratch, but the limit counts them alike: it depends on the batch, not on the kernel that runs.
   const int nsplit = zp::pick_splits(B, Hkv, NBmax);
   const size_t need = nsplit > 1
       ? (size_t)B * Hkv * nsplit * zp::gp_of(Hq / Hkv) * (D + 2) * sizeof(float) : 0;
