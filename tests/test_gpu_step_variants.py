@@ -70,6 +70,24 @@ def test_sampler_takes_the_best_of_all_draws(dtype, rows, V, spread):
     assert (upper >= lower * (1 - 1e-5)).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,V", [(1, 70001), (12, 50257), (13, 50257), (27, 25001), (28, 16384), (74, 12288), (75, 70001), (148, 300), (149, 300), (149, 70001), (223, 66000)])
+@pytest.mark.parametrize("given", [True, False])
+def test_sampler_over_the_numbers_of_rows(dtype, rows, V, given):
+    """Where the blocks a row is spread over and their threads change: the sampled token's ratio is the largest up to fp32 roundings."""
+    from zipage_b200.layers import step_ops as P
+    z = (torch.randn(rows, V, device="cuda", generator=_gen(V)) * 2).to(dtype)
+    t = 0.5 + torch.rand(rows, device="cuda", generator=_gen(rows))
+    q = torch.empty(rows, V, device="cuda").exponential_(1.0, generator=_gen(rows + V)) if given else None
+    tok = P.sample(z, t, noise=q, seed=77)
+    q = q.double().clamp_min(1e-10) if given else _draws(77, rows, V)
+    x = z.double() / t.double()[:, None]
+    e = torch.exp(x - x.max(-1, keepdim=True).values)
+    slack = 0.0 if given else 1e-6                        # of the built-in draws, as in the test above
+    lower, upper = (e / (q + slack)).max(-1).values, (e / (q - slack).clamp_min(1e-10)).gather(1, tok[:, None])[:, 0]
+    assert (upper >= lower * (1 - 1e-5)).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows", [1, 2, 7, 8])
 @pytest.mark.parametrize("n_out,k,bias", [(16, 32, False), (40, 96, True), (1000, 1024, True), (256, 2048 + 32, False)])

@@ -338,11 +338,10 @@ __device__ __forceinline__ float exp1_draw(uint64_t seed, uint32_t row, uint32_t
   return -__logf(u);
 }
 
-constexpr int SAMPLE_THREADS = 512;
-constexpr int SAMPLE_SLICE = 4096;    // a row is spread over more blocks while each has this many logits
+constexpr int SAMPLE_SLICE = 6144, SAMPLE_SLICE_MANY = 32768;    // a row is spread over more blocks while each has this many logits
 
-template <typename T, bool GIVEN>      // GIVEN: the draws are given
-__global__ void __launch_bounds__(SAMPLE_THREADS, 3)
+template <typename T, bool GIVEN, int SAMPLE_THREADS>      // GIVEN: the draws are given
+__global__ void __launch_bounds__(SAMPLE_THREADS, SAMPLE_THREADS == 512 ? 3 : 1)
 sample_kernel(const T* __restrict__ logits, const float* __restrict__ temperatures,
               const float* __restrict__ noise, int64_t* __restrict__ out, int V, int slice, uint64_t seed) {
   __shared__ float red[32], share_m, share_z, share_best;
@@ -386,6 +385,7 @@ sample_kernel(const T* __restrict__ logits, const float* __restrict__ temperatur
   };
   auto row_max = [&](float m) -> float {      // over the block, then over the row's blocks
     m = block_max(m, red);
+    if (ranks == 1) return m;
     if (threadIdx.x == 0) share_m = m;
     cluster_sync();
     for (uint32_t k = 0; k < ranks; ++k) m = fmaxf(m, ld_cluster(&share_m, k));
@@ -429,7 +429,8 @@ sample_kernel(const T* __restrict__ logits, const float* __restrict__ temperatur
     if (r > r1) {
       if (r > r0) { r1 = r0; q1 = q0; i1 = i0; r0 = r; q0 = q; i0 = i; }
       else { r1 = r; q1 = q; i1 = i; }
-      if (__float_as_int(r) > *(volatile int*)&bound) atomicMax(&bound, __float_as_int(r));      // (r >= 0: ordered as its bits)
+      if constexpr (!GIVEN)
+        if (__float_as_int(r) > *(volatile int*)&bound) atomicMax(&bound, __float_as_int(r));      // (r >= 0: ordered as its bits)
     }
   };
   const uint32_t hash0 = (uint32_t)seed ^ ((uint32_t)row * 0x9e3779b9u), hash1 = (uint32_t)(seed >> 32) ^ (uint32_t)row;
@@ -465,10 +466,12 @@ sample_kernel(const T* __restrict__ logits, const float* __restrict__ temperatur
     }
   });
   z = block_sum(z, red);
-  if (threadIdx.x == 0) share_z = z;
-  cluster_sync();
-  z = 0.f;
-  for (uint32_t k = 0; k < ranks; ++k) z += ld_cluster(&share_z, k);
+  if (ranks > 1) {
+    if (threadIdx.x == 0) share_z = z;
+    cluster_sync();
+    z = 0.f;
+    for (uint32_t k = 0; k < ranks; ++k) z += ld_cluster(&share_z, k);
+  }
   // the reference's value of a candidate: (exp(x / t - m) / Z) / q
   auto exact = [&](int i, float q) -> float {
     if (i == 0x7fffffff) return -INFINITY;
@@ -498,33 +501,44 @@ sample_kernel(const T* __restrict__ logits, const float* __restrict__ temperatur
     warp_best();
     if (lane == 0) { share_best = best; share_idx = besti; }
   }
-  cluster_sync();
-  if (rank == 0 && w == 0) {
-    best = lane < (int)ranks ? ld_cluster(&share_best, lane) : -INFINITY;
-    besti = lane < (int)ranks ? __float_as_int(ld_cluster(reinterpret_cast<const float*>(&share_idx), lane)) : 0x7fffffff;
-    warp_best();
-    if (lane == 0) out[row] = besti == 0x7fffffff ? 0 : besti;      // (no number in the row is above zero: any token)
+  if (ranks > 1) {
+    cluster_sync();
+    if (rank == 0 && w == 0) {
+      best = lane < (int)ranks ? ld_cluster(&share_best, lane) : -INFINITY;
+      besti = lane < (int)ranks ? __float_as_int(ld_cluster(reinterpret_cast<const float*>(&share_idx), lane)) : 0x7fffffff;
+      warp_best();
+    }
+    cluster_sync();    // (a block's shared memory stays until the others have read it)
   }
-  cluster_sync();      // (a block's shared memory stays until the others have read it)
+  if (rank == 0 && threadIdx.x == 0) out[row] = besti == 0x7fffffff ? 0 : besti;      // (no number in the row is above zero: any token)
 }
 
 template <typename T>
 static int launch_sample(const T* logits, const float* temperatures, const float* noise, int64_t* out, int rows, int V, uint64_t seed, cudaStream_t st) {
-  // (blocks of a row meet four times, which costs more than an even load gains: more than one only where rows leave SMs idle)
+  // Blocks of a row meet four times, which costs more than an even load gains unless SMs idle and a row is long.
+  // 151936 logits, 1, 2, 4, 8 blocks a row (us): 1 row 40, 27, 18, 15; 37: 41, 28, 28, 26; 55: 42, 29, 29, 36; 74: 42, 30, 37, 43; 90: 43, 43, 37, 50; 110: 44,
+  // 44, 49, 58; 222: 74, 64, 83, 105; 300: 103, 95, 101, 138.  32000: 1 row 14, 13, 12, 11; 74: 15, 15, 18, 27; 110: 15, 18, 24, 35.
+  // Given draws are loads: a block of 1024 threads where a row has an SM to itself.  151936 fp32 logits: 1 row 36, 26, 18, 15; 16: 37, 27, 20, 28; 37: 37, 28, 35,
+  // 42; 74: 43, 33, 54, 72; 110: 50, 60, 76, 114.
+  const bool wide = noise && rows <= 148;
+  const int most = wide ? (rows <= 12 ? 8 : rows <= 27 ? 4 : rows <= 74 ? 2 : 1) : rows <= 37 ? 8 : rows <= 100 ? 4 : rows <= 222 ? 2 : 1;
+  const int part = rows <= 74 ? SAMPLE_SLICE : SAMPLE_SLICE_MANY;
   int ranks = 1;
-  while (ranks < 8 && (int64_t)rows * 2 * ranks <= 3 * 148 && V / (2 * ranks) >= SAMPLE_SLICE) ranks *= 2;
+  while (ranks < most && V / (2 * ranks) >= part) ranks *= 2;
   const int slice = ((V + ranks - 1) / ranks + 63) / 64 * 64;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)rows * ranks);
-  cfg.blockDim = dim3(SAMPLE_THREADS);
-  cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = ranks; attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  const cudaError_t e = noise ? cudaLaunchKernelEx(&cfg, sample_kernel<T, true>, logits, temperatures, noise, out, V, slice, seed)
-                              : cudaLaunchKernelEx(&cfg, sample_kernel<T, false>, logits, temperatures, noise, out, V, slice, seed);
+  auto run = [&](auto kernel, int threads) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)rows * ranks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = ranks; attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = ranks > 1;      // (a block alone is a cluster as it is)
+    return cudaLaunchKernelEx(&cfg, kernel, logits, temperatures, noise, out, V, slice, seed);
+  };
+  const cudaError_t e = !noise ? run(sample_kernel<T, false, 512>, 512) : wide ? run(sample_kernel<T, true, 1024>, 1024) : run(sample_kernel<T, true, 512>, 512);
   if (e != cudaSuccess) { set_error("zp_sample: %s", cudaGetErrorString(e)); return ZP_ERR_CUDA; }
   return check_launch("zp_sample");
 }
