@@ -359,3 +359,18 @@ def test_which_windows_go_in_pairs(heads, kv_heads, lens, context, window, softc
 ])
 def test_which_windows_of_small_heads_take_tcgen05(lens, context, kernel):
     assert _plain_windows(16, 4, 64, lens, context, 0, 0.0) == kernel
+
+
+@pytest.mark.parametrize("B", [4, 5])                    # 128 tiles, of an SM each; 160 in pairs of heads
+def test_prompts_of_about_as_many_tiles_as_sms(B):
+    from zipage_b200.layers.attention import varlen_prefill_attention
+    heads, kv_heads, x, y = 32, 8, 33, 700
+    g = torch.Generator(device="cuda").manual_seed(B)
+    n = lambda rows, h: torch.randn(rows, h, D, device="cuda", generator=g).to(torch.bfloat16)
+    q, k, v = n(x * B, heads), n(y * B, kv_heads), n(y * B, kv_heads)
+    out = varlen_prefill_attention(q, k, v, x, _cu([x] * B), y, _cu([y] * B))
+    _no_device_error()
+    seen = torch.arange(y, device="cuda")[None] <= torch.arange(x, device="cuda")[:, None] + y - x
+    for b in range(B):
+        ref, mag = _softmax(q[b * x:b * x + x], k[b * y:b * y + y], v[b * y:b * y + y], D ** -0.5, seen)
+        assert ((out[b * x:b * x + x].double() - ref).abs() <= 2.0 ** -8 * 1.1 * 2 * mag + 1e-6).all()      # as in test_prefill_edges

@@ -570,14 +570,19 @@ static inline Rings rings_of(int nbq, int nbv) {
   return g;
 }
 
-// Pairs, unless every tile can have an SM to itself (an estimate from the rows of all sequences: the counts are on the device): a
-// launch that short is one tile's latency, which the second tile of a pair only adds to.
+// The most 128-row query tiles that the sequences can have, all heads (the counts are on the device).
+static inline int64_t most_tiles(int heads, int B, int total_q, int max_q) {
+  const int64_t by_rows = (int64_t)total_q / 128 + B, by_longest = (int64_t)B * ((max_q + 127) / 128);
+  return heads * (by_rows < by_longest ? by_rows : by_longest);
+}
+// Pairs, unless every tile can have an SM to itself: a launch that short is one tile's latency, which the second tile of a pair only adds to.
 // Prompts, single tiles / pairs: 1 x 100 tokens, 32 heads: 10.3 / 12.1 us; 4 of up to 400, 8 heads: 20.3 / 22.1; 16 of up to 100,
-// 16 heads (about 256 tiles by this count): 51.5 / 32.5.
+// 16 heads (256 tiles): 51.5 / 32.5.  (One query tile a block with a pass for the maxima and one for the weights, as it was before, had all its softmax
+// warps on that tile: at up to 148 tiles it took 0 to 3 us less of 10 to 30, from there on 1.2 to 3.5 times as long.)
 // (Windows and latents of few tiles have kernels of their own, and no single tiles here.)
 static inline int pick_pair(int heads_per_kv) { return heads_per_kv % 2 == 0 ? PAIR_HEADS : PAIR_ROWS; }
-static inline int pick_mode(int heads, int heads_per_kv, int B, int total_q) {
-  return (int64_t)heads * (total_q / 128 + B) <= 148 ? SINGLE : pick_pair(heads_per_kv);
+static inline int pick_mode(int heads, int heads_per_kv, int B, int total_q, int max_q) {
+  return most_tiles(heads, B, total_q, max_q) <= 148 ? SINGLE : pick_pair(heads_per_kv);
 }
 static inline dim3 grid_of(int mode, int heads, int B, int max_q, int& levels) {
   const int rows = mode == PAIR_ROWS ? 256 : 128;

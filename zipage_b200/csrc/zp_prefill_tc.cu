@@ -96,7 +96,7 @@ static int launch_prefill_tc(const void* q, const void* k, const void* v, Prefil
   if (int rc = make_tensor_map_5d(&p.tmV, UmmaFmt<T>::tm, v, dims, strides, box, sizeof(T))) return rc;
   p.rings = rings_of(2, 2);
   p.dv = 128;
-  p.mode = pick_mode(p.Hq, p.Hq / p.Hkv, B, total_q);
+  p.mode = pick_mode(p.Hq, p.Hq / p.Hkv, B, total_q, max_seqlen_q);
   const dim3 grid = grid_of(p.mode, p.Hq, B, max_seqlen_q, p.levels);
   return launch_attn(p, grid, st, "zp_varlen_prefill(tcgen05)");
 }
