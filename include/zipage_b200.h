@@ -319,6 +319,16 @@ int zp_qk_norm_rope_store(const void* qkv, const int64_t* positions, const float
                           int Hq, int Hkv, int D, int64_t qkv_stride, int64_t cache_stride_seq,
                           int64_t cache_stride_slot, int dtype, void* stream);
 
+/* The same, with the values packed as well: v_out [n_tokens, Hkv, D] or NULL (for attention over the rows themselves, which the
+ * reference hands a packed copy). */
+int zp_qk_norm_rope_store_v(const void* qkv, const int64_t* positions, const float* cos_sin,
+                            const void* q_weight, const void* k_weight, float eps, void* q_out,
+                            void* k_out, void* v_out, void* k_cache, void* v_cache, const int32_t* slot_mapping,
+                            void* query_cache, const int32_t* triples, int n_triples,
+                            const int32_t* n_triples_device, int n_tokens,
+                            int Hq, int Hkv, int D, int64_t qkv_stride, int64_t cache_stride_seq,
+                            int64_t cache_stride_slot, int dtype, void* stream);
+
 /* Replaces Sampler.calculate_probs + Sampler.sample, zipage/layers/sampler.py:17-31.
  * logits [n_rows, vocab] T, temperatures [n_rows] fp32; tokens_out [n_rows] int64 =
  * argmax(softmax(fp32 logits / T) / max(noise, 1e-10)), lowest index on ties.  noise [n_rows,

@@ -35,6 +35,35 @@ def test_qk_norm_rope_is_the_same_for_few_and_many_tokens(dtype, heads, kv_heads
         assert torch.equal(x, y)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("N", [1, 37, 1023, 1025])
+@pytest.mark.parametrize("kv_heads,D", [(8, 128), (3, 64)])
+@pytest.mark.parametrize("stored", [True, False])
+def test_values_are_packed_beside_the_keys(dtype, N, kv_heads, D, stored):
+    """With `return_k` v is a packed copy of qkv's columns, rows without a cache slot among them; without it a view."""
+    from zipage_b200.layers import step_ops as P
+    g, heads, dev = _gen(N), 4, "cuda"
+    wide = torch.randn(N, (heads + 2 * kv_heads) * D + 16, device=dev, generator=g).to(dtype)
+    qkv = wide[:, :-16]                                   # (rows further apart than they are long)
+    pos, cs = torch.randint(0, 4096, (N,), device=dev, generator=g), P.rope_cos_sin_cache(D, 4096, 1e6, dev)
+    w = [torch.ones(D, device=dev, dtype=dtype)] * 2
+    cache = {}
+    if stored:
+        slot = torch.randperm(1280, device=dev, generator=g)[:N].to(torch.int32)
+        slot[::5] = -1
+        cache = dict(k_cache=torch.zeros(5, 256, kv_heads, D, dtype=dtype, device=dev), v_cache=torch.zeros(5, 256, kv_heads, D, dtype=dtype, device=dev),
+                     slot_mapping=slot)
+    want = qkv[:, (heads + kv_heads) * D:].unflatten(1, (kv_heads, D))
+    _, _, v = P.qk_norm_rope_store(qkv, pos, cs, *w, 1e-6, heads, kv_heads, D, **cache)
+    assert v.is_contiguous() and torch.equal(v, want)
+    if stored:
+        rows = torch.zeros(1280, kv_heads, D, dtype=dtype, device=dev)
+        rows[slot[slot >= 0].long()] = want[slot >= 0]
+        assert torch.equal(cache["v_cache"].view(1280, kv_heads, D), rows)
+    _, k, v = P.qk_norm_rope_store(qkv, pos, cs, *w, 1e-6, heads, kv_heads, D, return_k=False)
+    assert k is None and v.data_ptr() == want.data_ptr() and torch.equal(v, want)
+
+
 def _draws(seed, rows, V):
     """The Exp(1) draws of the built-in generator (fp64 logarithm of the same uniform numbers)."""
     m = 0xFFFFFFFF

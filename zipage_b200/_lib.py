@@ -87,6 +87,7 @@ SIGNATURES = {
     "zp_silu_and_mul": (_I, [_P, _P, _I, _I, _I, _P]),
     "zp_small_linear": (_I, [_P, _L, _P, _P, _P, _I, _I, _I, _I, _P]),
     "zp_qk_norm_rope_store": (_I, [_P] * 5 + [_F] + [_P] * 7 + [_I, _P] + [_I] * 4 + [_L] * 3 + [_I, _P]),
+    "zp_qk_norm_rope_store_v": (_I, [_P] * 5 + [_F] + [_P] * 8 + [_I, _P] + [_I] * 4 + [_L] * 3 + [_I, _P]),
     "zp_sample": (_I, [_P, _P, _P, _P, _I, _I, C.c_uint64, _I, _P]),
     "zp_decode_inputs": (_I, [_P, _P, _P, _L, _P, _I, _I, _P, _P, _P, _P, _I, _I, _P]),
     "zp_prepare_decode": (_I, [_P, _P, _P, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P]),

@@ -163,7 +163,7 @@ silu_and_mul_kernel(const T* x, T* out, int I, Index total_vec) {
 // Fused q/k RMSNorm + rotary embedding + cache writes.  A warp walks some heads of one kind (q, k or v) of one token, four at a
 // time (eight lanes per head; a lane owns D/16 consecutive dims of each half of the head — the rotation pairs dim d with d + D/2
 // — and moves them as one vector), with the next four heads' loads in flight: q heads -> q_out; k heads -> k_out and the K
-// cache; v heads -> the V cache, a plain copy.  Rows past the tokens redo the q heads of a window token and write them into
+// cache; v heads -> v_out (packed, as attention over the rows themselves takes them) and the V cache, a plain copy.  Rows past the tokens redo the q heads of a window token and write them into
 // the observation-window buffer.
 //
 // What bounds it is the loads in flight: with one kind of head a warp keeps one weight and the token's cosines and sines in
@@ -178,7 +178,7 @@ constexpr int QK_SPREAD = 1024;
 struct QkArgs {
   const void* qkv; const int64_t* positions; const float* cos_sin;
   const void* q_weight; const void* k_weight;
-  void* q_out; void* k_out; void* k_cache; void* v_cache;
+  void* q_out; void* k_out; void* v_out; void* k_cache; void* v_cache;
   const int32_t* slot_mapping; void* query_cache; const int32_t* triples;
   const int32_t* n_triples_dev;   // NULL, or the device word that holds the number of valid triples
   int n_tokens, n_triples, Hq, Hkv;
@@ -268,12 +268,14 @@ __global__ void __launch_bounds__(256) qk_norm_rope_store_kernel(const QkArgs a)
   load_head(h_begin + hg, ca, cb);
   const int slot = !is_q && a.slot_mapping ? a.slot_mapping[n] : -1;
   if (is_v) {
-    if (slot == -1) return;
-    T* dst = reinterpret_cast<T*>(a.v_cache) + (int64_t)slot * a.Hkv * D;
+    if (slot == -1 && !a.v_out) return;
+    T* d0 = a.v_out ? reinterpret_cast<T*>(a.v_out) + (int64_t)n * a.Hkv * D : nullptr;
+    T* d1 = slot != -1 ? reinterpret_cast<T*>(a.v_cache) + (int64_t)slot * a.Hkv * D : nullptr;
     for (int h = h_begin + hg; h < h_end; h += 4) {
       load_head(h + 4, na, nb);
-      st_chunk<T, P>(dst + (int64_t)h * D + l8 * P, ca);
-      st_chunk<T, P>(dst + (int64_t)h * D + D / 2 + l8 * P, cb);
+      const int64_t at = (int64_t)h * D + l8 * P;
+      if (d0) { st_chunk<T, P>(d0 + at, ca); st_chunk<T, P>(d0 + at + D / 2, cb); }
+      if (d1) { st_chunk<T, P>(d1 + at, ca); st_chunk<T, P>(d1 + at + D / 2, cb); }
       ca = na; cb = nb;
     }
     return;
@@ -676,9 +678,9 @@ extern "C" int zp_silu_and_mul(const void* x, void* out, int n_rows, int inter, 
   return zp::check_launch("zp_silu_and_mul");
 }
 
-extern "C" int zp_qk_norm_rope_store(const void* qkv, const int64_t* positions, const float* cos_sin,
+extern "C" int zp_qk_norm_rope_store_v(const void* qkv, const int64_t* positions, const float* cos_sin,
                                      const void* q_weight, const void* k_weight, float eps,
-                                     void* q_out, void* k_out, void* k_cache, void* v_cache,
+                                     void* q_out, void* k_out, void* v_out, void* k_cache, void* v_cache,
                                      const int32_t* slot_mapping, void* query_cache,
                                      const int32_t* triples, int n_triples,
                                      const int32_t* n_triples_device, int n_tokens, int Hq,
@@ -693,14 +695,14 @@ extern "C" int zp_qk_norm_rope_store(const void* qkv, const int64_t* positions, 
     const size_t es = zp::dtype_size(dtype);
     const size_t vec = (D / 16) * es > 16 ? 16 : (D / 16) * es;   // the widest vector access used
     ZP_REQUIRE(((uintptr_t)qkv | (uintptr_t)q_weight | (uintptr_t)k_weight | (uintptr_t)q_out |
-                (uintptr_t)k_out | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)query_cache |
+                (uintptr_t)k_out | (uintptr_t)v_out | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)query_cache |
                 (uintptr_t)cos_sin) % 16 == 0 && (qkv_stride * es) % vec == 0 &&
                    (cache_stride_seq * es) % vec == 0 && (cache_stride_slot * es) % vec == 0,
                "zp_qk_norm_rope_store: pointers must be 16-byte aligned and strides vector-aligned");
   }
   zp::QkArgs a;
   a.qkv = qkv; a.positions = positions; a.cos_sin = cos_sin; a.q_weight = q_weight; a.k_weight = k_weight;
-  a.q_out = q_out; a.k_out = k_out; a.k_cache = k_cache; a.v_cache = v_cache;
+  a.q_out = q_out; a.k_out = k_out; a.v_out = v_out; a.k_cache = k_cache; a.v_cache = v_cache;
   a.slot_mapping = slot_mapping; a.query_cache = query_cache; a.triples = triples;
   a.n_triples_dev = n_triples_device;
   a.n_tokens = n_tokens; a.n_triples = n_triples; a.Hq = Hq; a.Hkv = Hkv;
@@ -716,6 +718,18 @@ extern "C" int zp_qk_norm_rope_store(const void* qkv, const int64_t* positions, 
     else zp::launch_early(zp::qk_norm_rope_store_kernel<T, 64>, grid, 256, 0, st, a);
   });
   return zp::check_launch("zp_qk_norm_rope_store");
+}
+
+extern "C" int zp_qk_norm_rope_store(const void* qkv, const int64_t* positions, const float* cos_sin,
+                                     const void* q_weight, const void* k_weight, float eps,
+                                     void* q_out, void* k_out, void* k_cache, void* v_cache,
+                                     const int32_t* slot_mapping, void* query_cache,
+                                     const int32_t* triples, int n_triples,
+                                     const int32_t* n_triples_device, int n_tokens, int Hq,
+                                     int Hkv, int D, int64_t qkv_stride, int64_t cache_stride_seq,
+                                     int64_t cache_stride_slot, int dtype, void* stream) {
+  return zp_qk_norm_rope_store_v(qkv, positions, cos_sin, q_weight, k_weight, eps, q_out, k_out, nullptr, k_cache, v_cache, slot_mapping, query_cache,
+                                 triples, n_triples, n_triples_device, n_tokens, Hq, Hkv, D, qkv_stride, cache_stride_seq, cache_stride_slot, dtype, stream);
 }
 
 extern "C" int zp_sample(const void* logits, const float* temperatures, const float* noise,

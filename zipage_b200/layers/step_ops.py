@@ -139,7 +139,8 @@ def qk_norm_rope_store(qkv, positions, cos_sin, q_weight, k_weight, eps, num_hea
     given, K/V rows written to the paged caches at slot_mapping and window queries written to
     query_cache at the (row, query_id, index) triples — one launch.  `query_slot_count`: a device
     int32 tensor with the number of valid rows of `query_slot_mapping` (as `prepare_decode` returns
-    it); without it every row is taken."""
+    it); without it every row is taken.  v [N,Hkv,D]: a packed copy with `return_k` (whose caller
+    attends over the rows themselves), else a view of qkv."""
     L.require_cuda(qkv, positions, cos_sin, q_weight, k_weight, k_cache, v_cache, slot_mapping,
                    query_cache, query_slot_mapping, query_slot_count)
     N = qkv.shape[0]
@@ -147,19 +148,20 @@ def qk_norm_rope_store(qkv, positions, cos_sin, q_weight, k_weight, eps, num_hea
     assert qkv.shape[1] == (Hq + 2 * Hkv) * D and qkv.stride(1) == 1
     assert positions.dtype == torch.int64 and cos_sin.dtype == torch.float32 and cos_sin.is_contiguous()
     q = torch.empty((N, Hq, D), dtype=qkv.dtype, device=qkv.device)
-    k = torch.empty((N, Hkv, D), dtype=qkv.dtype, device=qkv.device) if return_k else None
+    k, v = (torch.empty((N, Hkv, D), dtype=qkv.dtype, device=qkv.device) if return_k else None for _ in range(2))
     ntrip = 0 if query_slot_mapping is None else query_slot_mapping.shape[0]
     cs_seq = query_cache.stride(0) if query_cache is not None else 0
     cs_slot = query_cache.stride(1) if query_cache is not None else 0
     if k_cache is not None:
         assert k_cache.is_contiguous() and v_cache.is_contiguous()
-    L.check(L.load().zp_qk_norm_rope_store(
+    L.check(L.load().zp_qk_norm_rope_store_v(
         L.ptr(qkv), L.ptr(positions), L.ptr(cos_sin), L.ptr(q_weight), L.ptr(k_weight), float(eps),
-        L.ptr(q), L.ptr(k), L.ptr(k_cache), L.ptr(v_cache), L.ptr(slot_mapping), L.ptr(query_cache),
+        L.ptr(q), L.ptr(k), L.ptr(v), L.ptr(k_cache), L.ptr(v_cache), L.ptr(slot_mapping), L.ptr(query_cache),
         L.ptr(query_slot_mapping), ntrip, L.ptr(query_slot_count), N, Hq, Hkv, D, qkv.stride(0), cs_seq, cs_slot,
         L.dtype_code(qkv), L.stream_ptr()), "qk_norm_rope_store")
     _count(1)
-    v = qkv[:, (Hq + Hkv) * D:].view(N, Hkv, D)
+    if v is None:
+        v = qkv[:, (Hq + Hkv) * D:].view(N, Hkv, D)
     return q, k, v
 
 
