@@ -213,6 +213,25 @@ def test_prompts_whose_reference_moves(dtype, heads, kv_heads):
         a, b = a + x, b + y
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("key", [0, 31, 63, 64, 100, 127])
+@pytest.mark.parametrize("heads", [2, 40])               # a tile an SM (two groups of warps share a row) and pairs of tiles
+def test_prompts_whose_reference_moves_in_one_half_of_a_row(dtype, key, heads):
+    """One key of the third and of the fourth tile is far above all others: the half of the row without it has to follow."""
+    from zipage_b200.layers.attention import varlen_prefill_attention
+    n = 600
+    g = torch.Generator(device="cuda").manual_seed(key)
+    q, k, v = (torch.randn(n, heads, D, device="cuda", generator=g).to(dtype) for _ in range(3))
+    q[..., 0], k[..., 0] = 24.0, 0.0
+    k[256 + key, :, 0], k[384 + key, :, 0] = 24.0, 64.0   # 73 and 196 powers of two
+    out = varlen_prefill_attention(q, k, v, n, _cu([n]), n, _cu([n]), impl="tcgen05")
+    _no_device_error()
+    seen = torch.arange(n, device="cuda")[None] <= torch.arange(n, device="cuda")[:, None]
+    ref, mag = _softmax(q, k, v, D ** -0.5, seen)
+    unit = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * 1.1      # as in test_prefill_edges
+    assert ((out.double() - ref).abs() <= (unit * 2 + CLIMB_ERROR) * mag + 1e-6).all()
+
+
 @pytest.mark.parametrize("many", [False, True])          # launches of few and of many query tiles
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(8, 4, 128, 128), (6, 2, 48, 16), (3, 3, 72, 104)])
 @pytest.mark.parametrize("softcap,steep,window", [(30.0, False, 300), (0.0, True, 0), (0.0, True, 300)])

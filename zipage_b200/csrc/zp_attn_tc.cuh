@@ -12,12 +12,21 @@
 // when a score exceeds it by more than P::LAZY powers of two, which floats of either size carry without loss; a kernel
 // whose scores are bounded has a fixed one.
 //
-// What bounds it: per 128 x 128 scores the two products take 1024 clocks of the tensor pipe (1536 with hi + lo) and the
-// exponentials 1024 of the special-function unit, so neither may wait for the other; two tiles in flight hide the
-// softmax's latency, and as a thread owns a whole row no maximum or sum ever crosses threads.
+// What bounds it: the chain of a tile's step.  Per 128 x 128 scores the two products take 1024 clocks of the tensor pipe (1536 with hi +
+// lo) and the exponentials 1024 of the special-function unit, but a step of two tiles takes 3500 to 4000: with one warp per 32
+// rows 1040 clocks until the next scores are there (the rest of the second product, the first one, three hand-overs), 360 to load them,
+// 310 for the maximum, 1870 for exponentials and weights (12 to 13 a pair of numbers; a third of all issue slots are used, a fifth of the
+// warps' time goes into fetching instructions), 190 for the last hand-over.  On long prompts the clock falls from 1.83 to 1.6 GHz
+// (power), so that instructions count as much as clocks.
+//
+// Softmax warps: P::GROUPS groups of four a tile.  One group: a thread owns a whole row and no maximum or sum ever crosses threads.
+// Two groups split a row's keys and exchange its maximum through shared memory: half the loads, comparisons and exponentials follow
+// one another, for half as many instructions again.  That is the better way where one tile has the SM to itself (prompts of up to 148
+// tiles, 3 of 60 to 400 tokens: the call 48 -> 40 us), where a score costs more (capped windows 368 -> 342, uncapped 334 -> 325, latents 476 -> 470), and the
+// worse one for pairs of tiles of long prompts (16384 tokens 2.29 -> 2.36 ms) and biased windows (385 -> 421).
 //
 // Roles (one block per SM): warp 0 = work, TMA loads and TMEM, warp 1 = products, from warp 4 on softmax, P::GROUPS groups of
-// four warps a tile (two split its columns), which take over registers of the first group.  One thread issues the
+// four warps a tile, which take over registers of the first group.  One thread issues the
 // products of both tiles in turn, which keeps them half a step apart (with an issuer per tile they fell into step and
 // overlapped less: 2.43 ms at 1 x 16384).  Its MMAs run in order, so S_t of the next key tile is issued right behind the product that
 // reads p from the same columns.  A wait costs it some 200 clocks even where it is over, more than the MMAs behind it take
@@ -64,8 +73,8 @@ struct Item {
 struct __align__(16) Shared {
   uint4 work;                            // answer of cluster launch control
   Item item[2];                          // what the producer found, for the other roles
-  uint64_t wfull, ifull[2], iempty[2], qfull, qempty, kfull[NBAR], kempty[NBAR], vfull[NBAR], vempty[NBAR], sfull[2], pfull[2][2], pvdone[2], lfull[2];
-  float sum[2][2][128];                  // row sums of the column halves of each tile
+  uint64_t wfull, ifull[2], iempty[2], qfull, qempty, kfull[NBAR], kempty[NBAR], vfull[NBAR], vempty[NBAR], sfull[2], pfull[2][2], pvdone[2];
+  float rows[2][2][128];                 // of the column halves of each tile: a step's maxima, an item's sums
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -114,7 +123,7 @@ struct Factor {
 
 // What P has to bring:
 //   T                            element type;  SPLIT: weights as hi + lo (T = bf16);  MASKED: rows have a first visible key too
-//   GROUPS                       1, or 2 where the reference is fixed (halves of a row need no common maximum then)
+//   GROUPS                       groups of softmax warps a tile: 1, or 2 (CAPPED: 2)
 //   LAZY                         powers of two by which a score may exceed its row's reference;  CAPPED: the reference is fixed
 //   rings, error_word            members
 //   item(id, it)                 the work of block `id`; false: none
@@ -132,8 +141,10 @@ struct Factor {
 template <class P>
 __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const __grid_constant__ P p) {
   using T = typename P::T;
-  constexpr int GROUPS = P::GROUPS, COLS = 128 / GROUPS;      // columns of a group
-  static_assert(GROUPS == 1 || P::CAPPED, "one maximum per row");
+  constexpr int GROUPS = P::GROUPS, COLS = 128 / GROUPS, CHUNKS = COLS / 32;      // columns of a group
+  constexpr int UNIT = 64 / GROUPS;      // keys that a group hands over at a time
+  constexpr bool LATE = GROUPS == 1 && !P::SPLIT;      // the first of them behind half of the second's exponentials
+  static_assert(GROUPS == 2 || !P::CAPPED, "capped scores come in halves of a row");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* qbuf = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   if (qbuf - smem_raw > SLACK) {         // (no room for more padding)
@@ -148,8 +159,8 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&sh.ifull[i], 1); mbar_init(&sh.iempty[i], 1 + 8 * GROUPS);
-      mbar_init(&sh.sfull[i], 1); mbar_init(&sh.pvdone[i], 1); mbar_init(&sh.lfull[i], 8);
-      for (int u = 0; u < 2; ++u) mbar_init(&sh.pfull[i][u], 4);
+      mbar_init(&sh.sfull[i], 1); mbar_init(&sh.pvdone[i], 1);
+      for (int u = 0; u < 2; ++u) mbar_init(&sh.pfull[i][u], 4 * GROUPS);
     }
     mbar_init(&sh.wfull, 1); mbar_init(&sh.qfull, 1);
     mbar_init(&sh.qempty, 1);
@@ -293,16 +304,15 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
               const uint32_t pt = tmem + t * 128, ot = tmem + O_COL + t * 128;
 #pragma unroll
               for (int u = 0; u < 2; ++u) {                  // the softmax hands over 64 keys at a time
-                // an item's first product overwrites all of O: both groups have to be past the item before, whose output they read there
-                const bool first = GROUPS == 2 && j == 0;
-                if (first && u == 0) ok = ok && mbar_wait(&sh.pfull[t][1], cnt[t] & 1, abortp, p.error_word, 840);
-                if (!first || u == 0) ok = ok && mbar_wait(&sh.pfull[t][u], cnt[t] & 1, abortp, p.error_word, 831);
+                // (an item's first product overwrites all of O: every softmax warp of the tile is past the item before, whose output it read there)
+                ok = ok && mbar_wait(&sh.pfull[t][u], cnt[t] & 1, abortp, p.error_word, 831);
                 if (!ok) continue;
                 fence_after_sync();
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {                // 16 keys a step: 8 columns of p
-                  const uint64_t bd = smem_desc_mn(v0 + (4 * u + c) * 2048);
-                  const uint32_t a = pt + u * 64 + (c >> 1) * 32 + (c & 1) * 8;
+                  const int key16 = GROUPS == 2 ? (c >> 1) * 4 + 2 * u + (c & 1) : 4 * u + c;
+                  const uint64_t bd = smem_desc_mn(v0 + key16 * 2048);
+                  const uint32_t a = pt + (key16 >> 1) * 32 + (key16 & 1) * 8;
                   umma_ts(ot, a, bd, id_o, (j | u | c) ? 1u : 0u);
                   if (P::SPLIT) umma_ts(ot, a + 16, bd, id_o, 1u);
                 }
@@ -330,7 +340,14 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
     const int grp = (warp - 4) >> 2, t = grp / GROUPS, half = grp % GROUPS, quad = warp & 3;      // tile, its columns, TMEM lane quadrant
     const int r = quad * 32 + lane;                                                              // row of the tile
     const uint32_t lanes = tmem + (static_cast<uint32_t>(quad * 32) << 16), st = lanes + t * 128, ot = lanes + O_COL + t * 128;
-    uint32_t tiles = 0, cnt = 0, ends = 0, vslot = 0;      // key tiles of the items before, steps and items of this tile, place in the value ring
+    // Meeting of the two warps with the same rows; false: the block is giving up.  (A warp that leaves early arrives once more: the other one
+    // can be at one meeting at most before it sees the abort flag, which was raised before.)
+    const int pair = 1 + t * 4 + quad;
+    auto meet = [&]() -> bool {
+      asm volatile("barrier.cta.sync %0, 64;" ::"r"(pair) : "memory");
+      return __all_sync(0xffffffffu, !*abortp);
+    };
+    uint32_t tiles = 0, cnt = 0, vslot = 0;      // key tiles of the items before, steps of this tile, place in the value ring
     bool ok = true;
     for (uint32_t w = 0; ok; ++w) {
       ok = mbar_wait_warp(&sh.ifull[w & 1], (w >> 1) & 1, abortp, p.error_word, 832);
@@ -359,6 +376,26 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
           if constexpr (P::MASKED) m &= ~low_bits(row.lo - key) | low_bits(row.keep - key);
           return m;
         };
+        // UNIT keys' weights are written.  Value rows past the sequence become zeros (0 times another sequence's values could be
+        // NaN): those that the product behind this hand-over reads, whichever tile's comes first
+        auto hand_over = [&](int u) {
+          if (dry) return;
+          const int first = half * COLS + UNIT * u, left = max(it.keys - it.key0(j) - first, 0);
+          if (left < UNIT) {
+            const uint32_t k = tiles + j;
+            ok = mbar_wait_warp(&sh.vfull[k % NBAR], (k / NBAR) & 1, abortp, p.error_word, 835);
+#pragma unroll 1
+            for (int i = r; ok && i < (UNIT - left) * 8 * g.nbv; i += 128) {
+              const int line = i >> 3, blk = line / (UNIT - left), key = first + left + line % (UNIT - left);
+              *reinterpret_cast<int4*>(vring + (vslot * g.nbv + blk) * BLK + key * 128 + ((i & 7) << 4)) = make_int4(0, 0, 0, 0);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          }
+          tmem_st_wait();
+          fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh.pfull[t][u]);
+        };
         // weights of 32 keys, over their scores: hi in the first 16 columns, lo in the others
         auto weights = [&](uint32_t (&s)[32], int c, float mref) {
           const uint32_t y = P::CAPPED && !whole ? seen(key0 + c) : 0xffffffffu, at = st + half * COLS + c;
@@ -386,38 +423,27 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
             l2 = fadd2(l2, fadd2(make_float2(wt[0], wt[1]), make_float2(wt[2], wt[3])));
 #pragma unroll
             for (int u = 0; u < 4; u += 2) {
-              const typename Pair<T>::V x = Pair<T>::pack(wt[u], wt[u + 1]);
+              const float2 w2 = make_float2(wt[u], wt[u + 1]);
+              if constexpr (P::SPLIT && P::CAPPED) {         // (rounded in fp32 the upper parts need no unpacking)
+                const float2 f = round8(w2), rest = fsub2(w2, f);
+                hi[(i + u) >> 1] = upper_halves(f);
+                const typename Pair<T>::V z = Pair<T>::pack(rest.x, rest.y);
+                lo[(i + u) >> 1] = *reinterpret_cast<const uint32_t*>(&z);
+                continue;
+              }
+              const typename Pair<T>::V x = Pair<T>::pack(w2.x, w2.y);
               hi[(i + u) >> 1] = *reinterpret_cast<const uint32_t*>(&x);
               if constexpr (P::SPLIT) {
-                const float2 f = Pair<T>::unpack(x);
-                const typename Pair<T>::V z = Pair<T>::pack(wt[u] - f.x, wt[u + 1] - f.y);
+                const float2 rest = fsub2(w2, Pair<T>::unpack(x));
+                const typename Pair<T>::V z = Pair<T>::pack(rest.x, rest.y);
                 lo[(i + u) >> 1] = *reinterpret_cast<const uint32_t*>(&z);
               }
             }
           }
+          if (LATE && c == 64) hand_over(0);
           if (dry) return;
           tmem_st16(at, hi);
           if constexpr (P::SPLIT) tmem_st16(at + 16, lo);
-        };
-        // 64 keys' weights are written.  Value rows past the sequence become zeros (0 times another sequence's values could be
-        // NaN): those that the product behind this hand-over reads, whichever tile's comes first
-        auto hand_over = [&](int u) {
-          if (dry) return;
-          const int left = max(it.keys - it.key0(j) - 64 * u, 0);
-          if (left < 64) {
-            const uint32_t k = tiles + j;
-            ok = mbar_wait_warp(&sh.vfull[k % NBAR], (k / NBAR) & 1, abortp, p.error_word, 835);
-#pragma unroll 1
-            for (int i = r; ok && i < (64 - left) * 8 * g.nbv; i += 128) {
-              const int line = i >> 3, blk = line / (64 - left), key = 64 * u + left + line % (64 - left);
-              *reinterpret_cast<int4*>(vring + (vslot * g.nbv + blk) * BLK + key * 128 + ((i & 7) << 4)) = make_int4(0, 0, 0, 0);
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          }
-          tmem_st_wait();
-          fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sh.pfull[t][u]);
         };
         if constexpr (P::CAPPED) {
 #pragma unroll 1
@@ -426,14 +452,15 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
             tmem_ld32_issue(st + half * COLS + c, s);
             tmem_ld32_wait(s);
             weights(s, c, 0.f);
-            if (c & 32) hand_over((half * COLS + c) >> 6);
+            hand_over(c >> 5);
           }
         } else {
+          const uint32_t at = st + half * COLS;
           if (!whole) {
 #pragma unroll 1
-            for (int c = 0; c < 128; c += 32) {
+            for (int c = 0; c < COLS; c += 32) {
               uint32_t s[32];
-              tmem_ld32_issue(st + c, s);
+              tmem_ld32_issue(at + c, s);
               const uint32_t y = seen(key0 + c);
               tmem_ld32_wait(s);
               if (row.fac.sign != 1.f) {                     // (a factor that is negative or zero)
@@ -443,27 +470,41 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
 #pragma unroll
               for (int i = 0; i < 32; ++i)
                 if (!(y >> i & 1u)) s[i] = 0xff800000u;      // -inf
-              tmem_st32(st + c, s);
+              tmem_st32(at + c, s);
             }
             tmem_st_wait();
           }
-          uint32_t s[4][32];
+          uint32_t s[CHUNKS][32];
+          float m[CHUNKS];
+          if constexpr (GROUPS == 1) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) tmem_ld32_issue(st + c * 32, s[c]);
+            for (int c = 0; c < CHUNKS; ++c) tmem_ld32_issue(at + c * 32, s[c]);
 #pragma unroll
-          for (int c = 0; c < 4; ++c) tmem_ld32_wait(s[c]);
-          float m[4];
+            for (int c = 0; c < CHUNKS; ++c) tmem_ld32_wait(s[c]);
+          } else {
+            tmem_ld32_issue(at, s[0]);
+            tmem_ld32_wait(s[0]);
+            tmem_ld32_issue(at + 32, s[1]);      // (on its way while the first part is compared)
+          }
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < CHUNKS; ++c) {
+            if (GROUPS == 2 && c == 1) tmem_ld32_wait(s[1]);
             if constexpr (P::BIASED) row.transform(s[c], key0 + c * 32);
             m[c] = fmaxf(__uint_as_float(s[c][0]), __uint_as_float(s[c][1]));
 #pragma unroll
             for (int i = 2; i < 32; i += 2) m[c] = fmax3(m[c], __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
           }
-          m[0] = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+#pragma unroll
+          for (int c = 1; c < CHUNKS; ++c) m[0] = fmaxf(m[0], m[c]);
           if constexpr (!P::BIASED) m[0] *= row.fac.mag;
+          if (GROUPS == 2 && !dry) {                         // the row's maximum is that of both halves
+            sh.rows[t][half][r] = m[0];
+            ok = meet();
+            if (!ok) break;
+            m[0] = fmaxf(m[0], sh.rows[t][half ^ 1][r]);
+          }
           const bool moves = !dry && m[0] > ref + P::LAZY;
-          if (__any_sync(0xffffffffu, moves)) {
+          if (__any_sync(0xffffffffu, moves)) {              // (the same rows and the same answer in both halves' warps)
             const float fac = moves ? ex2_approx(ref - m[0]) : 1.f;
             if (moves) ref = m[0];
             l2.x *= fac;
@@ -473,20 +514,28 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
               if (!ok) break;
               fence_after_sync();
 #pragma unroll 1
-              for (int c = 0; c < 64 * g.nbv; c += 16) {
+              for (int c = 16 * half; c < 64 * g.nbv; c += 16 * GROUPS) {
                 uint32_t o[16];
                 tmem_ld16(ot + c, o);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * fac);
                 tmem_st16(ot + c, o);
               }
+              if constexpr (GROUPS == 2) {                   // (no weights are handed over before both halves of O are rescaled)
+                tmem_st_wait();
+                fence_before_sync();
+                ok = meet();
+                if (!ok) break;
+                fence_after_sync();
+              }
             }
           }
           const float mref = ref == -INFINITY ? 0.f : ref;      // (no key seen so far: every weight is exp2(-inf))
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < CHUNKS; ++c) {
             weights(s[c], c * 32, mref);
-            if (c & 1) hand_over(c >> 1);
+            if (GROUPS == 2) hand_over(c);
+            else if (LATE ? c == 3 : c & 1) hand_over(c >> 1);
           }
         }
         if (dry) {
@@ -505,14 +554,13 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
         ok = mbar_wait_warp(&sh.pvdone[t], (cnt & 1) ^ 1, abortp, p.error_word, 836);
         if (!ok) break;
         fence_after_sync();
-        if constexpr (GROUPS == 2) {      // (the halves' sums: both are past the item before, whose last product waited for both)
-          sh.sum[t][half][r] = l;
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sh.lfull[t]);
-          ok = mbar_wait_warp(&sh.lfull[t], ends & 1, abortp, p.error_word, 839);
+        if constexpr (GROUPS == 2) {      // (the last product waited for both halves' weights, and with them for their reads of the other's maximum)
+          sh.rows[t][half][r] = l;
+          ok = meet();
           if (!ok) break;
-          l = sh.sum[t][0][r] + sh.sum[t][1][r];
-          ++ends;
+          l = sh.rows[t][0][r] + sh.rows[t][1][r];
+          ok = meet();                                       // (the next step's maxima go to the same place)
+          if (!ok) break;
         }
       }
       const float inv = row.finish(p, ref, l);
@@ -549,6 +597,7 @@ __global__ void __launch_bounds__(threads_of(P::GROUPS), 1) attn_tc_kernel(const
       }
       fence_before_sync();      // (the next item's first product into O follows the next arrival of every softmax warp of this tile)
     }
+    if (GROUPS == 2 && !ok) asm volatile("barrier.cta.arrive %0, 64;" ::"r"(pair) : "memory");
   }
   fence_before_sync();
   __syncthreads();

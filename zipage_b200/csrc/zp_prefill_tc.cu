@@ -5,19 +5,22 @@
 // A work item is two heads of one key/value head over the same 128 queries, so that a key tile is fetched once for
 // both; where a key/value head has an odd number of heads it is two neighbouring query tiles of one head.
 //
-// Measured (32 / 8 heads, bf16; causal count), single calls and SM clock under load: 1 x 16384 tokens 2.11 to 2.17 ms at 1.72 GHz = 1030 TFLOP/s,
-// 4 x 4096 0.63 to 0.65 ms, 12 prompts of 60 to 1500 tokens 155 us at 1.86 GHz. One query tile a block with a pass for the row maxima and one for
-// the weights (what stood here before): 3.46 ms at 1.78 GHz, 1.09 ms, 282 us at 1.96 GHz.
+// Pairs have one group of softmax warps a tile, which hands over its first 64 weights behind half of the second 64's exponentials (the store
+// is over by then: 1 x 16384 tokens 2.30 -> 2.26 ms a call); single tiles have two.
+//
+// Measured (32 / 8 heads, bf16; causal count), single calls and SM clock: 1 x 16384 tokens 2.0 ms at 1.83 GHz = 1100 TFLOP/s, 2.25 ms at the
+// 1.62 GHz that are left after some dozens of them (power), 4 x 4096 0.63 ms, 12 prompts of 60 to 1500 tokens 150 us. One query tile a block with a
+// pass for the row maxima and one for the weights: 3.46 ms at 1.78 GHz, 1.09 ms, 282 us at 1.96 GHz.
 #include "zp_attn_tc.cuh"
 
 namespace zp {
 
 using namespace attn;
 
-template <typename T_> struct PrefillTc {
+template <typename T_, int GROUPS_> struct PrefillTc {
   using T = T_;
   static constexpr bool SPLIT = false, MASKED = false, CAPPED = false, BIASED = false, GATED = false;
-  static constexpr int GROUPS = 1;
+  static constexpr int GROUPS = GROUPS_;
   // weights up to 2^LAZY: bf16 has fp32's range; fp16 ends at 2^16
   static constexpr float LAZY = UmmaFmt<T>::fmt == 1 ? 40.f : 12.f;
   CUtensorMap tmQ, tmK, tmV;
@@ -80,8 +83,8 @@ template <typename T_> struct PrefillTc {
   };
 };
 
-template <typename T>
-static int launch_prefill_tc(const void* q, const void* k, const void* v, PrefillTc<T>& p, int B, int max_seqlen_q,
+template <typename T, int GROUPS>
+static int launch_prefill_tc(const void* q, const void* k, const void* v, PrefillTc<T, GROUPS>& p, int B, int max_seqlen_q,
                              int64_t kv_stride_page, int total_q, int total_k, cudaStream_t st) {
   const uint32_t box[5] = {64, 1, 128, 1, 1};
   {
@@ -96,7 +99,6 @@ static int launch_prefill_tc(const void* q, const void* k, const void* v, Prefil
   if (int rc = make_tensor_map_5d(&p.tmV, UmmaFmt<T>::tm, v, dims, strides, box, sizeof(T))) return rc;
   p.rings = rings_of(2, 2);
   p.dv = 128;
-  p.mode = pick_mode(p.Hq, p.Hq / p.Hkv, B, total_q, max_seqlen_q);
   const dim3 grid = grid_of(p.mode, p.Hq, B, max_seqlen_q, p.levels);
   return launch_attn(p, grid, st, "zp_varlen_prefill(tcgen05)");
 }
@@ -107,15 +109,18 @@ int varlen_prefill_tc(const void* q, const void* k, const void* v, const int32_t
                       const int32_t* table, void* out, int B, int max_seqlen_q, int NBmax, int Hq, int Hkv,
                       int BS, int64_t kv_stride_page, float scale_log2e, int total_q, int total_k, int dtype,
                       cudaStream_t st) {
+  const int mode = pick_mode(Hq, Hq / Hkv, B, total_q, max_seqlen_q);
   auto run = [&](auto p) {
     p.cu_q = cu_q; p.cu_k = cu_k; p.table = table; p.o = out;
     p.error_word = device_error_word();
+    p.mode = mode;
     p.NBmax = NBmax; p.Hq = Hq; p.Hkv = Hkv; p.BS = BS; p.scale_log2e = scale_log2e;
     if (!p.error_word) { set_error("zp_varlen_prefill(tcgen05): no device error word"); return (int)ZP_ERR_CUDA; }
     return launch_prefill_tc(q, k, v, p, B, max_seqlen_q, kv_stride_page, total_q, total_k, st);
   };
-  if (dtype == ZP_DTYPE_BF16) return run(PrefillTc<__nv_bfloat16>{});
-  if (dtype == ZP_DTYPE_F16) return run(PrefillTc<__half>{});
+  // (single tiles: two groups of softmax warps)
+  if (dtype == ZP_DTYPE_BF16) return mode == SINGLE ? run(PrefillTc<__nv_bfloat16, 2>{}) : run(PrefillTc<__nv_bfloat16, 1>{});
+  if (dtype == ZP_DTYPE_F16) return mode == SINGLE ? run(PrefillTc<__half, 2>{}) : run(PrefillTc<__half, 1>{});
   set_error("zp_varlen_prefill(tcgen05): 16-bit tensors only");
   return ZP_ERR_UNSUPPORTED;
 }

@@ -253,6 +253,26 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {  // a + b, both la
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
+__device__ __forceinline__ float2 fsub2(float2 a, float2 b) {  // a - b, both lanes
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "sub.rn.f32x2 rc, ra, rb;\n\tmov.b64 {%0, %1}, rc;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+// the upper halves of two floats, the first one's below the other's
+__device__ __forceinline__ uint32_t upper_halves(float2 v) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(d) : "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)));
+  return d;
+}
+// both lanes rounded to the 8 bits of a bf16's mantissa (Veltkamp's split: c = (2^16 + 1) w, c - (c - w); below 2^111)
+__device__ __forceinline__ float2 round8(float2 w) {
+  float2 c = w;
+  ffma2(c, w, make_float2(65536.f, 65536.f));
+  return fsub2(c, fsub2(c, w));
+}
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
