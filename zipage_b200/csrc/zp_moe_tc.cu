@@ -12,6 +12,11 @@
 //   GT_TILE    one 128-row load (rows that already lie in the order of the places);
 //   GT_GATHER  four more warps copy the rows' 16-byte pieces with cp.async (a gather load fetches rows at a
 //              small part of a tile load's rate), publishing a stage two stages later, when its copies have landed.
+//
+// What bounds many places: the operands on their way from L2, 48 KB a stage of a 128 x 256 tile.  With MT = 2 (gathered rows) an item is
+// two tiles of 128 places of one expert that share a stage's weights (32 KB a tile), each with an accumulator and an epilogue group of its
+// own; the second tile may be missing.  The accumulators are not doubled then, so an item's epilogue is not covered: 24576
+// places of 64 experts, K 2048, N 2048 gated 222 -> 202 us (1020 TFLOP/s; the tiles are 86 % full), K 1024 from rows in order 113 -> 121, which stays at one.
 #include <type_traits>
 
 #include "zp_moe.cuh"
@@ -22,7 +27,7 @@ namespace zp {
 using namespace tc;
 
 enum { GT_FEW = 0, GT_TILE = 1, GT_GATHER = 2 };
-constexpr int GT_LAG = 2;                 // stages between the issue of a stage's copies and its publication
+constexpr int gt_lag(int mt) { return mt == 2 ? 1 : 2; }      // stages between the issue of a stage's copies and its publication (of three, or of more)
 constexpr int GT_A = 16384;               // 128 rows x 64 entries
 constexpr int GT_MAXS = 8, GT_MAXE = 1024;
 
@@ -30,7 +35,7 @@ struct __align__(16) GtShared {
   uint64_t full[GT_MAXS], empty[GT_MAXS], afull[2], aempty[2];
   uint32_t tmem_base;
   int abort_flag;
-  int mtiles[GT_MAXE + 1];                // tiles of 128 places before each expert
+  int mtiles[GT_MAXE + 1];                // items (MT tiles of 128 places) before each expert
 };
 
 struct GtParams {
@@ -49,7 +54,7 @@ __device__ __forceinline__ void gt_gather4(void* dst, const CUtensorMap* m, uint
 }
 
 struct GtTile { int e, first, count, n0; };
-template <int BN> __device__ __forceinline__ GtTile gt_tile(const GtParams& p, const GtShared& sh, int t) {
+template <int BN, int MT> __device__ __forceinline__ GtTile gt_tile(const GtParams& p, const GtShared& sh, int t) {
   const int mi = t / p.ntn;
   int lo = 0, hi = p.a.E - 1;             // last expert whose tiles start at or before mi
   while (lo < hi) {
@@ -58,8 +63,8 @@ template <int BN> __device__ __forceinline__ GtTile gt_tile(const GtParams& p, c
   }
   GtTile r;
   r.e = lo;
-  r.first = p.a.offsets[lo] + (mi - sh.mtiles[lo]) * 128;
-  r.count = min(128, p.a.offsets[lo + 1] - r.first);
+  r.first = p.a.offsets[lo] + (mi - sh.mtiles[lo]) * (128 * MT);
+  r.count = min(128 * MT, p.a.offsets[lo + 1] - r.first);
   r.n0 = (t - mi * p.ntn) * BN;
   return r;
 }
@@ -75,18 +80,19 @@ template <int LEFT> __device__ __forceinline__ void gt_publish(uint64_t* bar, in
   if (lane == 0) mbar_arrive(bar);
 }
 
-template <int MODE> constexpr int gt_threads() { return MODE == GT_GATHER ? 320 : 192; }
+template <int MODE, int MT> constexpr int gt_threads() { return 64 + 128 * MT * (MODE == GT_GATHER ? 2 : 1); }
 
-template <int BN, int ACT, int MODE>
-__global__ void __launch_bounds__(gt_threads<MODE>(), 1)
+template <int BN, int ACT, int MODE, int MT>
+__global__ void __launch_bounds__((gt_threads<MODE, MT>()), 1)
 grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const GtParams p) {
-  constexpr int STAGE = GT_A + BN * 128;
+  static_assert(MT == 1 || MODE != GT_FEW, "pairs of tiles are for many places");
+  constexpr int B_AT = MT * GT_A, STAGE = B_AT + BN * 128, LAG = gt_lag(MT);
   extern __shared__ unsigned char smem_raw[];
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   GtShared& sh = *reinterpret_cast<GtShared*>(ring + p.stages * STAGE);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < p.stages; ++s) { mbar_init(&sh.full[s], MODE == GT_GATHER ? 5 : 1); mbar_init(&sh.empty[s], 1); }
+    for (int s = 0; s < p.stages; ++s) { mbar_init(&sh.full[s], MODE == GT_GATHER ? 1 + 4 * MT : 1); mbar_init(&sh.empty[s], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&sh.afull[i], 1); mbar_init(&sh.aempty[i], 4); }
     sh.abort_flag = 0;
     fence_mbar_init();
@@ -97,7 +103,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
   } else if (warp == 1) {
     int base = 0;
     for (int e0 = 0; e0 < p.a.E; e0 += 32) {
-      const int e = e0 + lane, c = e < p.a.E ? (p.a.offsets[e + 1] - p.a.offsets[e] + 127) >> 7 : 0;
+      const int e = e0 + lane, c = e < p.a.E ? (p.a.offsets[e + 1] - p.a.offsets[e] + 128 * MT - 1) / (128 * MT) : 0;
       int s = c;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -121,7 +127,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
       bool ok = true;
       int slot = 0, round = 0;
       for (int t = blockIdx.x; ok && t < total; t += gridDim.x) {
-        const GtTile tl = gt_tile<BN>(p, sh, t);
+        const GtTile tl = gt_tile<BN, MT>(p, sh, t);
         const int groups = (tl.count + 3) >> 2;
         int4 r;
         {
@@ -139,7 +145,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
           unsigned char* dst = ring + slot * STAGE;
           if (elect_one()) {
             mbar_arrive_expect_tx(&sh.full[slot], (uint32_t)(groups * 512 + BN * 128));
-            tma_load_5d(dst + GT_A, &tmW, &sh.full[slot], k * 64, tl.n0, tl.e, 0, 0);
+            tma_load_5d(dst + B_AT, &tmW, &sh.full[slot], k * 64, tl.n0, tl.e, 0, 0);
           }
           __syncwarp();
           if (lane < groups) gt_gather4(dst + lane * 512, &tmX, &sh.full[slot], k * 64, r);
@@ -150,13 +156,15 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
       bool ok = true;
       int slot = 0, round = 0;
       for (int t = blockIdx.x; ok && t < total; t += gridDim.x) {
-        const GtTile tl = gt_tile<BN>(p, sh, t);
+        const GtTile tl = gt_tile<BN, MT>(p, sh, t);
         for (int k = 0; k < p.kb; ++k) {
           if (!mbar_wait(&sh.empty[slot], (round & 1) ^ 1, abortp, p.error_word, 941)) { ok = false; break; }
           unsigned char* dst = ring + slot * STAGE;
-          mbar_arrive_expect_tx(&sh.full[slot], (uint32_t)((MODE == GT_TILE ? GT_A : 0) + BN * 128));
-          if (MODE == GT_TILE) tma_load_5d(dst, &tmX, &sh.full[slot], k * 64, tl.first, 0, 0, 0);
-          tma_load_5d(dst + GT_A, &tmW, &sh.full[slot], k * 64, tl.n0, tl.e, 0, 0);
+          const int own = (tl.count + 127) >> 7;           // tiles of the item
+          mbar_arrive_expect_tx(&sh.full[slot], (uint32_t)((MODE == GT_TILE ? own * GT_A : 0) + BN * 128));
+          if (MODE == GT_TILE)
+            for (int m = 0; m < own; ++m) tma_load_5d(dst + m * GT_A, &tmX, &sh.full[slot], k * 64, tl.first + m * 128, 0, 0, 0);
+          tma_load_5d(dst + B_AT, &tmW, &sh.full[slot], k * 64, tl.n0, tl.e, 0, 0);
           if (++slot == p.stages) { slot = 0; ++round; }
         }
       }
@@ -165,31 +173,44 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     if (elect_one()) {
       constexpr uint32_t ID = idesc_f16(1, 128, BN);
       bool ok = true;
-      int slot = 0, round = 0, i = 0;
+      int slot = 0, round = 0, i = 0, uses[2] = {0, 0};    // of the accumulators: two tiles in turn, or an item's two
       for (int t = blockIdx.x; ok && t < total; t += gridDim.x, ++i) {
-        const int acc = i & 1;
-        if (!mbar_wait(&sh.aempty[acc], ((i >> 1) & 1) ^ 1, abortp, p.error_word, 942)) break;
+        const int first = MT == 1 ? i & 1 : 0;
+        int own = 1;
+        if constexpr (MT == 2) own = (gt_tile<BN, MT>(p, sh, t).count + 127) >> 7;
+        for (int m = 0; m < own; ++m) {
+          const int acc = MT == 1 ? first : m;
+          ok = ok && mbar_wait(&sh.aempty[acc], ((acc ? uses[1] : uses[0]) & 1) ^ 1, abortp, p.error_word, 942);
+          if (acc) ++uses[1]; else ++uses[0];
+        }
+        if (!ok) break;
         fence_after_sync();
         for (int k = 0; k < p.kb; ++k) {
           if (!mbar_wait(&sh.full[slot], round & 1, abortp, p.error_word, 943)) { ok = false; break; }
           fence_after_sync();
           const uint32_t at = smem_u32(ring + slot * STAGE);
-          const uint64_t ad = smem_desc_sw128(at), bd = smem_desc_sw128(at + GT_A);
+          const uint64_t bd = smem_desc_sw128(at + B_AT);
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks) umma_f16(tmem + acc * BN, ad + 2u * ks, bd + 2u * ks, ID, (k | ks) ? 1u : 0u);
+          for (int m = 0; m < MT; ++m) {
+            if (m >= own) continue;
+            const uint64_t ad = smem_desc_sw128(at + m * GT_A);
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) umma_f16(tmem + (first + m) * BN, ad + 2u * ks, bd + 2u * ks, ID, (k | ks) ? 1u : 0u);
+          }
           umma_commit(&sh.empty[slot]);
           if (++slot == p.stages) { slot = 0; ++round; }
         }
-        if (ok) umma_commit(&sh.afull[acc]);
+        if (ok)
+          for (int m = 0; m < own; ++m) umma_commit(&sh.afull[first + m]);
       }
     }
-  } else if (warp >= 6) {                      // (GT_GATHER) eight lanes a row, four rows an instruction
+  } else if (warp >= 2 + 4 * MT) {                      // (GT_GATHER) eight lanes a row, four rows an instruction
     const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(p.a.x);
-    const int r0 = (warp - 6) * 32 + (lane >> 3), piece = lane & 7;
+    const int r0 = (warp - 2 - 4 * MT) * 32 + (lane >> 3), piece = lane & 7;
     bool ok = true;
     int slot = 0, round = 0, late = 0, pending = 0;          // late: the slot to publish next
     for (int t = blockIdx.x; ok && t < total; t += gridDim.x) {
-      const GtTile tl = gt_tile<BN>(p, sh, t);
+      const GtTile tl = gt_tile<BN, MT>(p, sh, t);
       const __nv_bfloat16* src[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -204,11 +225,11 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int r = r0 + 4 * i;
-          gt_copy16(dst + r * 128 + ((piece ^ (r & 7)) << 4), bytes ? src[i] + k * 64 : x, bytes);
+          if (MT == 1 || r0 < 128 || tl.count > 128) gt_copy16(dst + r * 128 + ((piece ^ (r & 7)) << 4), bytes ? src[i] + k * 64 : x, bytes);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (++pending > GT_LAG) {
-          gt_publish<GT_LAG>(&sh.full[late], lane);
+        if (++pending > LAG) {
+          gt_publish<LAG>(&sh.full[late], lane);
           --pending;
           if (++late == p.stages) late = 0;
         }
@@ -223,15 +244,22 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
   } else {
     const int q = warp & 3, row = q * 32 + lane;
     const uint32_t lane_base = tmem + (static_cast<uint32_t>(q * 32) << 16);
+    const int tile = (warp - 2) >> 2;      // (MT = 2: this group's of the item)
     const bool vec = p.a.Nout % 8 == 0;
     constexpr bool GATED = ACT == ZP_ACT_SILU_MUL;
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.a.out);
     bool ok = true;
-    int i = 0;
+    int i = 0, uses = 0;
     for (int t = blockIdx.x; t < total; t += gridDim.x, ++i) {
-      const GtTile tl = gt_tile<BN>(p, sh, t);
-      const int acc = i & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(&sh.afull[acc], (i >> 1) & 1, abortp, p.error_word, 944));
+      GtTile tl = gt_tile<BN, MT>(p, sh, t);
+      if constexpr (MT == 2) {
+        tl.first += 128 * tile;
+        tl.count = min(128, tl.count - 128 * tile);
+        if (tl.count <= 0) continue;
+      }
+      const int acc = MT == 1 ? i & 1 : tile;
+      ok = __all_sync(0xffffffffu, mbar_wait(&sh.afull[acc], (MT == 1 ? i >> 1 : uses) & 1, abortp, p.error_word, 944));
+      ++uses;
       if (!ok) break;
       fence_after_sync();
       if (q * 32 < tl.count) {
@@ -302,8 +330,8 @@ bool grouped_tc_supports(const GroupedArgs& a, int dtype) {
          ((uintptr_t)a.x | (uintptr_t)a.w | (uintptr_t)a.out) % 16 == 0;
 }
 
-template <int BN, int ACT, int MODE> static int gt_launch(const GroupedArgs& a, cudaStream_t st) {
-  constexpr int STAGE = GT_A + BN * 128;
+template <int BN, int ACT, int MODE, int MT> static int gt_launch(const GroupedArgs& a, cudaStream_t st) {
+  constexpr int STAGE = MT * GT_A + BN * 128;
   GtParams p;
   p.a = a;
   p.ntn = (a.Nout + BN - 1) / BN;
@@ -329,17 +357,24 @@ template <int BN, int ACT, int MODE> static int gt_launch(const GroupedArgs& a, 
     const uint32_t box[5] = {64, BN, 1, 1, 1};
     if (int rc = make_tensor_map_5d(&tmW, UmmaFmt<__nv_bfloat16>::tm, a.w, dims, strides, box, 2)) return rc;
   }
-  const auto kern = grouped_gemm_tc_kernel<BN, ACT, MODE>;
+  const auto kern = grouped_gemm_tc_kernel<BN, ACT, MODE, MT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) { set_error("zp_grouped_gemm(tcgen05): %s", cudaGetErrorString(e)); return ZP_ERR_CUDA; }
-  const int64_t most = ((int64_t)a.places / 128 + (a.places < a.E ? a.places : a.E)) * p.ntn;   // tiles, at most
-  kern<<<(int)(most < 148 ? (most < 1 ? 1 : most) : 148), gt_threads<MODE>(), smem, st>>>(tmX, tmW, p);
+  const int64_t most = ((int64_t)a.places / (128 * MT) + (a.places < a.E ? a.places : a.E)) * p.ntn;   // items, at most
+  kern<<<(int)(most < 148 ? (most < 1 ? 1 : most) : 148), gt_threads<MODE, MT>(), smem, st>>>(tmX, tmW, p);
   return check_launch("zp_grouped_gemm(tcgen05)");
 }
 
+// About so many tiles an SM from which gathered rows go two tiles an item.  Calls with both products of 64 (32) experts, one tile an item / two: 11 tiles
+// an SM 498 / 470 us, (10.8) 448 / 423, 8.6 403 / 390, 6.1 315 / 291; 5.8 (278 / 279), 5.2 290 / 290 and 143 / 142, 4.9 148 / 151, 2.6 227 / 239: the last
+// wave of larger items costs what the shared weights gain.
+constexpr int64_t GT_PAIR_TILES = 6 * 148;
+
 template <int BN, int ACT> static int gt_pick(const GroupedArgs& a, bool many, cudaStream_t st) {
-  if (!many) return gt_launch<BN, ACT, GT_FEW>(a, st);
-  return a.rows ? gt_launch<BN, ACT, GT_GATHER>(a, st) : gt_launch<BN, ACT, GT_TILE>(a, st);
+  if (!many) return gt_launch<BN, ACT, GT_FEW, 1>(a, st);
+  if constexpr (BN == 256)
+    if (a.rows && ((int64_t)a.places / 128 + a.E / 2) * ((a.Nout + BN - 1) / BN) >= GT_PAIR_TILES) return gt_launch<BN, ACT, GT_GATHER, 2>(a, st);
+  return a.rows ? gt_launch<BN, ACT, GT_GATHER, 1>(a, st) : gt_launch<BN, ACT, GT_TILE, 1>(a, st);
 }
 
 int grouped_gemm_tc(const GroupedArgs& a, cudaStream_t st) {
