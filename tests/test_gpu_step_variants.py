@@ -134,6 +134,22 @@ def test_small_linear(dtype, rows, n_out, k, bias):
     assert ((out.double() - ref).abs() <= unit * ref.abs() + 2.0 ** -24 * k * mag + 1e-7).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows", [1, 5, 8])
+@pytest.mark.parametrize("k", [992, 1056, 2016, 2048, 3072, 3104, 4064, 4096])
+def test_small_linear_over_the_splits_of_the_inner_dimension(dtype, rows, k):
+    """Warps and loads in flight depend on k: whole turns, turns that end early, warps of unequal parts."""
+    from zipage_b200.layers.step_ops import linear
+    g = _gen(rows + k)
+    layer = torch.nn.Linear(k, 72, bias=False, device="cuda", dtype=dtype)
+    x = torch.randn(rows, k, device="cuda", generator=g).to(dtype)
+    with torch.no_grad():
+        out, w = linear(layer, x), layer.weight.double()
+    ref, mag = x.double() @ w.T, x.double().abs() @ w.abs().T
+    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11              # as above
+    assert ((out.double() - ref).abs() <= unit * ref.abs() + 2.0 ** -24 * k * mag + 1e-7).all()
+
+
 def test_linear_leaves_the_rest_to_the_layer():
     from zipage_b200 import kernel as K
     from zipage_b200.layers.step_ops import SMALL_ROWS, linear

@@ -1,25 +1,24 @@
 // out = x weight^T (+ bias) for the few rows of a decode step: 16-bit tensors, fp32 accumulation, one rounding.
 //
 // Bound by latency: the weights of a small model are a few MB, which a library product of a few rows reads in 5 to 8 us.  Here a block has
-// 16 rows of the weight and its eight warps split the inner dimension, so that even a small weight is spread over many
+// 16 rows of the weight and its 8 or 16 warps split the inner dimension, so that even a small weight is spread over many
 // SMs with all its loads in flight; and the weight is requested from HBM while the kernel before this one ends.  Products
 // on mma.sync m16n8k16 (the weight's rows are the 16-row operand, eight rows of x the other).  The order of the inner dimension is
 // free as long as both operands agree: a lane's 16-byte load of eight consecutive elements is its part of two k-steps, and no shared
 // memory is needed before the sums of the warps meet.
-// 1 to 8 rows, bf16, weights not in L2, launches back to back (us, cuBLAS): 4096 x 1024 3.1 (5.0), 6144 x 1024 4.2 (5.2),
-// 1024 x 3072 5.5 (8.4 to 9.6).  Without the request ahead 2048 x 1024 took 3.6, with it 2.6 (cuBLAS 5.2).
+// 1 to 8 rows, bf16, weights not in L2, launches back to back (us, cuBLAS): 4096 x 1024 3.2 (5.0), 6144 x 1024 4.1 (5.2), 1024 x 2048 2.7,
+// 1024 x 3072 3.7 (8.4 to 9.6), 2048 x 4096 5.4.  Without the request ahead 2048 x 1024 took 3.6, with it 2.6 (cuBLAS 5.2).  With eight warps and four
+// steps in flight whatever the size the last three took 4.3, 5.9 and 9.4.
 #include "zp_mma.cuh"
 
 namespace zp {
 
-constexpr int LIN_WARPS = 8;
-constexpr int LIN_DEEP = 4;      // 32-element steps whose loads are in flight together
-
-template <typename T>
-__global__ void __launch_bounds__(LIN_WARPS * 32)
+// WARPS: of a block; DEEP: 32-element steps whose loads are in flight together
+template <typename T, int WARPS, int DEEP>
+__global__ void __launch_bounds__(WARPS * 32)
 small_linear_kernel(const T* x, int64_t x_stride, const T* weight, const T* bias, T* out,
                     int rows, int n_out, int k) {
-  __shared__ float part[LIN_WARPS][16][9];
+  __shared__ float part[WARPS][16][9];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
   const int n0 = blockIdx.x * 16;
   // the block's rows of the weight on their way to L2 while the kernel before this one ends
@@ -31,19 +30,19 @@ small_linear_kernel(const T* x, int64_t x_stride, const T* weight, const T* bias
   const T* w0 = weight + (int64_t)min(n0 + g, n_out - 1) * k + tq * 8;
   const T* w1 = weight + (int64_t)min(n0 + g + 8, n_out - 1) * k + tq * 8;
   const T* xr = x + (int64_t)min(g, rows - 1) * x_stride + tq * 8;
-  const int steps = k / 32, s_end = (warp + 1) * steps / LIN_WARPS;
+  const int steps = k / 32, s_end = (warp + 1) * steps / WARPS;
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int s = warp * steps / LIN_WARPS; s < s_end; s += LIN_DEEP) {
-    int4 a0[LIN_DEEP], a1[LIN_DEEP], b[LIN_DEEP];
+  for (int s = warp * steps / WARPS; s < s_end; s += DEEP) {
+    int4 a0[DEEP], a1[DEEP], b[DEEP];
 #pragma unroll
-    for (int d = 0; d < LIN_DEEP; ++d) {
+    for (int d = 0; d < DEEP; ++d) {
       const int at = min(s + d, s_end - 1) * 32;
       a0[d] = ld16(w0 + at);
       a1[d] = ld16(w1 + at);
       b[d] = ld16(xr + at);
     }
 #pragma unroll
-    for (int d = 0; d < LIN_DEEP; ++d) {
+    for (int d = 0; d < DEEP; ++d) {
       if (s + d >= s_end) break;
       const uint32_t lo[4] = {(uint32_t)a0[d].x, (uint32_t)a1[d].x, (uint32_t)a0[d].y, (uint32_t)a1[d].y};
       const uint32_t hi[4] = {(uint32_t)a0[d].z, (uint32_t)a1[d].z, (uint32_t)a0[d].w, (uint32_t)a1[d].w};
@@ -60,7 +59,7 @@ small_linear_kernel(const T* x, int64_t x_stride, const T* weight, const T* bias
   if (r < rows && n0 + n < n_out) {
     float v = 0.f;
 #pragma unroll
-    for (int w = 0; w < LIN_WARPS; ++w) v += part[w][n][r];
+    for (int w = 0; w < WARPS; ++w) v += part[w][n][r];
     if (bias) v += Elem<T>::to_f32(bias[n0 + n]);
     out[(int64_t)r * n_out + n0 + n] = Elem<T>::from_f32(v);
   }
@@ -78,8 +77,15 @@ extern "C" int zp_small_linear(const void* x, int64_t x_stride, const void* weig
   ZP_REQUIRE(((uintptr_t)x | (uintptr_t)weight) % 16 == 0, "zp_small_linear: x and weight must be 16-byte aligned");
   auto run = [&](auto t) {
     using T = decltype(t);
-    zp::launch_early(zp::small_linear_kernel<T>, dim3((n_out + 15) / 16), zp::LIN_WARPS * 32, 0, (cudaStream_t)stream, (const T*)x, x_stride,
-                     (const T*)weight, (const T*)bias, (T*)out, rows, n_out, k);
+    auto go = [&](auto kernel, int warps) {
+      zp::launch_early(kernel, dim3((n_out + 15) / 16), warps * 32, 0, (cudaStream_t)stream, (const T*)x, x_stride, (const T*)weight, (const T*)bias,
+                       (T*)out, rows, n_out, k);
+    };
+    // all of a warp's loads together: a second round is another trip to L2, which no other block of the SM covers
+    if (k <= 1024) go(zp::small_linear_kernel<T, 8, 4>, 8);
+    else if (k <= 2048) go(zp::small_linear_kernel<T, 16, 4>, 16);
+    else if (k <= 3072) go(zp::small_linear_kernel<T, 16, 6>, 16);
+    else go(zp::small_linear_kernel<T, 16, 8>, 16);
   };
   if (dtype == ZP_DTYPE_BF16) run(__nv_bfloat16());
   else if (dtype == ZP_DTYPE_F16) run(__half());
