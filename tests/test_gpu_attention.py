@@ -347,3 +347,31 @@ def test_varlen_prefill_tcgen05_pages_of_128_keys():
     torch.cuda.synchronize()
     assert _lib.device_error() == 0
     assert (out - ref).abs().max() <= 2e-2 * ref.abs().max()
+
+
+@pytest.mark.parametrize("dtype,unit", [(torch.bfloat16, 2.0 ** -8), (torch.float16, 2.0 ** -11)])
+@pytest.mark.parametrize("G", [1, 2, 3, 7, 8, 9, 16])
+@pytest.mark.parametrize("B,Hkv", [(1, 1), (5, 8), (9, 12), (20, 11)])      # 8, 8, 4 and 2 splits of a sequence
+@pytest.mark.parametrize("page", [64, 256])
+def test_paged_decode_of_splits_that_merge_in_a_cluster(dtype, unit, G, B, Hkv, page):
+    """Groups that the blocks of a cluster share out evenly or not, lengths at the edges of tiles and of splits, tables of up to 64 pages."""
+    from zipage_b200.layers.attention import paged_decode_attention
+    g = torch.Generator(device="cuda").manual_seed(G * B)
+    width = 4096 // page
+    lens = ([4096, 1, 64, 65, 1000, 2048, 513, 63, 127] + [300 + 17 * i for i in range(B)])[:B]
+    pages = [(n + page - 1) // page for n in lens]
+    ids = torch.randperm(sum(pages), device="cuda", generator=g).to(torch.int32)
+    table = torch.full((B, width), -1, dtype=torch.int32, device="cuda")
+    k, v = (torch.randn(sum(pages), page, Hkv, 128, device="cuda", generator=g).to(dtype) for _ in range(2))
+    q = torch.randn(B, 1, Hkv * G, 128, device="cuda", generator=g).to(dtype)
+    at = 0
+    for b, n in enumerate(pages):
+        table[b, :n] = ids[at:at + n]
+        at += n
+    out = paged_decode_attention(q, k, v, torch.tensor(lens, dtype=torch.int32, device="cuda"), table)
+    for b, n in enumerate(lens):
+        kk, vv = (t[table[b, :pages[b]].long()].flatten(0, 1)[:n].double() for t in (k, v))
+        w = torch.softmax(torch.einsum("hgd,nhd->hgn", q[b, 0].double().view(Hkv, G, 128), kk) * 128 ** -0.5, -1)
+        ref, mag = torch.einsum("hgn,nhd->hgd", w, vv), torch.einsum("hgn,nhd->hgd", w, vv.abs())
+        # weights and result are rounded to T once each
+        assert ((out[b, 0].double().view(Hkv, G, 128) - ref).abs() <= unit * 1.1 * 2 * mag + 1e-6).all()

@@ -124,6 +124,13 @@ __device__ __forceinline__ float ld_cluster(const float* p, uint32_t rank) {
   return v;
 }
 
+// and the way back
+__device__ __forceinline__ void st_cluster(float* p, uint32_t rank, float v) {
+  uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p)), ra;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ra), "f"(v) : "memory");
+}
+
 // ---- kernels that begin while the one before them ends ----------------------------------------------
 // A kernel launched by `launch_early` may start as soon as every block of the kernel before it on the stream has called
 // `let_next_begin` or is done.  All of its threads call `wait_for_previous` first: before it, nothing may be read that an
