@@ -14,7 +14,8 @@
 // Short contexts of few sequences are bound by the trips to memory that follow one another: the length, the page, the tiles two at a time, the
 // merges.  So a sequence's first pages are read beside its length, and every split writes its numbers into the shared memory of the block
 // that finishes them: one meeting of the cluster instead of two with the reads between them.  In a step of 4 sequences (700 to 2304 keys, 16 heads on 8) the
-// kernel 11.5 -> 9.6 us; a step of 2 sequences and 4 layers 145 -> 137, of 16 277 -> 268. (Three stages for grids of up to two blocks an SM gained nothing.)
+// kernel 11.5 -> 9.6 us; a step of 2 sequences and 4 layers 145 -> 137, of 16 277 -> 268.  The next kernel may begin
+// when the keys have been read: from the first line on, the projection behind it took 5.1 us instead of 3.3. (Three stages for grids of up to two blocks an SM gained nothing.)
 #include "zp_mma.cuh"
 
 namespace zp {
@@ -42,7 +43,6 @@ __global__ void __launch_bounds__(DM_THREADS) paged_decode_mma_kernel(const DmAr
   const int g = lane >> 2, tq = lane & 3;  // fragment row / column-pair index
   if (a.nsplit > 1 && !a.part) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   wait_for_previous();
-  let_next_begin();
   // the first pages of the sequence, one (two) a lane: the loads' addresses need not wait for the length and then for the page
   const int32_t* table = a.table + (int64_t)b * a.NBmax;
   const int page0 = lane < a.NBmax ? table[lane] : 0, page1 = lane + 32 < a.NBmax ? table[lane + 32] : 0;
@@ -174,6 +174,7 @@ __global__ void __launch_bounds__(DM_THREADS) paged_decode_mma_kernel(const DmAr
   // l sums over the 4 lanes of a row are still partial: finish them
   l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+  let_next_begin();      // (not before the keys are read: the next kernel's request for its weights comes between them)
   __syncthreads();
   float* mbuf = reinterpret_cast<float*>(smem);  // [4 warps][16 rows][130]: O(128), m, l
   // behind the tiles: what the other splits write here, their maxima and sums, and their numbers for this block's entries
