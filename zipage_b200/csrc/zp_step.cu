@@ -171,7 +171,8 @@ silu_and_mul_kernel(const T* x, T* out, int I, Index total_vec) {
 // tokens: 32 heads a warp, so that cosines, sines and weights are fetched once for eight turns.  Few tokens (below QK_SPREAD,
 // where a warp per token does not fill the SMs): four heads a warp, one turn of latency.
 // 32 / 8 heads of 128, bf16: 16384 tokens 89 us = 4.9 TB/s (16 heads a warp 96, 8 105, 4 130; one warp for all kinds 114), 4 tokens
-// 2.6 us (7.6).
+// 2.6 us (7.6).  12 prompts of 60 to 1500 tokens, values packed too: 51 us for three blocks an SM with registers to match (54 where the compiler
+// chooses for itself, 54 for four blocks, 57 for five).
 // ---------------------------------------------------------------------------------------------
 constexpr int QK_SPREAD = 1024;
 
@@ -237,7 +238,7 @@ __device__ __forceinline__ void norm_rope_head(const Chunk<T, D / 16>& ca, const
 }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(256) qk_norm_rope_store_kernel(const QkArgs a) {
+__global__ void __launch_bounds__(256, 3) qk_norm_rope_store_kernel(const QkArgs a) {
   constexpr int P = D / 16;
   const int lane = threadIdx.x & 31, l8 = lane & 7, hg = lane >> 3;   // 4 heads per warp at a time
   const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), part = blockIdx.y;
