@@ -13,8 +13,10 @@ struct ConvArgs {
 __device__ __forceinline__ float cv_ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float cv_rcp(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 constexpr int CV_THREADS = 256, CV_MAX_TAPS = 8;
-constexpr int cv_batch(int taps) { return 8 / taps * taps; }      // (whole turns of the circle of inputs)
-constexpr int cv_run(int taps) { return 4 * cv_batch(taps); }     // tokens of a thread
+// Tokens whose loads are in flight (whole turns of the circle of inputs), and tokens of a thread.  Up to four taps four blocks share an SM.  6200 tokens of 8192 channels, 4 taps: 56.5 us with four tokens in flight and four blocks an SM, 61.7 with eight and three (104 with
+// eight and four, 138 with four and five: registers spill); 16 tokens a thread 57.6, 48 57.2, 64 66.
+constexpr int cv_batch(int taps) { return (taps <= 4 ? 4 : 8) / taps * taps; }
+constexpr int cv_run(int taps) { return taps <= 4 ? 32 / cv_batch(taps) * cv_batch(taps) : 4 * cv_batch(taps); }
 
 template <typename T, int V> struct __align__(V == 1 ? sizeof(T) : 8) ChanVec { T e[V]; };        // V * sizeof(T) = 8, or one entry
 template <typename T, int V> __device__ __forceinline__ ChanVec<T, V> cv_load(const T* p) {
@@ -36,7 +38,7 @@ template <typename T, int V> __device__ __forceinline__ void cv_store(T* p, cons
 }
 
 template <typename T, int V, int TAPS, bool BIAS>
-__global__ void __launch_bounds__(CV_THREADS, TAPS <= 4 ? 3 : 2) short_conv_kernel(const ConvArgs a) {
+__global__ void __launch_bounds__(CV_THREADS, TAPS <= 4 ? 4 : 2) short_conv_kernel(const ConvArgs a) {
   constexpr int BATCH = cv_batch(TAPS), RUN = cv_run(TAPS);
   const int b = blockIdx.z, c = (blockIdx.x * CV_THREADS + threadIdx.x) * V;
   const int row0 = a.cu_q[b], count = a.cu_q[b + 1] - row0, ctx = a.context_lens[b], slot = a.slots[b];
