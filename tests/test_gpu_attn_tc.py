@@ -393,3 +393,29 @@ def test_prompts_of_about_as_many_tiles_as_sms(B):
     for b in range(B):
         ref, mag = _softmax(q[b * x:b * x + x], k[b * y:b * y + y], v[b * y:b * y + y], D ** -0.5, seen)
         assert ((out[b * x:b * x + x].double() - ref).abs() <= 2.0 ** -8 * 1.1 * 2 * mag + 1e-6).all()      # as in test_prefill_edges
+
+
+@pytest.mark.parametrize("B,kv_heads,dim", [(1, 8, 128), (18, 8, 128), (19, 8, 128), (27, 8, 128), (28, 8, 128), (56, 8, 128), (37, 8, 64), (20, 8, 96)])
+@pytest.mark.parametrize("width,window,keep", [(24, 0, 0), (25, 0, 0), (40, 512, 0), (40, 512, 64)])
+def test_decoded_windows_over_the_numbers_of_splits(B, kv_heads, dim, width, window, keep):
+    """Sequences and keys in sight around which the splits of a sequence change, and the workspace with them."""
+    from zipage_b200.layers.attention import window_attention
+    heads, page = 2 * kv_heads, 64
+    g = torch.Generator(device="cuda").manual_seed(B)
+    lens = [1 + (b * 37) % (width * page) for b in range(B)]
+    lens[0] = width * page
+    pages = B * width
+    table = torch.randperm(pages, device="cuda", generator=g).to(torch.int32).view(B, width)
+    k, v = (torch.randn(pages, page, kv_heads, dim, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(B, heads * dim, device="cuda", generator=g).to(torch.bfloat16)
+    out = torch.empty_like(q)
+    window_attention(q, k, v, torch.tensor(lens, dtype=torch.int32, device="cuda"), table, heads, dim, dim, dim ** -0.5, window, 0.0, out=out, keep=keep)
+    _no_device_error()
+    for b in list(range(0, B, 9)) + [B - 1]:
+        n = lens[b]
+        j = torch.arange(n, device="cuda")
+        seen = ((j > n - 1 - window) | (j < keep))[None] if window else torch.ones(1, n, dtype=torch.bool, device="cuda")
+        kk, vv = (t[table[b, :(n + page - 1) // page].long()].flatten(0, 1)[:n] for t in (k, v))
+        ref, mag = _softmax(q[b].view(1, heads, dim), kk, vv, dim ** -0.5, seen)
+        # weights as two bf16 numbers (2^-16), the result rounded once
+        assert ((out[b].view(1, heads, dim).double() - ref).abs() <= (2.0 ** -8 + 2.0 ** -14) * mag + 1e-6).all()

@@ -463,12 +463,23 @@ static int decode_smem(const WinArgs& a) {
 
 bool window_mma_supports(const WinArgs& a) { return a.KP <= 256 && a.VP <= 256 && a.Hq / a.Hkv <= 16; }
 
-int window_decode_splits(int B, int Hkv, int span) {
-  const int target = 148 * 4, tiles = (span + WM_TK - 1) / WM_TK;
-  int s = (target + B * Hkv - 1) / (B * Hkv);
-  if (s > (tiles + 1) / 2) s = (tiles + 1) / 2;   // at least two tiles each
+// Four blocks an SM and at least two tiles each; where the keys in sight are few, no more splits than the SMs hold at once (three blocks of 128
+// entries): a second wave of short blocks and the merge cost more than they share out.  Kernels with the merge, cold caches, window 1024, 8 key/value
+// heads of 128 (us; 1, 2, 3, 4, 6 splits; four an SM): 8 sequences 28, 21, 20, 19, 19 (18.5); 16: 29, 25, 25, 29, 31 (31); 24: 36, 30, 38, 37, 41 (37);
+// 32: 37, 47, 43, 44, 51 (43); 48: 46, 55, 60, 60, 70 (55); window 512, 32: 24, 32, 31, 31 (31).  2200 keys in sight, 32: 64, 67, 58, 61, 64 (59): those stay,
+// and so do sizes between those of the compiled kernels (96 entries, 20 sequences 31.5 for 29.1).
+constexpr int WD_FEW = 1536;
+int window_decode_splits(int B, int Hkv, int span, int VP) {
+  const int tiles = (span + WM_TK - 1) / WM_TK;
+  const int64_t pairs = (int64_t)B * Hkv;
+  int64_t s = (148 * 4 + pairs - 1) / pairs;
+  if (s > (tiles + 1) / 2) s = (tiles + 1) / 2;
   if (s > 32) s = 32;
-  return s < 1 ? 1 : s;
+  if (span <= WD_FEW && (VP == 64 || VP == 128)) {
+    const int smem = (16 + 4 * WM_TK) * row_bytes(VP) + 1024, held = 232448 / smem < 4 ? 232448 / smem : 4;
+    if (s > 148 * held / pairs) s = 148 * held / pairs;
+  }
+  return s < 1 ? 1 : (int)s;
 }
 
 template <typename K> static int set_smem(K kern, int bytes, const char* what) {
