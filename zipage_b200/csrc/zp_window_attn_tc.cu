@@ -7,13 +7,14 @@
 // of heads, two neighbouring query tiles of one head.
 //
 // A key tile is two 64-key boxes per 64 entries, so its halves may lie in different pages; head sizes that are no
-// multiples of 64 are filled with zeros by TMA.  The capped softmax is bound by the special-function unit: two
-// exponentials and a reciprocal per score; four reciprocals share one instruction, 1/a = bcd / (abcd).
+// multiples of 64 are filled with zeros by TMA.  The capped softmax takes two exponentials and a reciprocal per score; four reciprocals share
+// one instruction, 1/a = bcd / (abcd).  It is bound by its instructions, not by the special-function unit: with a quarter of the exponentials as
+// polynomials the call took 382 us instead of 367.
 //
 // A tile of its own per block, all softmax warps on it, left the tensor cores idle during each of its softmax turns.  Four portions of
 // 500 to 3000 tokens, 32 heads on 8, window 1024, cap 30: 302 us (344 so).  Uniform portions, no window: 4 x 2000 tokens 236 us (320),
 // 4 x 1000 85 (112); cap 30 and window 512: 86 (107).  Since then weights are handed over 32 keys at a time and split in fp32 (capped), and uncapped
-// windows have two groups of softmax warps: the first of these 277 us, without cap 7 us less than with one group.
+// windows have two groups of softmax warps: the first of these 309 -> 286 us in one profiler, without cap 7 us less than with one group.
 #include <algorithm>
 
 #include "zp_attn_tc.cuh"
@@ -166,7 +167,7 @@ static int launch_window_tc(const WinArgs& a, int max_q, int total_q, cudaStream
 }
 
 // Launches of few 128-row query tiles take the kernel of zp_window_attn_tc_short.cu (single tiles, whose waves are finer and whose code is
-// shorter to fetch).  Times of this file's kernel over that one's, heads of 128, portions of 96 to 2560 tokens, 32 heads on 8 unless noted; the
+// shorter to fetch; the figures are from before this file's kernel became 3 to 7 % faster, so the lines lie on the safe side).  Times of this file's kernel over that one's, heads of 128, portions of 96 to 2560 tokens, 32 heads on 8 unless noted; the
 // lines lie where no column is above 1 by more than a few percent:
 //   tiles        no context, no cap   cap   | window 512 or 1024, context 2000: no cap   cap   | no window, context 2000: no cap   cap
 //   320 .. 416   0.86 .. 1.00   0.91 .. 1.03 | 1.05 .. 1.14   1.12 .. 1.20                     | 0.95 .. 1.18   1.13 .. 1.26
