@@ -150,6 +150,24 @@ def test_small_linear_over_the_splits_of_the_inner_dimension(dtype, rows, k):
     assert ((out.double() - ref).abs() <= unit * ref.abs() + 2.0 ** -24 * k * mag + 1e-7).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n_out,k", [(40, 256), (40, 512), (40, 768), (40, 1024), (40, 1280), (40, 1536), (40, 1792), (72, 2048), (72, 2304), (2376, 3072), (2368, 3072),
+                                     (72, 3328), (2376, 3328), (2368, 3328), (72, 4096)])
+def test_small_linear_adds_eight_parts_of_the_inner_dimension(dtype, n_out, k):
+    """Whatever the number of loads in flight, the fp32 sums are those of eight consecutive eighths, added in order: 2^24 from the first, 1 + 1 from
+    both ends of the second and -2^24 from the last give 2; with the ones added one by one it would be 0."""
+    from zipage_b200.layers.step_ops import linear
+    layer = torch.nn.Linear(k, n_out, bias=False, device="cuda", dtype=dtype)
+    x, e = torch.zeros(3, k, device="cuda", dtype=dtype), k // 8
+    x[:, e - 1], x[:, e], x[:, 2 * e - 1], x[:, -1] = 4096, 1, 1, -4096
+    with torch.no_grad():
+        layer.weight.zero_()
+        layer.weight[:, [e - 1, -1]] = 4096
+        layer.weight[:, [e, 2 * e - 1]] = 1
+        out = linear(layer, x)
+    assert torch.equal(out, torch.full_like(out, 2))
+
+
 def test_linear_leaves_the_rest_to_the_layer():
     from zipage_b200 import kernel as K
     from zipage_b200.layers.step_ops import SMALL_ROWS, linear

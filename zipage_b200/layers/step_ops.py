@@ -53,11 +53,11 @@ class RMSNorm(nn.Module):
         return rms_norm(x, self.weight, self.eps, residual)
 
 
-# Rows, entries and sides of the weight up to which `linear` takes this library's kernel.  At 8 rows it takes 0.4 to 0.8 of cuBLAS's time
-# for weights of up to 2^23 entries (2048 x 1024: 2.7 us for 4.8; 6144 x 1024: 4.2 for 5.2; 1024 x 3072: 3.7 for 8.4); larger weights go either
-# way (8192 x 2048: 7.9 for 8.0; 5120 x 2048: 7.1 for 6.5; 12288 x 4096: 26 for 19, measured with fewer loads in flight), and so do 9 to 32 rows
-# (4096 x 4096: 11.4 for 9.5).  A block walks 16 whole rows of the weight, so long ones leave SMs idle (256 x 4096: 4.5 for 8.3; 256 x 8192: 17.9 for 13.1; 32 x
-# 65536: 145 for 13.6), and very many short ones are blocks of no work (32768 x 256: 6.7 for 7.2; 65536 x 128: 9.0 for 7.7).
+# Rows, entries and sides of the weight up to which `linear` takes this library's kernel.  At 8 rows it takes 0.4 to 0.7 of cuBLAS's time
+# for weights of up to 2^23 entries (2048 x 1024: 2.2 us for 5.1; 6144 x 1024: 3.6 for 5.3; 1024 x 3072: 3.8 for 8.8; 256 x 4096: 4.0 for 7.7); larger
+# ones go either way (4096 x 4096: 7.4 for 12.1; 5120 x 2048: 6.0 for 6.6; 8192 x 2048: 7.9 for 8.1; 12288 x 4096: 20.4 for 18.2).  A block walks 16 whole
+# rows of the weight, so very long ones leave SMs idle (256 x 8192: 7.0 for 12.6, but 32 x 65536: 33 for 13), and very many short ones are blocks of
+# little work (32768 x 256: 5.6 for 5.4).
 SMALL_ROWS, SMALL_WEIGHT, SMALL_K, SMALL_N = 8, 1 << 23, 4096, 1 << 15
 
 
