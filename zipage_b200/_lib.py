@@ -171,10 +171,19 @@ def ptr(t):
     return None if t is None else t.data_ptr()
 
 
+# The current stream of a device as a number: torch.cuda.current_stream() makes a Stream object of it, which took a third of the host time
+# of a small call.  The function is torch's own, not part of its interface, so a build without it goes by the object.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def stream_handle(device_index):
+    """The handle of that device's current stream."""
+    return torch.cuda.current_stream(device_index).cuda_stream if _raw_stream is None else _raw_stream(device_index)
+
+
 def stream_ptr():
-    """The current stream's handle.  (Asked for as a number: torch.cuda.current_stream() makes a Stream object of it, which took a third of
-    the host time of a small call.)"""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    """The handle of the current device's current stream."""
+    return stream_handle(torch.cuda.current_device())
 
 
 def dtype_code(t: torch.Tensor) -> int:

@@ -20,7 +20,7 @@ _ws_kept: list = []   # outgrown buffers stay: a captured graph may still name t
 
 
 def _workspace(device, nbytes):
-    key = (device.index, torch.cuda.current_stream().cuda_stream)
+    key = (device.index, L.stream_handle(device.index))
     buf = _ws_cache.get(key)
     if buf is None or buf.numel() < nbytes:
         if buf is not None:
