@@ -40,7 +40,7 @@ def test_qk_norm_rope_is_the_same_for_few_and_many_tokens(dtype, heads, kv_heads
 @pytest.mark.parametrize("kv_heads,D", [(8, 128), (3, 64)])
 @pytest.mark.parametrize("stored", [True, False])
 def test_values_are_packed_beside_the_keys(dtype, N, kv_heads, D, stored):
-    """With `return_k` v is a packed copy of qkv's columns, rows without a cache slot among them; without it a view."""
+    """v is a packed copy of qkv's columns, rows without a cache slot among them, or a view of them: as `return_v` says, or else `return_k`."""
     from zipage_b200.layers import step_ops as P
     g, heads, dev = _gen(N), 4, "cuda"
     wide = torch.randn(N, (heads + 2 * kv_heads) * D + 16, device=dev, generator=g).to(dtype)
@@ -62,6 +62,11 @@ def test_values_are_packed_beside_the_keys(dtype, N, kv_heads, D, stored):
         assert torch.equal(cache["v_cache"].view(1280, kv_heads, D), rows)
     _, k, v = P.qk_norm_rope_store(qkv, pos, cs, *w, 1e-6, heads, kv_heads, D, return_k=False)
     assert k is None and v.data_ptr() == want.data_ptr() and torch.equal(v, want)
+    # keys alone, without the copy of the values that their caller does not ask for; and the other way round
+    _, keys, v = P.qk_norm_rope_store(qkv, pos, cs, *w, 1e-6, heads, kv_heads, D, return_v=False)
+    assert keys.is_contiguous() and v.data_ptr() == want.data_ptr()
+    _, k, v = P.qk_norm_rope_store(qkv, pos, cs, *w, 1e-6, heads, kv_heads, D, return_k=False, return_v=True)
+    assert k is None and v.is_contiguous() and v.data_ptr() != want.data_ptr() and torch.equal(v, want)
 
 
 def _draws(seed, rows, V):

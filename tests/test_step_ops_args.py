@@ -47,6 +47,11 @@ def test_other_step_ops_reject_bad_arguments():
     assert lib.zp_qk_norm_rope_store(*args(D=96)) == INVALID
     assert "head_dim" in _err(lib)
     assert lib.zp_qk_norm_rope_store(*args(qkv=C.c_void_p(4100))) == INVALID
+    # the form that packs the values too checks the same and one pointer more, which may be missing
+    packed = lambda v_out, **kw: (lambda a: lib.zp_qk_norm_rope_store_v(*a[:8], v_out, *a[8:]))(args(**kw))
+    assert packed(p, n=0) == packed(None, n=0) == 0
+    assert packed(C.c_void_p(4100)) == INVALID and "aligned" in _err(lib)
+    assert packed(p, q_out=None) == packed(p, slots=p) == packed(p, D=96) == packed(p, qkv=C.c_void_p(4100)) == INVALID
     assert lib.zp_sample(None, None, None, None, 0, 1000, 0, 0, None) == 0
     assert lib.zp_sample(p, None, None, p, 2, 1000, 0, 0, None) == INVALID
     assert lib.zp_sample(p, p, None, p, 2, 0, 0, 0, None) == INVALID

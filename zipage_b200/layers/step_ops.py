@@ -134,13 +134,13 @@ def rope_cos_sin_cache(head_dim, max_position, base, device):
 
 def qk_norm_rope_store(qkv, positions, cos_sin, q_weight, k_weight, eps, num_heads, num_kv_heads,
                        head_dim, k_cache=None, v_cache=None, slot_mapping=None, query_cache=None,
-                       query_slot_mapping=None, return_k=True, query_slot_count=None):
+                       query_slot_mapping=None, return_k=True, query_slot_count=None, return_v=None):
     """qkv [N, (Hq+2Hkv)*D] -> q [N,Hq,D] (normalised, rotated), k [N,Hkv,D] (or None), and, when
     given, K/V rows written to the paged caches at slot_mapping and window queries written to
     query_cache at the (row, query_id, index) triples — one launch.  `query_slot_count`: a device
     int32 tensor with the number of valid rows of `query_slot_mapping` (as `prepare_decode` returns
-    it); without it every row is taken.  v [N,Hkv,D]: a packed copy with `return_k` (whose caller
-    attends over the rows themselves), else a view of qkv."""
+    it); without it every row is taken.  v [N,Hkv,D]: a packed copy with `return_v` (None: as `return_k`, whose callers
+    mostly attend over the rows themselves), else a view of qkv."""
     L.require_cuda(qkv, positions, cos_sin, q_weight, k_weight, k_cache, v_cache, slot_mapping,
                    query_cache, query_slot_mapping, query_slot_count)
     N = qkv.shape[0]
@@ -148,7 +148,8 @@ def qk_norm_rope_store(qkv, positions, cos_sin, q_weight, k_weight, eps, num_hea
     assert qkv.shape[1] == (Hq + 2 * Hkv) * D and qkv.stride(1) == 1
     assert positions.dtype == torch.int64 and cos_sin.dtype == torch.float32 and cos_sin.is_contiguous()
     q = torch.empty((N, Hq, D), dtype=qkv.dtype, device=qkv.device)
-    k, v = (torch.empty((N, Hkv, D), dtype=qkv.dtype, device=qkv.device) if return_k else None for _ in range(2))
+    k, v = (torch.empty((N, Hkv, D), dtype=qkv.dtype, device=qkv.device) if wanted else None
+            for wanted in (return_k, return_k if return_v is None else return_v))
     ntrip = 0 if query_slot_mapping is None else query_slot_mapping.shape[0]
     cs_seq = query_cache.stride(0) if query_cache is not None else 0
     cs_slot = query_cache.stride(1) if query_cache is not None else 0
