@@ -2,11 +2,13 @@
 (zipage_b200/csrc/zp_attn_tc.cuh, two groups) on the CPU.
 
 The issuer of products, the tensor pipe and the two warps of a row (one per half of the keys) of both tiles run as coroutines under random
-schedules.  The warps exchange a step's maxima and an item's sums through one place in shared memory and meet there; both hand over two
-units of weights a step.  Checked: no deadlock; what a warp reads there is the other's number of the same step or item; products read
-the weights of their step; a rescaled accumulator is the step before's and is whole before the next product; an item's output is
-its own.  With one meeting instead of two at an item's end the next step's maximum overwrites a sum that is still to be read.  A warp that
-gives up arrives once more on its way out; without that its partner waits for good.
+schedules.  Both hand over two units of weights a step, and a product waits for both.  The warps exchange an item's sums through one place in
+shared memory and meet there; scores without a cap a step's maxima too (capped ones have a fixed reference: their warps do not meet
+in a step, and never rescale).  Checked: no deadlock; what a warp reads there is the other's number of the same step or item; products read
+the weights of their step; a rescaled accumulator is the step before's and is whole before the next product (also without the meeting that follows
+a rescale); an item's output is its own.  Without a cap, one meeting instead of two at an item's end lets the next step's maximum overwrite a sum that
+is still to be read.  A product that waits for one group alone reads weights that are not there yet.  A product has to be reported before the next scores
+are, as in the form of one group.  A warp that gives up arrives once more on its way out; without that its partner waits for good.
 """
 import random
 from collections import deque
@@ -26,11 +28,11 @@ class Meeting:                          # barrier.cta.sync / .arrive of two warp
             self.n, self.phase = 0, self.phase + 1
 
 
-def run(seed, meetings=2, fail_at=None, arrives_on_exit=True, n_items=25):
+def run(seed, capped=False, meetings=2, rescale_meets=True, waits_for_both=True, done_before_scores=True, fail_at=None, arrives_on_exit=True, n_items=25):
     rnd = random.Random(seed)
     items = [(rnd.randint(0, 3), rnd.randint(0, 3)) for _ in range(n_items)]
     sfull, pvdone = [Bar(1), Bar(1)], [Bar(1), Bar(1)]
-    pfull = [[Bar(2), Bar(2)] for _ in range(2)]
+    pfull = [[Bar(2 if waits_for_both else 1) for _ in range(2)] for _ in range(2)]
     pipe, over, abort = deque(), [False], [False]
     scores, weights, out = [None, None], [[[None] * 2, [None] * 2] for _ in range(2)], [None, None]
     meeting, place = [Meeting(), Meeting()], [[None, None], [None, None]]
@@ -64,10 +66,15 @@ def run(seed, meetings=2, fail_at=None, arrives_on_exit=True, n_items=25):
                         pipe.append(("product", t, (w, j), u))
                         yield
                     cnt[t] += 1
-                    pipe.append(("commit", pvdone[t]))
+                    if done_before_scores:
+                        pipe.append(("commit", pvdone[t]))
                     if j + 1 < n[t]:
                         pipe.append(("scores", t, (w, j + 1)))
                         pipe.append(("commit", sfull[t]))
+                    if not done_before_scores:
+                        for _ in range(rnd.choice([0, 0, 200])):
+                            yield
+                        pipe.append(("commit", pvdone[t]))
                     yield
 
     def tensor_pipe():
@@ -121,20 +128,23 @@ def run(seed, meetings=2, fail_at=None, arrives_on_exit=True, n_items=25):
                     yield from wait(sfull[t], cnt & 1)
                     if scores[t] != (w, j):
                         raise Violation("scores of another step")
-                    yield from swap(("max", w, j))
-                    if j > 0 and (w + j) % 3 == 0:        # the reference moves
+                    if not capped:
+                        yield from swap(("max", w, j))
+                    if not capped and j > 0 and (w + j) % 3 == 0:        # the reference moves
                         yield from wait(pvdone[t], (cnt & 1) ^ 1)
                         if out[t][:2] != [w, j - 1]:
                             raise Violation("another step's accumulator is rescaled")
                         if out[t][2] == {0, 1}:
                             out[t][2] = set()
                         out[t][2].add(half)
-                        yield from meet()
+                        if rescale_meets:
+                            yield from meet()
                     for u in range(2):
                         for _ in range(rnd.randint(0, 3)):
                             yield
                         weights[t][u][half] = (w, j)
-                        pfull[t][u].arrive()
+                        if waits_for_both or half == 0:
+                            pfull[t][u].arrive()
                     cnt += 1
                 if n[t]:
                     yield from wait(pvdone[t], (cnt & 1) ^ 1)
@@ -173,35 +183,50 @@ def run(seed, meetings=2, fail_at=None, arrives_on_exit=True, n_items=25):
         raise Violation("a wait ran out")
 
 
-@pytest.mark.parametrize("seed", range(20))
-def test_the_halves_of_a_row_agree(seed):
-    run(seed)
-
-
-def test_one_meeting_at_the_end_of_an_item_is_unsafe():
-    failures = 0
-    for seed in range(10):
+def broken(seeds, fail_item=None, **how):
+    """What the checks say of a broken form; at least one schedule has to show it.  `fail_item`: a warp gives up in one of so many items."""
+    said = []
+    for seed in range(seeds):
         try:
-            run(seed, meetings=1)
+            run(seed, fail_at=(0, 0, seed % fail_item, 0) if fail_item else None, **how)
         except Violation as e:
-            assert "partner" in str(e)
-            failures += 1
-    assert failures > 0
+            said.append(str(e))
+    assert said
+    return said
+
+
+@pytest.mark.parametrize("capped", [False, True])
+@pytest.mark.parametrize("seed", range(20))
+def test_the_halves_of_a_row_agree(seed, capped):
+    run(seed, capped)
 
 
 @pytest.mark.parametrize("seed", range(10))
-def test_a_warp_that_gives_up_holds_nobody_up(seed):
+def test_nothing_hangs_on_the_meeting_after_a_rescale(seed):
+    run(seed, rescale_meets=False)
+
+
+def test_one_meeting_at_the_end_of_an_item_is_unsafe():
+    assert all("partner" in s for s in broken(10, meetings=1))
+
+
+@pytest.mark.parametrize("capped", [False, True])
+def test_a_product_that_waits_for_one_group_is_unsafe(capped):
+    assert all("weights" in s for s in broken(10, capped=capped, waits_for_both=False))
+
+
+@pytest.mark.parametrize("capped", [False, True])
+def test_reporting_a_product_after_the_next_scores_is_unsafe(capped):
+    broken(10, capped=capped, done_before_scores=False)
+
+
+@pytest.mark.parametrize("capped", [False, True])
+@pytest.mark.parametrize("seed", range(10))
+def test_a_warp_that_gives_up_holds_nobody_up(seed, capped):
     for t in range(2):
         for half in range(2):
-            run(seed, fail_at=(t, half, seed % 5, 0))
+            run(seed, capped, fail_at=(t, half, seed % 5, 0))
 
 
 def test_leaving_without_an_arrival_is_unsafe():
-    failures = 0
-    for seed in range(6):
-        try:
-            run(seed, fail_at=(0, 0, seed % 3, 0), arrives_on_exit=False)
-        except Violation as e:
-            assert "deadlock" in str(e)
-            failures += 1
-    assert failures > 0
+    assert all("deadlock" in s for s in broken(6, fail_item=3, arrives_on_exit=False))

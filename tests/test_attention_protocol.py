@@ -1,12 +1,12 @@
-"""Model check of the hand-over of accumulators in the shared tcgen05 attention pipeline (zipage_b200/csrc/zp_attn_tc.cuh) on the CPU.
+"""Model check of the hand-over of accumulators in the shared tcgen05 attention pipeline (zipage_b200/csrc/zp_attn_tc.cuh) on the CPU: one
+group of softmax warps a tile (two groups: test_attention_halves_protocol.py).
 
 The issuer of products, the tensor pipe (which works the issued products and commits off in order) and the softmax warps of both
 tiles are replayed as coroutines over models of the mbarriers, under random schedules and random numbers of key tiles per item.  Checked:
 no deadlock; a softmax warp reads the scores of its own step; the product reads the weights of its own step; and the output of
-an item is read from that item's accumulator, although the next item's first product overwrites all of it.  With two groups of warps a
-tile that last point needs both groups' hand-over before an item's first product: the variant that waits for one of them alone
-reads the next item's accumulator within a few items.  A wait for a product compares the parity of its barrier, so that the product
-before has to be reported before the next scores are: the other order takes the one for the other.
+an item is read from that item's accumulator, although the next item's first product overwrites all of it.  A wait for a product
+compares the parity of its barrier, so that the product before has to be reported before the next scores are: the other order takes the one
+for the other.
 """
 import random
 from collections import deque
@@ -15,10 +15,10 @@ import pytest
 
 from test_slot_protocol import Bar, Violation
 
-WARPS = 4                              # of a group
+WARPS = 4
 
 
-def run(seed, groups, first_waits_for_both=True, done_before_scores=True, n_items=25):
+def run(seed, done_before_scores=True, n_items=25):
     rnd = random.Random(seed)
     items = [(rnd.randint(0, 3), rnd.randint(0, 3)) for _ in range(n_items)]      # key tiles of the two query tiles
     sfull, pvdone = [Bar(1), Bar(1)], [Bar(1), Bar(1)]
@@ -42,8 +42,6 @@ def run(seed, groups, first_waits_for_both=True, done_before_scores=True, n_item
                     if j >= n[t]:
                         continue
                     for u in range(2):
-                        if groups == 2 and first_waits_for_both and j == 0 and u == 0:
-                            yield from wait(pfull[t][1], cnt[t] & 1)
                         yield from wait(pfull[t][u], cnt[t] & 1)
                         pipe.append(("product", t, (w, j), u))
                         yield
@@ -82,18 +80,18 @@ def run(seed, groups, first_waits_for_both=True, done_before_scores=True, n_item
                     raise Violation("products of two items in one accumulator")
                 out[t] = (step[0], step[1])
 
-    def softmax_warp(t, group):
+    def softmax_warp(t):
         cnt = 0
         for w, n in enumerate(items):
             for j in range(n[t]):
                 yield from wait(sfull[t], cnt & 1)
                 if scores[t] != (w, j):
                     raise Violation("scores of another step")
-                if groups == 1 and j > 0 and (w + j) % 3 == 0:        # the reference moves, and the accumulator with it
+                if j > 0 and (w + j) % 3 == 0:        # the reference moves, and the accumulator with it
                     yield from wait(pvdone[t], (cnt & 1) ^ 1)
                     if out[t] != (w, j - 1):
                         raise Violation("another step's accumulator is rescaled")
-                for u in range(2) if groups == 1 else (group,):
+                for u in range(2):
                     for _ in range(rnd.randint(0, 3)):
                         yield
                     weights[t][u] = (w, j)
@@ -106,7 +104,7 @@ def run(seed, groups, first_waits_for_both=True, done_before_scores=True, n_item
                         raise Violation("an item's output is read from another accumulator")
                     yield
 
-    procs = [issuer(), tensor_pipe()] + [softmax_warp(t, g) for t in range(2) for g in range(groups) for _ in range(WARPS)]
+    procs = [issuer(), tensor_pipe()] + [softmax_warp(t) for t in range(2) for _ in range(WARPS)]
     alive, steps = [True] * len(procs), 0
     while any(alive):
         i = rnd.randrange(len(procs))
@@ -120,29 +118,16 @@ def run(seed, groups, first_waits_for_both=True, done_before_scores=True, n_item
             raise Violation("deadlock")
 
 
-@pytest.mark.parametrize("groups", [1, 2])
 @pytest.mark.parametrize("seed", range(20))
-def test_an_items_output_is_its_own(seed, groups):
-    run(seed, groups)
+def test_an_items_output_is_its_own(seed):
+    run(seed)
 
 
-def test_waiting_for_one_of_two_groups_is_unsafe():
+def test_reporting_a_product_after_the_next_scores_is_unsafe():
     failures = 0
     for seed in range(10):
         try:
-            run(seed, 2, first_waits_for_both=False)
-        except Violation as e:
-            assert "output" in str(e)
-            failures += 1
-    assert failures > 0
-
-
-@pytest.mark.parametrize("groups", [1, 2])
-def test_reporting_a_product_after_the_next_scores_is_unsafe(groups):
-    failures = 0
-    for seed in range(10):
-        try:
-            run(seed, groups, done_before_scores=False)
+            run(seed, done_before_scores=False)
         except Violation:
             failures += 1
     assert failures > 0
