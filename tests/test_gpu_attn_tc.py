@@ -215,11 +215,10 @@ def test_prompts_whose_reference_moves(dtype, heads, kv_heads):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("key", [0, 31, 63, 64, 100, 127])
-@pytest.mark.parametrize("heads", [2, 40])               # a tile an SM (two groups of warps share a row) and pairs of tiles
-def test_prompts_whose_reference_moves_in_one_half_of_a_row(dtype, key, heads):
+@pytest.mark.parametrize("heads,n", [(2, 512), (2, 600), (40, 600)])      # a tile an SM, two groups of warps that share a row or one; pairs of tiles
+def test_prompts_whose_reference_moves_in_one_half_of_a_row(dtype, key, heads, n):
     """One key of the third and of the fourth tile is far above all others: the half of the row without it has to follow."""
     from zipage_b200.layers.attention import varlen_prefill_attention
-    n = 600
     g = torch.Generator(device="cuda").manual_seed(key)
     q, k, v = (torch.randn(n, heads, D, device="cuda", generator=g).to(dtype) for _ in range(3))
     q[..., 0], k[..., 0] = 24.0, 0.0

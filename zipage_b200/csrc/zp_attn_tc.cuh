@@ -21,9 +21,9 @@
 //
 // Softmax warps: P::GROUPS groups of four a tile.  One group: a thread owns a whole row and no maximum or sum ever crosses threads.
 // Two groups split a row's keys and exchange its maximum through shared memory: half the loads, comparisons and exponentials follow
-// one another, for half as many instructions again.  That is the better way where one tile has the SM to itself (prompts of up to 148
-// tiles, 3 of 60 to 400 tokens: the call 48 -> 40 us), where a score costs more (capped windows 368 -> 342, uncapped 334 -> 325, latents 476 -> 470), and the
-// worse one for pairs of tiles of long prompts (16384 tokens 2.29 -> 2.36 ms) and biased windows (385 -> 421).
+// one another, for half as many instructions again.  That is the better way for single tiles of few keys (see zp_prefill_tc.cu) and where a score costs more
+// (calls with uncapped windows 334 -> 325 us, latents 476 -> 470; capped windows have no maximum to exchange and meet at an item's end alone), and the
+// worse one for single tiles of many keys, pairs of tiles of long prompts (16384 tokens 2.29 -> 2.36 ms) and biased windows (385 -> 421).
 //
 // Roles (one block per SM): warp 0 = work, TMA loads and TMEM, warp 1 = products, from warp 4 on softmax, P::GROUPS groups of
 // four warps a tile, which take over registers of the first group.  One thread issues the

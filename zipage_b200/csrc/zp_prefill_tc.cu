@@ -5,8 +5,11 @@
 // A work item is two heads of one key/value head over the same 128 queries, so that a key tile is fetched once for
 // both; where a key/value head has an odd number of heads it is two neighbouring query tiles of one head.
 //
-// Pairs have one group of softmax warps a tile, which hands over its first 64 weights behind half of the second 64's exponentials (the store
-// is over by then: 1 x 16384 tokens 2.30 -> 2.26 ms a call); single tiles have two.
+// One group of softmax warps a tile, which hands over its first 64 weights behind half of the second 64's exponentials (the store
+// is over by then: 1 x 16384 tokens 2.30 -> 2.26 ms a call); two for single tiles of up to four key tiles.  The second group's earlier
+// start is the gain, the exchange of every step's maximum the price.  Kernel alone, one group / two (us): prompts of 40 tokens 10.4 / 10.0,
+// 300 14.5 / 14.3, 400 16.8 / 16.6, 8 of 40 11.1 / 10.7; 700 20.5 / 21.0, 1500 31.6 / 33.1, 2000 (8 heads) 39.4 / 41.5; behind 256 cached keys
+// 40 tokens 14.5 / 14.5, 200 16.2 / 16.6, 700 23.9 / 24.7; behind 1024 40 tokens 26.0 / 26.8.
 //
 // Measured (32 / 8 heads, bf16; causal count), single calls and SM clock: 1 x 16384 tokens 2.0 ms at 1.83 GHz = 1100 TFLOP/s, 2.25 ms at the
 // 1.62 GHz that are left after some dozens of them (power), 4 x 4096 0.63 ms, 12 prompts of 60 to 1500 tokens 150 us. One query tile a block with a
@@ -118,9 +121,9 @@ int varlen_prefill_tc(const void* q, const void* k, const void* v, const int32_t
     if (!p.error_word) { set_error("zp_varlen_prefill(tcgen05): no device error word"); return (int)ZP_ERR_CUDA; }
     return launch_prefill_tc(q, k, v, p, B, max_seqlen_q, kv_stride_page, total_q, total_k, st);
   };
-  // (single tiles: two groups of softmax warps)
-  if (dtype == ZP_DTYPE_BF16) return mode == SINGLE ? run(PrefillTc<__nv_bfloat16, 2>{}) : run(PrefillTc<__nv_bfloat16, 1>{});
-  if (dtype == ZP_DTYPE_F16) return mode == SINGLE ? run(PrefillTc<__half, 2>{}) : run(PrefillTc<__half, 1>{});
+  const bool two = mode == SINGLE && !table && max_seqlen_q <= 512 && total_k <= total_q;      // groups of softmax warps
+  if (dtype == ZP_DTYPE_BF16) return two ? run(PrefillTc<__nv_bfloat16, 2>{}) : run(PrefillTc<__nv_bfloat16, 1>{});
+  if (dtype == ZP_DTYPE_F16) return two ? run(PrefillTc<__half, 2>{}) : run(PrefillTc<__half, 1>{});
   set_error("zp_varlen_prefill(tcgen05): 16-bit tensors only");
   return ZP_ERR_UNSUPPORTED;
 }
