@@ -36,3 +36,17 @@ def test_prompts_of_single_tiles_and_few_keys_have_two_groups(heads, kv_heads, n
         k, v, table = draw(n, kv_heads), draw(n, kv_heads), None
     form = _form(r"attn_tc_kernel<zp::PrefillTc", lambda: varlen_prefill_attention(q, k, v, n, cu, n + cached, cuk, block_table=table, impl="tcgen05"))
     assert form[1].rstrip("> ") == str(groups)
+
+
+@pytest.mark.parametrize("E,K,n_out,tiles", [
+    (16, 512, 4096, 1), (16, 1024, 1536, 2), (16, 1024, 1024, 1), (16, 2048, 1024, 1),              # 1250 places an expert; 4.4 tiles an SM at 1024 columns, 6.6 at 1536
+    (32, 1024, 2048, 1), (32, 1024, 3072, 2), (32, 1536, 1536, 1), (32, 1536, 2048, 2), (32, 2048, 1536, 2), (32, 2048, 1024, 1)])      # 625
+def test_gathered_rows_go_in_pairs_where_the_shared_weights_pay(E, K, n_out, tiles):
+    from zipage_b200.layers.feed_forward import grouped_gemm
+    M = 20000
+    x = torch.randn(5000, K, device="cuda", generator=_gen(K)).to(torch.bfloat16)
+    w = (torch.randn(E, n_out, K, device="cuda", generator=_gen(n_out)) / K ** 0.5).to(torch.bfloat16)
+    rows = torch.randint(0, 5000, (M,), device="cuda", generator=_gen(1)).to(torch.int32)
+    off = (torch.arange(E + 1, device="cuda") * (M // E)).to(torch.int32)
+    form = _form("grouped_gemm_tc_kernel", lambda: grouped_gemm(x, w, off, M, rows=rows, act="silu_mul"))
+    assert form == ["256", "2", "2", str(tiles)]

@@ -72,7 +72,7 @@ template <int BN, int MT> __device__ __forceinline__ GtTile gt_tile(const GtPara
 __device__ __forceinline__ void gt_copy16(uint32_t dst, const void* src, int bytes) {   // the rest of 16 bytes becomes zero
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
-// the copies of the stage issued GT_LAG stages ago (or, LEFT = 0, all) have landed: tell the tensor cores
+// the copies of the stage issued LEFT stages ago (LEFT = 0: all of them) have landed: tell the tensor cores
 template <int LEFT> __device__ __forceinline__ void gt_publish(uint64_t* bar, int lane) {
   asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -85,7 +85,7 @@ template <int MODE, int MT> constexpr int gt_threads() { return 64 + 128 * MT * 
 template <int BN, int ACT, int MODE, int MT>
 __global__ void __launch_bounds__((gt_threads<MODE, MT>()), 1)
 grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const GtParams p) {
-  static_assert(MT == 1 || MODE != GT_FEW, "pairs of tiles are for many places");
+  static_assert(MT == 1 || MODE == GT_GATHER, "pairs of tiles are for gathered rows");
   constexpr int B_AT = MT * GT_A, STAGE = B_AT + BN * 128, LAG = gt_lag(MT);
   extern __shared__ unsigned char smem_raw[];
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -160,10 +160,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
         for (int k = 0; k < p.kb; ++k) {
           if (!mbar_wait(&sh.empty[slot], (round & 1) ^ 1, abortp, p.error_word, 941)) { ok = false; break; }
           unsigned char* dst = ring + slot * STAGE;
-          const int own = (tl.count + 127) >> 7;           // tiles of the item
-          mbar_arrive_expect_tx(&sh.full[slot], (uint32_t)((MODE == GT_TILE ? own * GT_A : 0) + BN * 128));
-          if (MODE == GT_TILE)
-            for (int m = 0; m < own; ++m) tma_load_5d(dst + m * GT_A, &tmX, &sh.full[slot], k * 64, tl.first + m * 128, 0, 0, 0);
+          mbar_arrive_expect_tx(&sh.full[slot], (uint32_t)((MODE == GT_TILE ? GT_A : 0) + BN * 128));
+          if (MODE == GT_TILE) tma_load_5d(dst, &tmX, &sh.full[slot], k * 64, tl.first, 0, 0, 0);
           tma_load_5d(dst + B_AT, &tmW, &sh.full[slot], k * 64, tl.n0, tl.e, 0, 0);
           if (++slot == p.stages) { slot = 0; ++round; }
         }
@@ -365,15 +363,23 @@ template <int BN, int ACT, int MODE, int MT> static int gt_launch(const GroupedA
   return check_launch("zp_grouped_gemm(tcgen05)");
 }
 
-// About so many tiles an SM from which gathered rows go two tiles an item.  Calls with both products of 64 (32) experts, one tile an item / two: 11 tiles
-// an SM 498 / 470 us, (10.8) 448 / 423, 8.6 403 / 390, 6.1 315 / 291; 5.8 (278 / 279), 5.2 290 / 290 and 143 / 142, 4.9 148 / 151, 2.6 227 / 239: the last
-// wave of larger items costs what the shared weights gain.
-constexpr int64_t GT_PAIR_TILES = 6 * 148;
+// Whether gathered rows go two tiles an item.  An item's epilogue is not covered then, its last wave is larger, and its second tile may be missing, which
+// the shared weights have to make up for: never where K is below 1024, from about 6 tiles an SM on where experts have 1024 places and more each or K is
+// 2048 or more, else from as many more as K is smaller.  Time with two over time with one, products of 8 to 64 experts:
+//   K 256 1.00 to 1.25 (gated 1.1 to 1.4), 512 0.96 to 1.35, 768 0.92 to 1.25, whatever the tiles;
+//   K 1024, 7 tiles an SM, 1024 places an expert and more, 0.91 to 0.96; fewer places, 6 to 10 tiles, 0.99 to 1.16, 11 and more 0.89 to 1.03 (one of 19 1.07);
+//   K 1536, 7 tiles, 1024 places and more 0.90 to 0.94; fewer, 6 and 7 tiles, 0.99 to 1.10, 8 and more 0.84 to 1.06 (mostly below 0.97);
+//   K 2048, 6 tiles and more, 0.84 to 1.02.
+// Fewer tiles (calls with both products): 5.8 (278 / 279), 5.2 290 / 290 and 143 / 142, 4.9 148 / 151, 2.6 227 / 239 us.
+static bool gt_pairs(const GroupedArgs& a, int bn) {
+  const int64_t tiles = ((int64_t)a.places / 128 + a.E / 2) * ((a.Nout + bn - 1) / bn);
+  return a.K >= 1024 && tiles >= 6 * 148 && (a.places / 1024 >= a.E || tiles * (a.K < 2048 ? a.K : 2048) >= (int64_t)148 * 12 * 1024);
+}
 
 template <int BN, int ACT> static int gt_pick(const GroupedArgs& a, bool many, cudaStream_t st) {
   if (!many) return gt_launch<BN, ACT, GT_FEW, 1>(a, st);
   if constexpr (BN == 256)
-    if (a.rows && ((int64_t)a.places / 128 + a.E / 2) * ((a.Nout + BN - 1) / BN) >= GT_PAIR_TILES) return gt_launch<BN, ACT, GT_GATHER, 2>(a, st);
+    if (a.rows && gt_pairs(a, BN)) return gt_launch<BN, ACT, GT_GATHER, 2>(a, st);
   return a.rows ? gt_launch<BN, ACT, GT_GATHER, 1>(a, st) : gt_launch<BN, ACT, GT_TILE, 1>(a, st);
 }
 
