@@ -50,3 +50,30 @@ def test_gathered_rows_go_in_pairs_where_the_shared_weights_pay(E, K, n_out, til
     off = (torch.arange(E + 1, device="cuda") * (M // E)).to(torch.int32)
     form = _form("grouped_gemm_tc_kernel", lambda: grouped_gemm(x, w, off, M, rows=rows, act="silu_mul"))
     assert form == ["256", "2", "2", str(tiles)]
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("taps,bias", [(2, False), (4, False), (4, True)])
+def test_convolutions_of_many_blocks_have_fewer_tokens_in_flight(dtype, taps, bias):
+    """3072 channels in one call, where four blocks an SM leave fewer waves than three, and in thirds, where they do not; three taps stay as they are."""
+    from zipage_b200.layers.short_conv import short_conv
+    g, C, lens = _gen(taps), 3072, [2528, 31, 1, 700]
+    n = sum(lens)
+    x = torch.randn(n, C, device="cuda", generator=g).to(dtype)
+    cu, ctx, slots = _cu(lens), torch.tensor(lens, dtype=torch.int32, device="cuda") + 5, torch.arange(4, dtype=torch.int32, device="cuda")
+    ring0 = torch.randn(4, taps, C, device="cuda", generator=g).to(dtype)
+    w, b = torch.randn(taps, C, device="cuda", generator=g), torch.randn(C, device="cuda", generator=g) if bias else None
+
+    def run(step, taps=taps):
+        out, rings = torch.empty_like(x), []
+        for c in range(0, C, step):
+            s = slice(c, c + step)
+            rings.append(ring0[:, :taps, s].contiguous())
+            short_conv(x[:, s], w[:taps, s].contiguous(), rings[-1], ctx, slots, cu, max(lens), out[:, s], bias=None if b is None else b[s].contiguous())
+        return out, torch.cat(rings, -1)
+    many = lambda *a: _form("short_conv_kernel", lambda: run(*a))[-1] in ("true", "1")
+    assert many(C) and not many(C // 3)
+    for whole, parts in zip(run(C), run(C // 3)):
+        assert torch.equal(whole, parts)
+    if taps == 4:
+        assert not many(C, 3)

@@ -13,10 +13,10 @@ struct ConvArgs {
 __device__ __forceinline__ float cv_ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float cv_rcp(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 constexpr int CV_THREADS = 256, CV_MAX_TAPS = 8;
-// Tokens whose loads are in flight (whole turns of the circle of inputs), and tokens of a thread.  Up to four taps four blocks share an SM.  6200 tokens of 8192 channels, 4 taps: 56.5 us with four tokens in flight and four blocks an SM, 61.7 with eight and three (104 with
-// eight and four, 138 with four and five: registers spill); 16 tokens a thread 57.6, 48 57.2, 64 66.
-constexpr int cv_batch(int taps) { return (taps <= 4 ? 4 : 8) / taps * taps; }
-constexpr int cv_run(int taps) { return taps <= 4 ? 32 / cv_batch(taps) * cv_batch(taps) : 4 * cv_batch(taps); }
+// Tokens whose loads are in flight (whole turns of the circle of inputs), and tokens of a thread.  MANY: four in flight instead of eight, so
+// that four blocks share an SM instead of three.
+constexpr int cv_batch(int taps, bool many) { return (many ? 4 : 8) / taps * taps; }
+constexpr int cv_run(int taps) { return 4 * cv_batch(taps, false); }
 
 template <typename T, int V> struct __align__(V == 1 ? sizeof(T) : 8) ChanVec { T e[V]; };        // V * sizeof(T) = 8, or one entry
 template <typename T, int V> __device__ __forceinline__ ChanVec<T, V> cv_load(const T* p) {
@@ -37,9 +37,10 @@ template <typename T, int V> __device__ __forceinline__ void cv_store(T* p, cons
   else *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(&r);
 }
 
-template <typename T, int V, int TAPS, bool BIAS>
-__global__ void __launch_bounds__(CV_THREADS, TAPS <= 4 ? 4 : 2) short_conv_kernel(const ConvArgs a) {
-  constexpr int BATCH = cv_batch(TAPS), RUN = cv_run(TAPS);
+template <typename T, int V, int TAPS, bool BIAS, bool MANY>
+__global__ void __launch_bounds__(CV_THREADS, MANY ? 4 : TAPS <= 4 ? 3 : 2) short_conv_kernel(const ConvArgs a) {
+  constexpr int BATCH = cv_batch(TAPS, MANY), RUN = cv_run(TAPS);
+  static_assert(RUN % BATCH == 0, "whole batches");
   const int b = blockIdx.z, c = (blockIdx.x * CV_THREADS + threadIdx.x) * V;
   const int row0 = a.cu_q[b], count = a.cu_q[b + 1] - row0, ctx = a.context_lens[b], slot = a.slots[b];
   const int t0 = blockIdx.y * RUN, t1 = min(count, t0 + RUN);
@@ -127,9 +128,27 @@ template <typename T> __global__ void __launch_bounds__(256) conv_keep_kernel(co
     ring[(int64_t)((ctx - 1 - j) % a.taps) * a.C] = reinterpret_cast<const T*>(a.x)[(int64_t)(row0 + count - 1 - j) * a.x_stride + c];
 }
 
+// Four tokens in flight where four blocks an SM leave fewer waves of them than three: a wave takes up to 1.3 times as long.  6200 tokens in four
+// portions, bf16, four taps, eight / four in flight (us): 1024 channels (316 blocks) 18.5 / 19.0, 2048 (632) 22.0 / 24.8, 3072 (948) 34.0 / 26.3,
+// 4096 (1264) 39.3 / 39.1, 6144 (1896) 51.9 / 46.3, 8192 (2528) 67.4 / 59.2; 100 tokens (32) 14.8 / 15.8.  fp16 and fp32, bias and two taps alike.
+// Three taps lose by it (53.1 / 53.4 at best, 100 tokens 10.3 / 14.0); with one tap, or one channel a thread, four blocks share an SM anyway.
+// Other runs than 32 tokens at 8192 channels: 16 57.6, 48 57.2, 64 66 for 56.5; eight in flight in the registers of four blocks 104, four in those of
+// five 138.
+static bool conv_many(int64_t blocks) { return (blocks + 4 * 148 - 1) / (4 * 148) < (blocks + 3 * 148 - 1) / (3 * 148); }
+
+template <typename T, int V, int TAPS, bool BIAS> static void launch_conv(const ConvArgs& a, dim3 grid, cudaStream_t st) {
+  if constexpr (V > 1 && (TAPS == 2 || TAPS == 4)) {
+    if (conv_many((int64_t)grid.x * grid.y * grid.z)) {
+      short_conv_kernel<T, V, TAPS, BIAS, true><<<grid, CV_THREADS, 0, st>>>(a);
+      return;
+    }
+  }
+  short_conv_kernel<T, V, TAPS, BIAS, false><<<grid, CV_THREADS, 0, st>>>(a);
+}
+
 template <typename T, int V, bool BIAS> static int conv_by_taps(const ConvArgs& a, dim3 grid, cudaStream_t st) {
   switch (a.taps) {
-#define ZP_CONV(n) case n: short_conv_kernel<T, V, n, BIAS><<<grid, CV_THREADS, 0, st>>>(a); break
+#define ZP_CONV(n) case n: launch_conv<T, V, n, BIAS>(a, grid, st); break
     ZP_CONV(1); ZP_CONV(2); ZP_CONV(3); ZP_CONV(4); ZP_CONV(5); ZP_CONV(6); ZP_CONV(7); ZP_CONV(8);
 #undef ZP_CONV
     default: return ZP_ERR_UNSUPPORTED;
