@@ -77,3 +77,36 @@ def test_convolutions_of_many_blocks_have_fewer_tokens_in_flight(dtype, taps, bi
         assert torch.equal(whole, parts)
     if taps == 4:
         assert not many(C, 3)
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("width,n,kind,three", [(1024, 1480, "experts", (1, 1, 0)), (1024, 1481, "experts", (0, 0, 0)), (1024, 592, "experts", (1, 1, 1)),
+                                                (1536, 2000, "experts", (1, 1, 0)), (2048, 592, "experts", (1, 1, 1)), (4096, 444, "experts", (1, 1, 1)),
+                                                (4096, 445, "experts", (0, 0, 0)), (2048, 100, "plain", (0, 0, 0)), (2048, 100, "pair", (0, 0, 0)),
+                                                (5120, 8, "experts", (0, 0, 0)), (1030, 8, "experts", (0, 0, 0))])
+def test_layer_boundaries_with_registers_for_the_experts_rows(dtype, width, n, kind, three):
+    """Rows in one call and in parts of at most 400: the same bits, whichever form they take."""
+    from zipage_b200.layers.row_ops import join_norms
+    g, top = _gen(width + n), 5
+    z = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, a, w1, w2 = z(n, width), z(n, width).to(dtype), z(width), z(width)
+    more = {}
+    if kind == "experts":
+        y, pos, wts = z(n * top, width).to(dtype), torch.randperm(n * top, device="cuda", generator=g).to(torch.int32).view(n, top), z(n, top)
+    elif kind == "pair":
+        m = [z(n, width).to(dtype) for _ in range(2)]
+
+    def run(step):
+        out = []
+        for i in range(0, n, step):
+            s = slice(i, i + step)
+            if kind == "experts":
+                more.update(y=y, pos=pos[s], weights=wts[s])
+            elif kind == "pair":
+                more.update(pair=((m[0][s], w1), (m[1][s], w2)))
+            r = x[s].clone()
+            out.append([r] + join_norms(r, [(w1, w2), (w2, None)], 1e-5, dtype, a=a[s], **more))
+        return [torch.cat(t) for t in zip(*out)]
+    for whole, parts in zip(run(n), run(400)):
+        assert torch.equal(whole, parts)
+    assert (_form("join_norms_kernel", lambda: run(n))[-1] == "3") == bool(three[list(TYPES).index(dtype)])

@@ -159,10 +159,11 @@ gelu_tanh_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t n, int64_
 // ---------------------------------------------------------------------------------------------
 // x += ls_a * a + ls_b * (sigmoid(gate) * b + sum_k w_k y[pos_k]) + pair_scale * (rms(m1) * mw1 + rms(m2) * mw2);  out_i = T(norm of x with w_i, bias_i), the layer
 // norm or (rms) the one that takes no mean off.
-// Bound by the loads in flight: with registers for three blocks an SM the experts' rows of an entry are all on their way together (4096 rows of
-// 2048, six experts: 51.5 us; 57.4 in the 34 registers that the compiler chooses for itself, 57.3 in those for five blocks).
 // Every part may be missing.  One block per row; VPT float4 per thread stay in registers (VPT = 0: any
 // row length, each thread reads back the entries of x that it wrote).
+//
+// Bound by the loads in flight, of a thread and of an SM: BLOCKS = 3 leaves registers for four of an entry's expert rows at a time, 0 is the
+// compiler's choice, with fewer registers and more blocks (see launch_join_rows).
 // ---------------------------------------------------------------------------------------------
 struct JoinArgs {
   float* x;
@@ -230,8 +231,8 @@ __device__ __forceinline__ void join_norm(const JoinArgs& p, int64_t row, int c,
 }
 
 constexpr int JOIN_TOP = 64;
-template <typename T, int VPT, bool PAIR>
-__global__ void __launch_bounds__(256, 3) join_norms_kernel(const JoinArgs p) {
+template <typename T, int VPT, bool PAIR, int BLOCKS = 0>
+__global__ void __launch_bounds__(256, BLOCKS) join_norms_kernel(const JoinArgs p) {
   __shared__ float red[32];
   __shared__ float swts[JOIN_TOP];
   __shared__ int32_t spos[JOIN_TOP];
@@ -315,12 +316,31 @@ __global__ void __launch_bounds__(256, 3) join_norms_kernel(const JoinArgs p) {
   }
 }
 
+// Up to so many rows get the registers of three blocks an SM, where experts' rows are gathered and no pair is; more blocks an SM are better
+// everywhere else.  The compiler's own / three blocks (us; bf16, top 6): rows of 1024, 16 of them 4.7 / 4.4, 444 7.0 / 6.6, 1500 13.5 / 12.8, 4096 27.7 /
+// 29.4; of 2048 16 10.2 / 8.4, 444 11.6 / 9.9, 4096 57.3 / 50.5; of 4096 16 13.7 / 13.2, 600 18.3 / 28.5, 4096 100 / 110; of 6144 4096 158 /
+// 200.  fp32: of 1024 600 7.9 / 7.6, 1500 15.9 / 17.4; of 2048 600 12.9 / 12.1, 1500 28.6 / 31.2; of 4096 444 19.1 / 18.2, 600 22.5 / 31.7.  Without
+// experts: 4096 rows of 1024 13.5 / 14.4, of 5120 63 / 73; pairs of 2048 35.6 / 43.7.
+template <typename T, int VPT> constexpr int join_rows_of_three() {
+  if (VPT == 4) return 3 * 148;
+  if (sizeof(T) == 4) return 4 * 148;
+  return VPT == 1 ? 10 * 148 : 0x7fffffff;
+}
+template <typename T, int VPT, bool PAIR> static void launch_join_rows(const JoinArgs& p, int n_rows, cudaStream_t st) {
+  if constexpr (!PAIR && VPT <= 4) {
+    if (p.y && n_rows <= join_rows_of_three<T, VPT>()) {
+      join_norms_kernel<T, VPT, PAIR, 3><<<n_rows, 256, 0, st>>>(p);
+      return;
+    }
+  }
+  join_norms_kernel<T, VPT, PAIR><<<n_rows, 256, 0, st>>>(p);
+}
 template <typename T, bool PAIR> static void launch_join(const JoinArgs& p, int n_rows, bool vec, cudaStream_t st) {
   if (!vec) join_norms_kernel<T, 0, PAIR><<<n_rows, 256, 0, st>>>(p);
-  else if (p.H <= 1024) join_norms_kernel<T, 1, PAIR><<<n_rows, 256, 0, st>>>(p);
-  else if (p.H <= 2048) join_norms_kernel<T, 2, PAIR><<<n_rows, 256, 0, st>>>(p);
-  else if (p.H <= 4096) join_norms_kernel<T, 4, PAIR><<<n_rows, 256, 0, st>>>(p);
-  else join_norms_kernel<T, 8, PAIR><<<n_rows, 256, 0, st>>>(p);
+  else if (p.H <= 1024) launch_join_rows<T, 1, PAIR>(p, n_rows, st);
+  else if (p.H <= 2048) launch_join_rows<T, 2, PAIR>(p, n_rows, st);
+  else if (p.H <= 4096) launch_join_rows<T, 4, PAIR>(p, n_rows, st);
+  else launch_join_rows<T, 8, PAIR>(p, n_rows, st);
 }
 
 // ---------------------------------------------------------------------------------------------
