@@ -110,3 +110,28 @@ def test_layer_boundaries_with_registers_for_the_experts_rows(dtype, width, n, k
     for whole, parts in zip(run(n), run(400)):
         assert torch.equal(whole, parts)
     assert (_form("join_norms_kernel", lambda: run(n))[-1] == "3") == bool(three[list(TYPES).index(dtype)])
+
+
+@pytest.mark.parametrize("dtype,D,n,blocks", [
+    (torch.bfloat16, 128, 64, 3), (torch.bfloat16, 128, 6000, 3), (torch.float16, 128, 64, 3), (torch.float16, 128, 1900, 3), (torch.float16, 128, 2000, 0),
+    (torch.float16, 128, 1000, 0), (torch.float32, 128, 64, 0), (torch.float32, 128, 1500, 0), (torch.float32, 128, 1600, 3), (torch.float32, 128, 1000, 3),
+    (torch.float16, 64, 2000, 3), (torch.float32, 64, 64, 3)])
+@pytest.mark.parametrize("packed", [True, False])
+def test_registers_of_the_head_norms(dtype, D, n, blocks, packed):
+    """One call and parts of 500 rows: the same bits, whichever form they take."""
+    from zipage_b200.layers import step_ops as P
+    heads, kv_heads, g = 32, 8, _gen(n)
+    qkv = torch.randn(n, (heads + 2 * kv_heads) * D, device="cuda", generator=g).to(dtype)
+    pos, cs = torch.randint(0, 4096, (n,), device="cuda", generator=g), P.rope_cos_sin_cache(D, 4096, 1e6, "cuda")
+    w = [(1 + 0.1 * torch.randn(D, device="cuda", generator=g)).to(dtype) for _ in range(2)]
+    slot = torch.randperm(n, device="cuda", generator=g).to(torch.int32)
+
+    def run(step):
+        cache = [torch.zeros((n + 255) // 256, 256, kv_heads, D, dtype=dtype, device="cuda") for _ in range(2)]
+        parts = [P.qk_norm_rope_store(qkv[i:i + step], pos[i:i + step], cs, *w, 1e-6, heads, kv_heads, D, *cache, slot[i:i + step], return_v=packed)
+                 for i in range(0, n, step)]
+        return [torch.cat(t) for t in zip(*parts)] + cache
+    for whole, parts in zip(run(n), run(500)):
+        assert torch.equal(whole, parts)
+    form = _form("qk_norm_rope_store_kernel", lambda: run(n))
+    assert form[:3] == [TYPES[dtype], str(D), str(blocks)] and (form[3] in ("true", "1")) == packed

@@ -171,8 +171,14 @@ silu_and_mul_kernel(const T* x, T* out, int I, Index total_vec) {
 // tokens: 32 heads a warp, so that cosines, sines and weights are fetched once for eight turns.  Few tokens (below QK_SPREAD,
 // where a warp per token does not fill the SMs): four heads a warp, one turn of latency.
 // 32 / 8 heads of 128, bf16: 16384 tokens 89 us = 4.9 TB/s (16 heads a warp 96, 8 105, 4 130; one warp for all kinds 114), 4 tokens
-// 2.6 us (7.6).  12 prompts of 60 to 1500 tokens, values packed too: 51 us for three blocks an SM with registers to match (54 where the compiler
-// chooses for itself, 54 for four blocks, 57 for five).
+// 2.6 us (7.6).
+//
+// Registers (BLOCKS: of so many blocks an SM; 0: what the compiler takes for itself), heads of 128; those of 64 are the same either way.
+// bf16 has 66 by itself and 79 of three blocks, which never lose: 4 tokens 1.72 -> 1.64 us, 2000 15.0 -> 13.5, 8192 43.5 -> 41.4, 12 prompts
+// of 60 to 1500 tokens with packed values 54 -> 51 (54 for four blocks, 57 for five).  fp16 has 64 by itself, which is four blocks, or 78 of
+// three: more registers are better while the blocks are no more than a wave or so (1100 tokens 12.1 -> 10.5, 1600 13.8 -> 11.1), more blocks
+// from there on (1000 tokens in 1500 blocks 8.8 -> 9.5, 8192 38.7 -> 41.4).  fp32 has 90 by itself, two blocks, and spills a few
+// in the 80 of three: 1100 tokens 12.1 -> 16.0, 4 tokens 1.70 -> 1.78, but 1000 12.9 -> 11.9 and 8192 68.8 -> 65.1.
 // ---------------------------------------------------------------------------------------------
 constexpr int QK_SPREAD = 1024;
 
@@ -237,8 +243,8 @@ __device__ __forceinline__ void norm_rope_head(const Chunk<T, D / 16>& ca, const
   }
 }
 
-template <typename T, int D>
-__global__ void __launch_bounds__(256, 3) qk_norm_rope_store_kernel(const QkArgs a) {
+template <typename T, int D, int BLOCKS, bool PACK>
+__global__ void __launch_bounds__(256, BLOCKS) qk_norm_rope_store_kernel(const QkArgs a) {
   constexpr int P = D / 16;
   const int lane = threadIdx.x & 31, l8 = lane & 7, hg = lane >> 3;   // 4 heads per warp at a time
   const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), part = blockIdx.y;
@@ -269,14 +275,24 @@ __global__ void __launch_bounds__(256, 3) qk_norm_rope_store_kernel(const QkArgs
   load_head(h_begin + hg, ca, cb);
   const int slot = !is_q && a.slot_mapping ? a.slot_mapping[n] : -1;
   if (is_v) {
-    if (slot == -1 && !a.v_out) return;
-    T* d0 = a.v_out ? reinterpret_cast<T*>(a.v_out) + (int64_t)n * a.Hkv * D : nullptr;
-    T* d1 = slot != -1 ? reinterpret_cast<T*>(a.v_cache) + (int64_t)slot * a.Hkv * D : nullptr;
+    if constexpr (PACK) {
+      T* d0 = reinterpret_cast<T*>(a.v_out) + (int64_t)n * a.Hkv * D;
+      T* d1 = slot != -1 ? reinterpret_cast<T*>(a.v_cache) + (int64_t)slot * a.Hkv * D : nullptr;
+      for (int h = h_begin + hg; h < h_end; h += 4) {
+        load_head(h + 4, na, nb);
+        const int64_t at = (int64_t)h * D + l8 * P;
+        st_chunk<T, P>(d0 + at, ca); st_chunk<T, P>(d0 + at + D / 2, cb);
+        if (d1) { st_chunk<T, P>(d1 + at, ca); st_chunk<T, P>(d1 + at + D / 2, cb); }
+        ca = na; cb = nb;
+      }
+      return;
+    }
+    if (slot == -1) return;
+    T* dst = reinterpret_cast<T*>(a.v_cache) + (int64_t)slot * a.Hkv * D;
     for (int h = h_begin + hg; h < h_end; h += 4) {
       load_head(h + 4, na, nb);
-      const int64_t at = (int64_t)h * D + l8 * P;
-      if (d0) { st_chunk<T, P>(d0 + at, ca); st_chunk<T, P>(d0 + at + D / 2, cb); }
-      if (d1) { st_chunk<T, P>(d1 + at, ca); st_chunk<T, P>(d1 + at + D / 2, cb); }
+      st_chunk<T, P>(dst + (int64_t)h * D + l8 * P, ca);
+      st_chunk<T, P>(dst + (int64_t)h * D + D / 2 + l8 * P, cb);
       ca = na; cb = nb;
     }
     return;
@@ -715,8 +731,17 @@ extern "C" int zp_qk_norm_rope_store_v(const void* qkv, const int64_t* positions
   a.nk = (Hkv + a.per - 1) / a.per;
   const dim3 grid((n_tokens + n_triples + 7) / 8, a.nq + 2 * a.nk);   // eight warps per block, one token each
   ZP_DISPATCH_DTYPE(dtype, T, {
-    if (D == 128) zp::launch_early(zp::qk_norm_rope_store_kernel<T, 128>, grid, 256, 0, st, a);
-    else zp::launch_early(zp::qk_norm_rope_store_kernel<T, 64>, grid, 256, 0, st, a);
+    constexpr bool bf16 = std::is_same<T, __nv_bfloat16>::value;
+    const int64_t blocks = (int64_t)grid.x * grid.y;
+    const bool three = bf16 || (std::is_same<T, float>::value ? blocks > 4 * 148 : blocks <= 5 * 148);
+    auto go = [&](auto pack) {
+      constexpr bool PACK = decltype(pack)::value;
+      if (D == 64) zp::launch_early(zp::qk_norm_rope_store_kernel<T, 64, 3, PACK>, grid, 256, 0, st, a);
+      else if (three) zp::launch_early(zp::qk_norm_rope_store_kernel<T, 128, 3, PACK>, grid, 256, 0, st, a);
+      else zp::launch_early(zp::qk_norm_rope_store_kernel<T, 128, bf16 ? 3 : 0, PACK>, grid, 256, 0, st, a);
+    };
+    if (v_out) go(std::true_type());
+    else go(std::false_type());
   });
   return zp::check_launch("zp_qk_norm_rope_store");
 }
