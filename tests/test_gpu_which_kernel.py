@@ -7,14 +7,15 @@ import torch
 from test_gpu_attn_tc import _cu, _kernels
 
 pytestmark = pytest.mark.gpu
-TYPES = {torch.bfloat16: "__nv_bfloat16", torch.float16: "__half", torch.float32: "float"}
+TYPES = {torch.bfloat16: "13__nv_bfloat16", torch.float16: "6__half", torch.float32: "f"}      # (as they are in a symbol)
 
 
 def _form(name, call):
-    """Template arguments of the kernel `name` that `call` launches."""
-    found = set(re.findall(name + r"<([^()]*(?:\(\w+\)[^()]*)*)>\(", _kernels(call)))
+    """Template arguments of the kernel (or, of a kernel's parameters) `name` that `call` launches."""
+    argument = "13__nv_bfloat16|6__half|f|L[ib][0-9]+E"
+    found = set(re.findall(f"{len(name)}{name}I((?:{argument})+)E", _kernels(call)))
     assert len(found) == 1, found
-    return [re.sub(r"\(\w+\)", "", a).strip() for a in found.pop().split(",")]
+    return [re.sub("^L[ib]([0-9]+)E$", r"\1", a) for a in re.findall(argument, found.pop())]
 
 
 def _gen(seed):
@@ -34,8 +35,8 @@ def test_prompts_of_single_tiles_and_few_keys_have_two_groups(heads, kv_heads, n
         k, v, table = draw(pages, 256, kv_heads), draw(pages, 256, kv_heads), torch.arange(pages, dtype=torch.int32, device="cuda")[None]
     else:
         k, v, table = draw(n, kv_heads), draw(n, kv_heads), None
-    form = _form(r"attn_tc_kernel<zp::PrefillTc", lambda: varlen_prefill_attention(q, k, v, n, cu, n + cached, cuk, block_table=table, impl="tcgen05"))
-    assert form[1].rstrip("> ") == str(groups)
+    form = _form("PrefillTc", lambda: varlen_prefill_attention(q, k, v, n, cu, n + cached, cuk, block_table=table, impl="tcgen05"))
+    assert form == [TYPES[torch.bfloat16], str(groups)]
 
 
 @pytest.mark.parametrize("E,K,n_out,tiles", [
@@ -71,7 +72,7 @@ def test_convolutions_of_many_blocks_have_fewer_tokens_in_flight(dtype, taps, bi
             rings.append(ring0[:, :taps, s].contiguous())
             short_conv(x[:, s], w[:taps, s].contiguous(), rings[-1], ctx, slots, cu, max(lens), out[:, s], bias=None if b is None else b[s].contiguous())
         return out, torch.cat(rings, -1)
-    many = lambda *a: _form("short_conv_kernel", lambda: run(*a))[-1] in ("true", "1")
+    many = lambda *a: _form("short_conv_kernel", lambda: run(*a))[-1] == "1"
     assert many(C) and not many(C // 3)
     for whole, parts in zip(run(C), run(C // 3)):
         assert torch.equal(whole, parts)
@@ -134,4 +135,4 @@ def test_registers_of_the_head_norms(dtype, D, n, blocks, packed):
     for whole, parts in zip(run(n), run(500)):
         assert torch.equal(whole, parts)
     form = _form("qk_norm_rope_store_kernel", lambda: run(n))
-    assert form[:3] == [TYPES[dtype], str(D), str(blocks)] and (form[3] in ("true", "1")) == packed
+    assert form[:3] == [TYPES[dtype], str(D), str(blocks)] and form[3] == str(int(packed))
