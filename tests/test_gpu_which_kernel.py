@@ -136,3 +136,40 @@ def test_registers_of_the_head_norms(dtype, D, n, blocks, packed):
         assert torch.equal(whole, parts)
     form = _form("qk_norm_rope_store_kernel", lambda: run(n))
     assert form[:3] == [TYPES[dtype], str(D), str(blocks)] and form[3] == str(int(packed))
+
+
+def _decoded(B, kp, vp, window=1024, width=35):
+    """Arguments of a decoded window of 16 heads on 8, every sequence with all of its keys."""
+    g, page = _gen(B + kp), 64
+    draw = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    table = torch.randperm(B * width, device="cuda", generator=g).to(torch.int32).view(B, width)
+    ctx = torch.full((B,), width * page, dtype=torch.int32, device="cuda")
+    return draw(B, 16 * kp), draw(B * width, page, 8, kp), draw(B * width, page, 8, vp), ctx, table, 16, kp, vp, kp ** -0.5, window
+
+
+@pytest.mark.parametrize("B,kp,vp,merged", [
+    (24, 128, 128, True), (28, 128, 128, False), (32, 128, 128, False), (60, 128, 128, True), (40, 64, 64, True), (48, 64, 64, False), (8, 256, 256, True),
+    (16, 256, 256, False), (16, 192, 128, True), (32, 192, 128, False), (48, 192, 128, True), (24, 96, 96, True)])
+def test_decoded_windows_split_as_the_sms_hold_blocks(B, kp, vp, merged):
+    """More than one split leaves a merge behind it; the shared memory of a block counts keys and values by their own sizes."""
+    from zipage_b200.layers.attention import window_attention
+    args = _decoded(B, kp, vp)
+    names = _kernels(lambda: window_attention(*args))
+    assert ("window_decode_merge_kernel" in names) == merged
+    out, (q, k, v, _, table) = window_attention(*args), args[:5]
+    for b in (0, B - 1):
+        kk, vv = (t[table[b].long()].flatten(0, 1)[-1024:].double().repeat_interleave(2, 1) for t in (k, v))
+        w = torch.softmax(torch.einsum("hd,nhd->hn", q[b].double().view(16, kp), kk) * kp ** -0.5, -1)
+        ref, mag = torch.einsum("hn,nhd->hd", w, vv), torch.einsum("hn,nhd->hd", w, vv.abs())
+        # weights as two bf16 numbers (2^-16), the result rounded once
+        assert ((out[b].view(16, vp).double() - ref).abs() <= (2.0 ** -8 + 2.0 ** -14) * mag + 1e-6).all()
+
+
+def test_decoded_windows_take_a_workspace_sized_for_a_larger_batch(monkeypatch):
+    from zipage_b200 import _lib as L
+    from zipage_b200.layers import attention as A
+    buf = torch.empty(L.load().zp_window_attention_workspace_bytes(48, 16, 8, 128, 1024), dtype=torch.uint8, device="cuda")
+    args = _decoded(24, 128, 128)
+    want = A.window_attention(*args)
+    monkeypatch.setattr(A, "_workspace", lambda device, nbytes: buf)
+    assert buf.numel() and torch.equal(A.window_attention(*args), want)

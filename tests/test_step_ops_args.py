@@ -76,3 +76,15 @@ def test_small_linear_rejects_bad_arguments():
                 dict(x=C.c_void_p(4100)), dict(w=C.c_void_p(4100)), dict(k=1 << 27), dict(n=2 ** 31 - 1)):
         assert call(**bad) == INVALID, bad
     assert call(dtype=7) != 0
+
+
+def test_window_workspace_covers_every_split_that_a_decode_step_may_take():
+    """Four blocks an SM and at least two tiles of 64 keys each, whatever the head sizes: a caller may size its buffer once, for its largest batch."""
+    lib = L.load()
+    for B in (1, 8, 20, 24, 37, 48, 74, 100):
+        for kv_heads in (1, 8):
+            for dim in (64, 96, 128, 256):
+                for span in (64, 200, 1024, 1536, 1537, 4096):
+                    splits = max(1, min(-(-592 // (B * kv_heads)), ((span + 63) // 64 + 1) // 2, 32))
+                    want = B * 16 * splits * (dim + 2) * 4 if splits > 1 else 0
+                    assert lib.zp_window_attention_workspace_bytes(B, 16, kv_heads, dim, span) == want

@@ -132,7 +132,8 @@ static int launch_simt(const WinArgs& a, int max_q, cudaStream_t st) {
 bool window_mma_supports(const WinArgs& a);
 int window_prefill_mma(const WinArgs& a, int max_q, int dtype, cudaStream_t st);
 int window_decode_mma(const WinArgs& a, int dtype, cudaStream_t st);
-int window_decode_splits(int B, int Hkv, int span, int VP);
+int window_decode_most_splits(int B, int Hkv, int span);
+int window_decode_splits(const WinArgs& a, int span);
 // tcgen05 prefill kernel (zp_window_attn_tc.cu)
 bool window_tc_supports(const WinArgs& a, int total_q, int dtype);
 int window_prefill_tc(const WinArgs& a, int max_q, int total_q, bool forced, cudaStream_t st);
@@ -157,7 +158,7 @@ extern "C" int zp_store_kv_padded(const void* k, const void* v, void* k_cache, v
 
 extern "C" size_t zp_window_attention_workspace_bytes(int B, int Hq, int Hkv, int VP, int span) {
   if (B < 1 || Hkv < 1 || Hq < Hkv) return 0;
-  const int ns = zp::window_decode_splits(B, Hkv, span, VP);
+  const int ns = zp::window_decode_most_splits(B, Hkv, span);
   return ns > 1 ? (size_t)B * Hq * ns * (VP + 2) * sizeof(float) : 0;
 }
 
@@ -209,7 +210,7 @@ extern "C" int zp_window_attention(const void* q, const void* k_cache, const voi
     int span = NBmax * BS;
     if (window > 0 && window + keep < span) span = window + keep;
     if (chunk > 0 && chunk + keep < span) span = chunk + keep;
-    a.nsplit = zp::window_decode_splits(B, Hkv, span, VP);
+    a.nsplit = zp::window_decode_splits(a, span);
     if (a.nsplit > 1) {
       const size_t need = (size_t)B * Hq * a.nsplit * (VP + 2) * sizeof(float);
       ZP_REQUIRE(workspace && workspace_bytes >= need, "zp_window_attention: workspace of %zu bytes, %zu needed",

@@ -12,6 +12,8 @@
 //   c tanh(s / c) - c = -2 c / (1 + E),
 // so a weight costs two exponentials and one reciprocal.  Caps up to c log2(e) = 100 do the same against 0: weights
 // within 2^-100 .. 2^100.
+#include <algorithm>
+
 #include "zp_mma.cuh"
 #include "zp_window_attn.cuh"
 
@@ -463,23 +465,34 @@ static int decode_smem(const WinArgs& a) {
 
 bool window_mma_supports(const WinArgs& a) { return a.KP <= 256 && a.VP <= 256 && a.Hq / a.Hkv <= 16; }
 
-// Four blocks an SM and at least two tiles each; where the keys in sight are few, no more splits than the SMs hold at once (three blocks of 128
-// entries): a second wave of short blocks and the merge cost more than they share out.  Kernels with the merge, cold caches, window 1024, 8 key/value
-// heads of 128 (us; 1, 2, 3, 4, 6 splits; four an SM): 8 sequences 28, 21, 20, 19, 19 (18.5); 16: 29, 25, 25, 29, 31 (31); 24: 36, 30, 38, 37, 41 (37);
-// 32: 37, 47, 43, 44, 51 (43); 48: 46, 55, 60, 60, 70 (55); window 512, 32: 24, 32, 31, 31 (31).  2200 keys in sight, 32: 64, 67, 58, 61, 64 (59): those stay,
-// and so do sizes between those of the compiled kernels (96 entries, 20 sequences 31.5 for 29.1).
-constexpr int WD_FEW = 1536;
-int window_decode_splits(int B, int Hkv, int span, int VP) {
+// Splits of a sequence's keys: four blocks an SM and at least two tiles each.  That is the most that a call takes whatever its head sizes, and what
+// the workspace is sized by.
+int window_decode_most_splits(int B, int Hkv, int span) {
   const int tiles = (span + WM_TK - 1) / WM_TK;
   const int64_t pairs = (int64_t)B * Hkv;
   int64_t s = (148 * 4 + pairs - 1) / pairs;
   if (s > (tiles + 1) / 2) s = (tiles + 1) / 2;
   if (s > 32) s = 32;
-  if (span <= WD_FEW && (VP == 64 || VP == 128)) {
-    const int smem = (16 + 4 * WM_TK) * row_bytes(VP) + 1024, held = 232448 / smem < 4 ? 232448 / smem : 4;
-    if (s > 148 * held / pairs) s = 148 * held / pairs;
-  }
   return s < 1 ? 1 : (int)s;
+}
+// Where the keys in sight are few, no more splits than the SMs hold at once: a second wave of short blocks and the merge cost more than they share
+// out.  Kernels with the merge, cold caches, 8 key/value heads, us for 1, 2, 3, 4, 6 splits (most):
+//   heads of 128, window 1024: 8 sequences 28, 21, 20, 18.7, 19.1 (18.5); 16 28, 25, 24.5, 27 (30); 24 35, 30, 38 (36); 28 35, 41 (40); 32 36, 46 (41); 48 43 (52);
+//     60 71 (70); 300 keys: 28 sequences 16, 22 (23), 60 30 (35); 2200 keys in sight, 32 sequences 64, 77 (66): those stay;
+//   of 64, window 1024: 16 22, 19, 18, 17 (18); 40 31 (28); 48 31 (36); 300 keys, where a fifth block an SM does not pay: 40 13 (15);
+//   of 256: 8 42, 29 (41), 16 42 (60); keys of 192 and values of 128, two blocks an SM, worth their while from three quarters of the SMs' places on:
+//     16 51, 38 (41), 24 61, 60, 53 (58), 32 61 (74).
+// Other sizes of three or four blocks an SM go either way (96, 16 sequences 25.6 for 25.2, 20 30 for 28, 24 31 for 34) and stay.
+constexpr int WD_FEW = 1536, WD_FEWER = 768;
+int window_decode_splits(const WinArgs& a, int span) {
+  const int most = window_decode_most_splits(a.B, a.Hkv, span);
+  const int by_regs = a.VP <= 64 && span > WD_FEWER ? 6 : a.VP <= 128 ? 4 : 2, held = std::min(by_regs, 233472 / (decode_smem(a) + 1024));      // blocks an SM
+  const bool compiled = a.KP == a.VP && (a.VP == 64 || a.VP == 128);
+  if (span > WD_FEW || (!compiled && held > 2)) return most;
+  const int64_t pairs = (int64_t)a.B * a.Hkv, slots = 148 * held, fit = slots / pairs;
+  if (fit == 0) return compiled && span <= WD_FEWER ? 1 : most;
+  if (!compiled && 4 * fit * pairs < 3 * slots) return most;
+  return (int)std::min<int64_t>(most, fit);
 }
 
 template <typename K> static int set_smem(K kern, int bytes, const char* what) {
