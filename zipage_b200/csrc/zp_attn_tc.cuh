@@ -631,7 +631,8 @@ static inline int64_t most_tiles(int heads, int B, int total_q, int max_q) {
 // Prompts, single tiles / pairs: 1 x 100 tokens, 32 heads: 10.3 / 12.1 us; 4 of up to 400, 8 heads: 20.3 / 22.1; 16 of up to 100,
 // 16 heads (256 tiles): 51.5 / 32.5.  (One query tile a block with a pass for the maxima and one for the weights, as it was before, had all its softmax
 // warps on that tile: at up to 148 tiles it took 0 to 3 us less of 10 to 30, from there on 1.2 to 3.5 times as long.)
-// (Windows and latents of few tiles have kernels of their own, and no single tiles here.)
+// (Measured with one group of softmax warps; two for few keys take up to 0.4 us off a single tile.  Windows and latents of few tiles have
+// kernels of their own, and no single tiles here.)
 static inline int pick_pair(int heads_per_kv) { return heads_per_kv % 2 == 0 ? PAIR_HEADS : PAIR_ROWS; }
 static inline int pick_mode(int heads, int heads_per_kv, int B, int total_q, int max_q) {
   return most_tiles(heads, B, total_q, max_q) <= 148 ? SINGLE : pick_pair(heads_per_kv);

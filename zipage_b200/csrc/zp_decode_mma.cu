@@ -13,9 +13,10 @@
 //
 // Short contexts of few sequences are bound by the trips to memory that follow one another: the length, the page, the tiles two at a time, the
 // merges.  So a sequence's first pages are read beside its length, and every split writes its numbers into the shared memory of the block
-// that finishes them: one meeting of the cluster instead of two with the reads between them.  In a step of 4 sequences (700 to 2304 keys, 16 heads on 8) the
-// kernel 11.5 -> 9.6 us; a step of 2 sequences and 4 layers 145 -> 137, of 16 277 -> 268.  The next kernel may begin
-// when the keys have been read: from the first line on, the projection behind it took 5.1 us instead of 3.3. (Three stages for grids of up to two blocks an SM gained nothing.)
+// that finishes them: one meeting of the cluster instead of two with the reads between them.  In a step of 4 sequences (700 to
+// 2304 keys, 16 heads on 8) the kernel 11.5 -> 9.6 us; a step of 2 sequences and 4 layers 145 -> 137, of 16 277 -> 268.  The next
+// kernel may begin when the keys have been read: from the first line on, the projection behind it took 5.1 us instead of 3.3.  (Three
+// stages for grids of up to two blocks an SM gained nothing.)
 #include "zp_mma.cuh"
 
 namespace zp {

@@ -85,7 +85,7 @@ struct LatentPrefillTc {
 // Launches of up to so many 128-row query tiles (about: the counts are on the device) take the kernel of zp_latent_prefill_tc_short.cu.
 // Kernel times of the two, 16 and 32 heads of 128 + 64 (us, this file / short): 32 tiles 13 / 11; 176: 23 to 36 / 13 to 29; 352: 29 to
 // 47 / 22 to 39; 448, equal portions 32 / 40, continued ones 67 / 58; 512: 48 to 76 / 57 to 75, 128-token portions 64 / 48; 560: 52 to
-// 98 / 73 to 112; 1216: 122 to 178 / 187 to 236.
+// 98 / 73 to 112; 1216: 122 to 178 / 187 to 236.  (Measured with one group of softmax warps a tile here; two are up to 3 % faster.)
 constexpr int64_t LATENT_SHORT = 512;
 // Portions of up to one tile leave the second tile of every item empty, which costs the more the longer the work on the first lasts: with
 // a context of four times the portions such launches go there too, whatever their number.  32 portions of 128, 100, 64, 32 tokens,

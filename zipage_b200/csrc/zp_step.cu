@@ -163,8 +163,8 @@ silu_and_mul_kernel(const T* x, T* out, int I, Index total_vec) {
 // Fused q/k RMSNorm + rotary embedding + cache writes.  A warp walks some heads of one kind (q, k or v) of one token, four at a
 // time (eight lanes per head; a lane owns D/16 consecutive dims of each half of the head — the rotation pairs dim d with d + D/2
 // — and moves them as one vector), with the next four heads' loads in flight: q heads -> q_out; k heads -> k_out and the K
-// cache; v heads -> v_out (packed, as attention over the rows themselves takes them) and the V cache, a plain copy.  Rows past the tokens redo the q heads of a window token and write them into
-// the observation-window buffer.
+// cache; v heads -> v_out (PACK: as attention over the rows themselves takes them) and the V cache, a plain copy.  Rows past the tokens
+// redo the q heads of a window token and write them into the observation-window buffer.
 //
 // What bounds it is the loads in flight: with one kind of head a warp keeps one weight and the token's cosines and sines in
 // registers (twice the warps per SM that a walk over all heads of a token left room for), and v heads do no arithmetic.  Many

@@ -167,8 +167,9 @@ static int launch_window_tc(const WinArgs& a, int max_q, int total_q, cudaStream
 }
 
 // Launches of few 128-row query tiles take the kernel of zp_window_attn_tc_short.cu (single tiles, whose waves are finer and whose code is
-// shorter to fetch; the figures are from before this file's kernel became 3 to 7 % faster, so the lines lie on the safe side).  Times of this file's kernel over that one's, heads of 128, portions of 96 to 2560 tokens, 32 heads on 8 unless noted; the
-// lines lie where no column is above 1 by more than a few percent:
+// shorter to fetch).  Times of this file's kernel over that one's, heads of 128, portions of 96 to 2560 tokens, 32 heads on 8 unless noted; the
+// lines lie where no column is above 1 by more than a few percent.  (Measured before this file's kernel became 3 to 7 % faster: a call
+// just below a line may now take the slower kernel by as much.)
 //   tiles        no context, no cap   cap   | window 512 or 1024, context 2000: no cap   cap   | no window, context 2000: no cap   cap
 //   320 .. 416   0.86 .. 1.00   0.91 .. 1.03 | 1.05 .. 1.14   1.12 .. 1.20                     | 0.95 .. 1.18   1.13 .. 1.26
 //   448 .. 576   0.70 .. 0.76   0.72 .. 0.82 | 0.83 .. 0.90   0.90 .. 0.97                     | 0.82 .. 0.96   0.90 .. 0.99
